@@ -357,7 +357,7 @@ int launch_cfl(epp_ctx* ctx, int set, float cfl, const InstPhys* used, InstPhys*
     a.n_inst = ctx->n_inst;
     a.n_cells = ctx->n_cells;
     a.n_max = ctx->n;
-    a.chunks = ctx->cfl_chunks;
+    a.chunks = std::min(ctx->cfl_chunks, blocks_for(ctx->n, 256));   // no block without a particle to read
     a.vm = FUSED ? ctx->tmp.vm : ctx->S[set].vm;
     a.xh = FUSED ? ctx->tmp.xh : ctx->S[set].xh;
     a.tagm = ctx->S[set].tagm;
@@ -369,7 +369,7 @@ int launch_cfl(epp_ctx* ctx, int set, float cfl, const InstPhys* used, InstPhys*
     a.partial = ctx->cfl_partial;
     a.time = ctx->sim_time;
     a.ticket = ctx->cfl_ticket;
-    k_cfl<D, FUSED><<<ctx->n_inst * ctx->cfl_chunks, 256, 0, ctx->stream>>>(a);
+    k_cfl<D, FUSED><<<ctx->n_inst * a.chunks, 256, 0, ctx->stream>>>(a);
     CK_LAUNCH();
     return EPP_OK;
 }

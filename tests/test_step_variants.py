@@ -1,0 +1,53 @@
+"""Kernel variants the step picks by size: the same results on both sides of each rule."""
+import numpy as np
+import pytest
+
+from epp import abi, casegen
+from epp.algorithm import DeviceParticleSystem
+from epp.classes import NeighbourSystem
+
+SYM = abi.EPP_CRITERION_SYMMETRY
+CONT = abi.EPP_ACTION_DAMBREAK_CONTINUITY
+
+
+def device(case, n_instances=1, max_nb=1):
+    ns = NeighbourSystem(case.domain, casegen.DAM_BREAK_ACTIVE_PAIRS, max_neighbour_number=max_nb)
+    d = DeviceParticleSystem(case.ps, ns, n_instances=n_instances)
+    if n_instances > 1:
+        d.ctx.set_instance_physics(case.inst_dt, case.inst_c0)
+    d.syncto()
+    return d
+
+
+def stir(case, seed, speed=0.5, jitter=0.1):
+    """Random velocities and displacements of the fluid, so that every pair term is in play."""
+    rng = np.random.default_rng(seed)
+    x, v, fl = case.ps["PositionVec"], case.ps["VelocityVec"], case.ps["Tag"] == casegen.FLUID_TAG
+    x[fl] += np.float32(jitter * case.meta["dx"]) * rng.uniform(-1, 1, x[fl].shape).astype(np.float32)
+    v[fl] = speed * rng.standard_normal(v[fl].shape).astype(np.float32)
+    case.ps["PositionVec"] = x
+    case.ps["VelocityVec"] = v
+
+
+# instances per fold warp of the CFL reduction (8 warps): one each, all taken, some twice
+@pytest.mark.gpu
+@pytest.mark.parametrize("n_inst", [1, 8, 17])
+def test_cfl_dt_of_every_instance(n_inst):
+    columns = [(0.5 + 0.04 * k, 1.0 + 0.08 * k) for k in range(n_inst)]
+    b = casegen.dam_break_batch(columns=columns, dx=0.05)
+    stir(b, 3)
+    phys = b.physics
+    phys.cfl = 0.1
+    d = device(b, n_inst if n_inst > 1 else 1)
+    d.ctx.search(SYM, CONT, phys, 0)
+    d.ctx.step(3, phys)
+    dt, _ = d.ctx.step_dt(phys, n_inst)
+    d.asyncto()
+    v, h = d.host["VelocityVec"].astype(np.float64), d.host["H"].astype(np.float64)
+    fl = (d.host["Tag"] == casegen.FLUID_TAG) & (d.host.is_alive[: b.n] == 1)
+    for k, (r0, r1) in enumerate(b.rows):
+        on = np.arange(r0, r1)[fl[r0:r1]]
+        c0 = np.float64(np.float32(b.inst_c0[k])) if n_inst > 1 else np.float64(np.float32(phys.c0))
+        want = np.float32(np.float64(np.float32(0.1)) * h[on].min() / (c0 + np.sqrt((v[on] ** 2).sum(1).max())))
+        assert dt[k] == want, (k, dt[k], want)
+    d.close()
