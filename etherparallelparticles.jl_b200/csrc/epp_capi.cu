@@ -22,7 +22,6 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kProfileStages = EPP_PROFILE_STAGES;
 constexpr int kIntegralBlocks = 592;   // 4 x 148 SMs
-
 inline int blocks_for(long long n, int t = kThreads) { return (int)((n + t - 1) / t); }
 
 struct Arena {
@@ -211,22 +210,22 @@ int join_integrals(epp_ctx* ctx, int k = -1) {
 }
 
 size_t state_bytes(int cap) {
-    // xh, vm, dv, comp, rp4 (float4) + rho, drho, vol, p, tagm, id, cell (4 B), aligned
-    return (size_t)cap * (5 * 16 + 7 * 4) + 12 * 256;
+    // xh, vm, dv, comp (float4) + rho, drho, vol, p, tagm, id, cell (4 B), aligned
+    return (size_t)cap * (4 * 16 + 7 * 4) + 12 * 256;
 }
 
 size_t arena_bytes(int cap, int n_cells, int D, int n_tiles) {
     size_t b = 2 * state_bytes(cap);
     b += (size_t)cap * 3 * 16 + 3 * 256;                 // fused temp
+    b += (size_t)cap * (16 + 32) + 512;           // rp4, 2D neighbour records (both sets)
     b += (size_t)(n_cells + 2) * 4 + 256;                // count
     b += 2 * ((size_t)(n_cells + 2) * 4 + 256);          // start[2]
-    b += (size_t)cap * 8 * 2 + 512;                      // cs, perm
     b += (size_t)(n_tiles + 1) * 8 + 256;                // scan state
     b += 2 * ((size_t)(n_cells + 1) * 4 + 256 + 256);    // occ[2], meta[2]
     b += 256 * 3;                                        // status, pairs
     b += 2 * ((size_t)cap * 4 + 256);                    // nCount of each set
     b += (size_t)cap * 4 * (3 * D + 6) + 256;            // stage_f
-    b += (size_t)cap * 4 * SI_COUNT + 256;               // stage_i
+    b += (size_t)cap * 4 * SI_COUNT + 256;               // stage_i (cs and perm of the sort inside)
     b += (size_t)kIntegralBlocks * 8 * 8 + 8 * 8 + 4 * 256;
     b += 4 * ((size_t)cap * 4 + 256);                    // filter / extrapolation sums, gap by row
     b += 2 * 256;                                                                  // instance tables (small)
@@ -272,7 +271,6 @@ void fill_state(Arena& a, State& s, int cap) {
     s.tagm = a.take<int>(cap);
     s.id = a.take<int>(cap);
     s.cell = a.take<int>(cap);
-    s.rp4 = a.take<float4>(cap);
 }
 
 // The CFL tables (epp_physics.cfl > 0): c0 and B of every instance (its own c0 in a batch with
@@ -421,13 +419,31 @@ int launch_build(epp_ctx* ctx, int set, int crit, unsigned long long* pairs) {
     return EPP_OK;
 }
 
+// Lanes per particle of a list pass.  A small system leaves most schedulers with a warp or none, and
+// the pass is then as long as one thread's walk; four lanes per particle shorten it until the extra
+// prologues, epilogues and shuffles outweigh that.  Measured, us with 1 and 4 lanes:
+//   2D momentum    22,279 particles 21.4 / 15.2   49,048: 24.1 / 21.8   86,533: 33 / 36   515,018: 68 / 114
+//   3D continuity  33,123 particles 29.7 / 18.5   165,888: 51 / 47      955,668: 214 / 280
+//   3D momentum    33,123 particles 30.9 / 19.2   165,888: 64 / 48      955,668: 308 / 271 (always 4)
+template <int D, class Act>
+int list_lanes(const epp_ctx* ctx) {
+    if (kListInter<D, Act>) return 4;
+    return ctx->n <= (D == 2 ? 60000 : 250000) ? 4 : 1;
+}
+
 // Family 0, a pair action over the lists of the last search pass (same order and positions).
 template <int D, class Act, bool EPI = false>
 int launch_list(epp_ctx* ctx, int set, int crit, const Act& act) {
     PairArgs A = pair_args(ctx, set, crit);
     TileMask M{ctx->cap, ctx->nlist};
-    k_list<D, Act, EPI><<<blocks_for(ctx->n, ctx->pass_threads), ctx->pass_threads, 0, ctx->stream>>>(
-        A, M, ctx->ncnt[set], act, ctx->scan_state, ctx->n_tiles + 1);
+    auto launch = [&](auto LL) {
+        constexpr int L = decltype(LL)::value;
+        k_list<D, Act, EPI, L><<<blocks_for((long long)ctx->n * L, ctx->pass_threads), ctx->pass_threads, 0, ctx->stream>>>(
+            A, M, ctx->ncnt[set], act, ctx->scan_state, ctx->n_tiles + 1);
+    };
+    if constexpr (kListInter<D, Act>) launch(std::integral_constant<int, 4>{});
+    else if (list_lanes<D, Act>(ctx) == 4) launch(std::integral_constant<int, 4>{});
+    else launch(std::integral_constant<int, 1>{});
     CK_LAUNCH();
     return EPP_OK;
 }
@@ -843,7 +859,7 @@ int run_interaction(epp_ctx* ctx, int action, const epp_physics* phys) {
         return rc;
     }
     if (action == EPP_ACTION_DAMBREAK_MOMENTUM) {
-        k_prep_rp4<<<blocks_for(ctx->n), kThreads, 0, ctx->stream>>>(ctx->start[ctx->cur], ctx->n_cells, ctx->n,
+        k_prep_rp4<D><<<blocks_for(ctx->n), kThreads, 0, ctx->stream>>>(ctx->start[ctx->cur], ctx->n_cells, ctx->n,
                                                                       ctx->S[ctx->cur]);
         CK_LAUNCH();
         ActMomG<D, false> act;
@@ -922,7 +938,7 @@ int run_step(epp_ctx* ctx, int n_steps, const epp_physics& phys, bool accel) {
         ctx->rpn_valid = false;
     }
     if (!ctx->rpn_valid || !same_phys(ctx->rpn_phys, phys)) {
-        k_density_preview<<<blocks_for(ctx->n), kThreads, 0, ctx->stream>>>(
+        k_density_preview<D><<<blocks_for(ctx->n), kThreads, 0, ctx->stream>>>(
             ctx->start[ctx->cur], ctx->n_cells, ctx->n, ctx->S[ctx->cur], dev_phys(ctx, phys));
         CK_LAUNCH();
         ctx->rpn_walls = false;
@@ -1073,6 +1089,10 @@ int32_t epp_create(const epp_config* cfg, epp_ctx** out) {
     ctx->tmp.xh = a.take<float4>(ctx->cap);
     ctx->tmp.vm = a.take<float4>(ctx->cap);
     ctx->tmp.comp = a.take<float4>(ctx->cap);
+    // one density preview and one record buffer for both sets: the gather of a step has read the old
+    // set's before the search pass writes the new set's
+    ctx->S[0].rp4 = ctx->S[1].rp4 = a.take<float4>(ctx->cap);
+    ctx->S[0].rec = ctx->S[1].rec = a.take<float4>(2 * (size_t)ctx->cap);
     ctx->count = a.take<int>(ctx->n_cells + 2);
     ctx->start[0] = a.take<int>(ctx->n_cells + 2);
     ctx->start[1] = a.take<int>(ctx->n_cells + 2);
@@ -1080,15 +1100,18 @@ int32_t epp_create(const epp_config* cfg, epp_ctx** out) {
     ctx->occ[1] = a.take<int>(ctx->n_cells + 1);
     ctx->meta[0] = a.take<int>(64);
     ctx->meta[1] = a.take<int>(64);
-    ctx->cs = a.take<int2>(ctx->cap);
-    ctx->perm = a.take<int2>(ctx->cap);
     ctx->scan_state = a.take<unsigned long long>(ctx->n_tiles + 1);
     ctx->status = a.take<unsigned>(1);
     ctx->pairs = a.take<unsigned long long>(1);
     ctx->ncnt[0] = a.take<int>(ctx->cap);
     ctx->ncnt[1] = a.take<int>(ctx->cap);
     ctx->stage_f = a.take<float>((size_t)ctx->cap * (3 * D + 6));
+    // the sort's (cell, slot) and permutation live in the int staging columns: those are only in use
+    // inside epp_upload and epp_download, these only between a bin pass and its gather
+    static_assert(SI_COUNT >= 4, "cs and perm take four ints a particle");
     ctx->stage_i = a.take<int>((size_t)ctx->cap * SI_COUNT);
+    ctx->cs = reinterpret_cast<int2*>(ctx->stage_i);
+    ctx->perm = ctx->cs + ctx->cap;
     ctx->ipartial = a.take<double>(kIntegralBlocks * 8);
     ctx->iresult = a.take<double>(8);
     ctx->iticket = a.take<unsigned>(1);
@@ -1859,8 +1882,12 @@ int32_t epp_profile_step(epp_ctx* ctx, const epp_physics* phys, float* stage_ms)
         ctx->rpn_valid = false;
     }
     if (!ctx->rpn_valid || !same_phys(ctx->rpn_phys, *phys)) {
-        k_density_preview<<<blocks_for(ctx->n), kThreads, 0, ctx->stream>>>(
-            ctx->start[ctx->cur], ctx->n_cells, ctx->n, ctx->S[ctx->cur], dev_phys(ctx, *phys));
+        auto preview = [&](auto Dt) {
+            k_density_preview<decltype(Dt)::value><<<blocks_for(ctx->n), kThreads, 0, ctx->stream>>>(
+                ctx->start[ctx->cur], ctx->n_cells, ctx->n, ctx->S[ctx->cur], dev_phys(ctx, *phys));
+        };
+        if (ctx->D == 2) preview(std::integral_constant<int, 2>{});
+        else preview(std::integral_constant<int, 3>{});
         CK_LAUNCH();
     }
     if (ctx->last_crit != EPP_CRITERION_SYMMETRY) ctx->nlist_valid = false;

@@ -146,7 +146,7 @@ struct CPCont {
         if (!(ff || fw || wf)) return out;
         // every operation rounded on its own (no contraction into fused multiply-adds), so the term
         // is the same bit for bit wherever a pass evaluates it
-        const float r = sqrtf(g.dr2);
+        const float r = root(g.dr2);
         float hinv, kdw, hh;
         pair_consts<D>(tc, xj.w, hinv, kdw, hh);
         const float dwr = pair_dwr<D, GEN>(P.kernel, __fmul_rn(r, hinv), hinv, kdw);
@@ -170,9 +170,9 @@ struct CPCont {
         if (ti == P.fluid || ti == P.wall) {
             const int inst = inst_of(s.tagm[i]);
             const float rho = __fadd_rn(rho_i, __fmul_rn(drho, P.dt_of(inst)));
-            s.rp4[i] = make_rp4(rho, eos(P, inst, rho));
+            store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)));
         } else {
-            s.rp4[i] = make_rp4(rho_i, s.p[i]);
+            store_rp<D>(s, i, make_rp4(rho_i, s.p[i]));
         }
     }
     __device__ __forceinline__ void end_idle(int i, int ti) const { end(i, ti, make_float4(0, 0, 0, 0), 0); }
@@ -267,59 +267,95 @@ struct CPMom {
         if constexpr (GEN) return Nb{__ldg(&m.s.vm[j]), __ldg(&m.s.rp4[j]), gap_of(j)};
         else return Nb{__ldg(&m.s.vm[j]), __ldg(&m.s.rp4[j])};
     }
+    // The benchmark physics' pair (the dam break's classic fluid-fluid, balanced fluid-wall pressure
+    // and artificial viscosity) as one factor: du += pair_force d.  Straight-line (the viscosity is a
+    // select: warps hold approaching and receding pairs alike) with one reciprocal for the viscosity's
+    // three densities; every operation has its own rounding or an explicit fused multiply-add, so the
+    // value does not depend on the kernel that evaluates it.  z_j = p_j / rho_j^2.
+    __device__ __forceinline__ float pair_force(const Self& me, int tj, float hj, float mj, float rhoj, float zj,
+                                                float dr2, float vdx, const TargetConst& tc) const {
+        const DevPhys& P = m.P;
+        const bool ff = tj == P.fluid;
+        float hinv = tc.hinv, kdw = tc.kdw, hh = tc.hh;
+        if (hj != tc.h) {
+            const float4 c = hpair_consts<D>(tc.h, hj);
+            hinv = c.x;
+            kdw = c.y;
+            hh = c.z;
+        }
+        const float u = fmaxf(__fsub_rn(2.0f, __fmul_rn(root(dr2), hinv)), 0.0f);   // W = dW = 0 at q >= 2
+        const float md = __fmul_rn(mj, __fmul_rn(kdw, __fmul_rn(__fmul_rn(u, u), u)));
+        float s = __fadd_rn(me.rp.z, zj);                                              // iClassicPressure!
+        if (!ff) s = __fmul_rn(__fmaf_rn(me.rp.y, rcp_fast(rhoj), __fmul_rn(zj, rhoj)), me.rp.w);   // iBalancedPressure!
+        // sArtificialViscosity!: approaching pairs only
+        const bool ref = P.visc == EPP_VISCOSITY_REFERENCE;
+        const float az = __fmaf_rn(__fmul_rn(0.01f, hh), hh, dr2);
+        const float phi = __fmul_rn(vdx, rcp_fast(__fmul_rn(hinv, az)));
+        const float k = rcp_fast(__fmul_rn(__fadd_rn(me.rp.x, rhoj), ref ? rhoj : 1.0f));
+        const float w = __fmul_rn(__fmul_rn(__fmaf_rn(P.beta, phi, -__fmul_rn(P.alpha, me.c0)), phi),
+                                  __fmul_rn(k, __fmul_rn(2.0f, ref ? me.rp.w : 1.0f)));
+        if (vdx < 0.0f) s = __fadd_rn(s, w);
+        return u > 0.0f && (ff || tj == P.wall) ? -__fmul_rn(md, s) : 0.0f;
+    }
     __device__ __forceinline__ float4 term(const Self& me, const Nb& nb, int ti, int tj, float4 xj,
                                            const PairGeo& g, const TargetConst& tc) const {
         float4 out = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const DevPhys& P = m.P;
-        const bool ff = tj == P.fluid;
-        const bool fw = tj == P.wall;
-        if (!(ff || fw)) return out;
-        const float r = sqrtf(g.dr2);
-        float hinv, kdw, hh;
-        pair_consts<D>(tc, xj.w, hinv, kdw, hh);
-        const float dwr = pair_dwr<D, GEN>(P.kernel, r * hinv, hinv, kdw);
-        if (dwr == 0.0f) return out;
-        const float4 rpi = me.rp, rpj = nb.rp, vi = me.v, vj = nb.v;
-        float p_rho_2;
-        if constexpr (!GEN) {   // the dam break's pair: classic fluid-fluid, balanced fluid-wall
-            p_rho_2 = ff ? rpi.z + rpj.z : (rpi.y + rpj.y) * rpi.w * rpj.w;
+        if constexpr (!GEN) {
+            const float4 vi = me.v, vj = nb.v;
+            float vdx = __fmaf_rn(g.dy, __fsub_rn(vi.y, vj.y), __fmul_rn(g.dx, __fsub_rn(vi.x, vj.x)));
+            if (D == 3) vdx = __fmaf_rn(g.dz, __fsub_rn(vi.z, vj.z), vdx);
+            const float f = pair_force(me, tj, xj.w, vj.w, nb.rp.x, nb.rp.z, g.dr2, vdx, tc);
+            out.x = __fmul_rn(f, g.dx);
+            out.y = __fmul_rn(f, g.dy);
+            if (D == 3) out.z = __fmul_rn(f, g.dz);
+            return out;
         } else {
-            p_rho_2 = pressure_term(ff ? P.pff : P.pfw, rpi, rpj);
+            const bool ff = tj == P.fluid;
+            const bool fw = tj == P.wall;
+            if (!(ff || fw)) return out;
+            const float r = root(g.dr2);
+            float hinv, kdw, hh;
+            pair_consts<D>(tc, xj.w, hinv, kdw, hh);
+            const float dwr = pair_dwr<D, GEN>(P.kernel, r * hinv, hinv, kdw);
+            if (dwr == 0.0f) return out;
+            const float4 rpi = me.rp, rpj = nb.rp, vi = me.v, vj = nb.v;
+            float p_rho_2 = pressure_term(ff ? P.pff : P.pfw, rpi, rpj);
             if (P.tensile) {   // iPressureCorrection (Pressure.jl:10-22)
                 const float w = kern_value<D>(P.kernel, r, hinv);
                 const float w_gap = kern_value<D>(P.kernel, 0.5f * (me.gap + nb.gap), hinv);
                 p_rho_2 += fabsf(p_rho_2) * __fdiv_rn(0.01f * w, w_gap);
             }
-        }
-        const float fp = p_rho_2 * (-vj.w * dwr);
-        out.x = fp * g.dx;
-        out.y = fp * g.dy;
-        if (D == 3) out.z = fp * g.dz;
-        if (GEN && P.visc == EPP_VISCOSITY_CLASSIC) {
-            // iClassicViscosity! (Viscosity.jl:10-26): 2 mu m_j r dW / (rho_i rho_j (r^2 + 0.01 h^2))
-            // times (u_i - u_j); r dW = r^2 (dW / r)
-            const float az = g.dr2 + 0.01f * hh * hh;
-            const float force = __fdividef(2.0f * P.mu * vj.w * g.dr2 * dwr * rpi.w * rpj.w, az);
-            out.x += force * (vi.x - vj.x);
-            out.y += force * (vi.y - vj.y);
-            if (D == 3) out.z += force * (vi.z - vj.z);
+            const float fp = p_rho_2 * (-vj.w * dwr);
+            out.x = fp * g.dx;
+            out.y = fp * g.dy;
+            if (D == 3) out.z = fp * g.dz;
+            if (P.visc == EPP_VISCOSITY_CLASSIC) {
+                // iClassicViscosity! (Viscosity.jl:10-26): 2 mu m_j r dW / (rho_i rho_j (r^2 + 0.01 h^2))
+                // times (u_i - u_j); r dW = r^2 (dW / r)
+                const float az = g.dr2 + 0.01f * hh * hh;
+                const float force = __fdividef(2.0f * P.mu * vj.w * g.dr2 * dwr * rpi.w * rpj.w, az);
+                out.x += force * (vi.x - vj.x);
+                out.y += force * (vi.y - vj.y);
+                if (D == 3) out.z += force * (vi.z - vj.z);
+                return out;
+            }
+            float vdx = g.dx * (vi.x - vj.x);
+            vdx += g.dy * (vi.y - vj.y);
+            if (D == 3) vdx += g.dz * (vi.z - vj.z);
+            if (vdx < 0.0f) {
+                const float rhob = 0.5f * (rpi.x + rpj.x);
+                const float az = g.dr2 + 0.01f * hh * hh;
+                const float phi = __fdividef(vdx, hinv * az);
+                float force = __fdividef((-P.alpha * me.c0 + P.beta * phi) * phi, rhob);
+                if (P.visc == EPP_VISCOSITY_REFERENCE) force *= (-vj.w * rpi.w * rpj.w) * dwr;
+                else force *= -vj.w * dwr;
+                out.x += force * g.dx;
+                out.y += force * g.dy;
+                if (D == 3) out.z += force * g.dz;
+            }
             return out;
         }
-        float vdx = g.dx * (vi.x - vj.x);
-        vdx += g.dy * (vi.y - vj.y);
-        if (D == 3) vdx += g.dz * (vi.z - vj.z);
-        if (vdx < 0.0f) {
-            const float rhob = 0.5f * (rpi.x + rpj.x);
-            const float az = g.dr2 + 0.01f * hh * hh;
-            const float phi = __fdividef(vdx, hinv * az);
-            float force = __fdividef((-P.alpha * me.c0 + P.beta * phi) * phi, rhob);
-            if (P.visc == EPP_VISCOSITY_REFERENCE) force *= (-vj.w * rpi.w * rpj.w) * dwr;
-            else force *= -vj.w * dwr;
-            out.x += force * g.dx;
-            out.y += force * g.dy;
-            if (D == 3) out.z += force * g.dz;
-        }
-        return out;
     }
     __device__ __forceinline__ float4 contrib(int i, int j, int ti, int tj, float4 xi, float4 xj,
                                               const PairGeo& g, const TargetConst& tc) const {
@@ -424,7 +460,7 @@ struct CPExtrap {
     __device__ __forceinline__ void end(int i, int, float4 sum, int) const {
         if (FUSED) {
             const float p = sum.x > 0.0f ? __fdiv_rn(sum.y, sum.x) : P.p0;
-            s.rp4[i] = make_rp4(s.rp4[i].x, p);
+            store_rp<D>(s, i, make_rp4(s.rp4[i].x, p));
         } else {
             wv[i] += sum.x;
             wvp[i] += sum.y;

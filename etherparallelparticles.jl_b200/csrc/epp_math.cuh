@@ -66,6 +66,9 @@ struct State {
     int* id;         // 0-based row of the particle in the caller's matrices
     int* cell;       // 0-based cell (n_cells = dead bin)
     float4* rp4;     // (rho, p, p/rho^2, 1/rho) that the next momentum pass reads
+    float4* rec;     // 2D: what the momentum pass gathers of a neighbour, in one 32-byte load: (x, y, vx,
+                     // vy), (h, m, rho, p/rho^2), written with rp4.  Like rp4, one buffer serves both
+                     // state sets: it holds the current order.
 };
 
 struct NeighbourList {   // EPP_SEARCH_EMIT_LIST output, column-major [k * cap + i]
@@ -211,6 +214,43 @@ __device__ __forceinline__ void advance(const DevPhys& P, float dt, const float 
 __device__ __forceinline__ float4 make_rp4(float rho, float p) {
     return make_float4(rho, p, __fdiv_rn(p, __fmul_rn(rho, rho)), __fdiv_rn(1.0f, rho));
 }
+
+// rp4 of particle i and, in 2D, its neighbour record.
+template <int D>
+__device__ __forceinline__ void store_rp(const State& s, int i, float4 rp) {
+    s.rp4[i] = rp;
+    if (D == 2) {
+        const float4 x = s.xh[i], v = s.vm[i];
+        s.rec[2 * (size_t)i] = make_float4(x.x, x.y, v.x, v.y);
+        s.rec[2 * (size_t)i + 1] = make_float4(x.w, v.w, rp.x, rp.z);
+    }
+}
+
+// A neighbour record in one 256-bit load through the read-only path.
+struct Rec8 {
+    float4 a, b;
+};
+__device__ __forceinline__ Rec8 load_rec(const float4* rec, int j) {
+    Rec8 r;
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(r.a.x), "=f"(r.a.y), "=f"(r.a.z), "=f"(r.a.w), "=f"(r.b.x), "=f"(r.b.y), "=f"(r.b.z), "=f"(r.b.w)
+        : "l"(rec + 2 * (size_t)j));
+    return r;
+}
+
+// Square root by Newton's iteration on 1 / sqrt(x) from the approximate reciprocal root, the last
+// step on the residual x - s^2: no branch for special operands.  Equal to the IEEE square root for
+// every mantissa (both binades of 1, 2^-20, 2^-40, 2^20 and 2^-93 compared with __fsqrt_rn on
+// B200); arguments below 1e-30 (coincident particles) give 1e-15, whose q = r / h rounds as 0 does
+// in 2 - q.  Infinity gives NaN: outside the support, as the infinite root is.
+__device__ __forceinline__ float root(float x) {
+    x = fmaxf(x, 1e-30f);
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    const float s = __fmul_rn(x, y);
+    return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, y), s);
+}
+__device__ __forceinline__ float rcp_fast(float x) { return __fdividef(1.0f, x); }
 
 // The cell grid of a domain, on the host, in FP32 as the Domain2D constructor computes it
 // (Domain2D.jl:28-67): n_a = floor(span_a / gap) cells per axis, gap_a = span_a / n_a and

@@ -77,7 +77,7 @@ __global__ void k_filter_finish(const int* start, int n_cells, int n_max, State 
     }
     if (preview && (ti == P.fluid || ti == P.wall)) {
         const float rn = __fadd_rn(s.rho[i], __fmul_rn(s.drho[i], P.dt_of(inst)));
-        s.rp4[i] = make_rp4(rn, eos(P, inst, rn));
+        store_rp<D>(s, i, make_rp4(rn, eos(P, inst, rn)));
     }
 }
 
@@ -99,6 +99,7 @@ __global__ void k_extrap_finish(const int* start, int n_cells, int n_max, State 
 }
 
 // Density preview used when the fused step starts from a state whose rpn is not current.
+template <int D>
 __global__ void k_density_preview(const int* start, int n_cells, int n_max, State s, DevPhys P) {
     const int n_alive = min(start[n_cells], n_max);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -107,9 +108,9 @@ __global__ void k_density_preview(const int* start, int n_cells, int n_max, Stat
     if (ti == P.fluid || ti == P.wall) {
         const int inst = inst_of(s.tagm[i]);
         const float rho = __fadd_rn(s.rho[i], __fmul_rn(s.drho[i], P.dt_of(inst)));
-        s.rp4[i] = make_rp4(rho, eos(P, inst, rho));
+        store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)));
     } else {
-        s.rp4[i] = make_rp4(s.rho[i], s.p[i]);
+        store_rp<D>(s, i, make_rp4(s.rho[i], s.p[i]));
     }
 }
 

@@ -92,6 +92,7 @@ __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
     return r;
 }
 
+
 template <int D>
 struct TileConf {
     static constexpr int NRMAX = D == 2 ? 3 : 9;   // stencil rows: ranges of a tile or of one particle
@@ -450,90 +451,230 @@ __device__ __noinline__ float4 neighbours_by_stencil(const PairArgs& A, int i, f
     return sum;
 }
 
-// A pair action over the neighbour lists written by the last search pass (same positions,
-// cells and criterion): one thread per particle walking its own list, the next entries already
-// in flight.  EPI: fused momentum step (integrate + bin for every
-// particle, dead bin included; block 0 clears the scan state).
-template <int D, class Act, bool EPI>
-__global__ void __launch_bounds__(128, D == 2 ? 9 : 4)   // 2D: 9 blocks (56 registers) beat 8, 10 and 12
+// What a list pass gathers of a neighbour (Rec), the pair's term (Term) and the sum of the terms (Acc),
+// by action.  By default position and the action's own fields, the term from Act::term, each component
+// added with its own rounding.  `from` is a term as lane `src` of the group holds it.
+template <int D, class Act>
+struct ListTerm {
+    struct Me {
+        float4 x;
+        typename Act::Self s;
+        TargetConst tc;
+        int tag;
+    };
+    struct Rec {
+        float4 x;
+        typename Act::Nb nb;
+    };
+    struct Term {
+        float x, y, z;
+    };
+    using Acc = Term;
+    static __device__ __forceinline__ Me me(const Act& act, int i, float4 xi, int ti) {
+        return Me{xi, act.self(i), target_const<D>(xi.w), ti};
+    }
+    static __device__ __forceinline__ Rec load(const PairArgs& A, const Act& act, const Me& m, int j, int tj) {
+        return Rec{__ldg(&A.s.xh[j]), act.fetch(j, m.tag, tj)};
+    }
+    static __device__ __forceinline__ Term term(const Act& act, const Me& m, const Rec& r, int tj) {
+        const float4 t = act.term(m.s, r.nb, m.tag, tj, r.x, geometry<D>(m.x, r.x), m.tc);
+        return Term{t.x, t.y, t.z};
+    }
+    static __device__ __forceinline__ Term from(unsigned group, const Term& t, int src) {
+        return Term{__shfl_sync(group, t.x, src), Act::NC > 1 ? __shfl_sync(group, t.y, src) : 0.0f,
+                    Act::NC > 2 && D == 3 ? __shfl_sync(group, t.z, src) : 0.0f};
+    }
+    static __device__ __forceinline__ void add(Acc& a, const Term& t) {
+        a.x = __fadd_rn(a.x, t.x);
+        if (Act::NC > 1) a.y = __fadd_rn(a.y, t.y);
+        if (Act::NC > 2 && D == 3) a.z = __fadd_rn(a.z, t.z);
+    }
+};
+
+// The benchmark physics' momentum: du += f d as fused multiply-adds.  2D: all of a neighbour from its
+// 32-byte record, one load in place of three 16-byte gathers; x and y through the packed f32x2 pipe.
+template <int D, bool FUSED>
+struct ListTerm<D, CPMom<D, FUSED, false>> {
+    using Act = CPMom<D, FUSED, false>;
+    struct Me {
+        f32x2 x, v;
+        float z, vz;
+        typename Act::Self s;
+        TargetConst tc;
+    };
+    struct Rec3 {
+        float4 x, v, rp;
+    };
+    using Rec = typename std::conditional<D == 2, Rec8, Rec3>::type;
+    struct Term {
+        float f, dx, dy, dz;
+    };
+    struct Acc {
+        float x, y, z;
+    };
+    static __device__ __forceinline__ Me me(const Act& act, int i, float4 xi, int) {
+        const typename Act::Self s = act.self(i);
+        return Me{f2_pack(xi.x, xi.y), f2_pack(s.v.x, s.v.y), xi.z, s.v.z, s, target_const<D>(xi.w)};
+    }
+    static __device__ __forceinline__ Rec load(const PairArgs& A, const Act&, const Me&, int j, int) {
+        if constexpr (D == 2) return load_rec(A.s.rec, j);
+        else return Rec{__ldg(&A.s.xh[j]), __ldg(&A.s.vm[j]), __ldg(&A.s.rp4[j])};
+    }
+    static __device__ __forceinline__ Term term(const Act& act, const Me& m, const Rec& r, int tj) {
+        float px, py, ux, uy;   // the neighbour's position and velocity
+        if constexpr (D == 2) {
+            px = r.a.x, py = r.a.y, ux = r.a.z, uy = r.a.w;
+        } else {
+            px = r.x.x, py = r.x.y, ux = r.v.x, uy = r.v.y;
+        }
+        Term t;
+        const f32x2 d = f2_sub(m.x, f2_pack(px, py));
+        float ex, ey, vx, vy;
+        f2_unpack(d, t.dx, t.dy);
+        f2_unpack(f2_mul(d, d), ex, ey);
+        f2_unpack(f2_sub(m.v, f2_pack(ux, uy)), vx, vy);
+        float dr2 = __fadd_rn(ex, ey);
+        float vdx = __fmaf_rn(t.dy, vy, __fmul_rn(t.dx, vx));
+        if constexpr (D == 2) {
+            t.dz = 0.0f;
+            t.f = act.pair_force(m.s, tj, r.b.x, r.b.y, r.b.z, r.b.w, dr2, vdx, m.tc);
+        } else {
+            t.dz = __fsub_rn(m.z, r.x.z);
+            dr2 = __fadd_rn(dr2, __fmul_rn(t.dz, t.dz));
+            vdx = __fmaf_rn(t.dz, __fsub_rn(m.vz, r.v.z), vdx);
+            t.f = act.pair_force(m.s, tj, r.x.w, r.v.w, r.rp.x, r.rp.z, dr2, vdx, m.tc);
+        }
+        return t;
+    }
+    static __device__ __forceinline__ Term from(unsigned group, const Term& t, int src) {
+        return Term{__shfl_sync(group, t.f, src), __shfl_sync(group, t.dx, src), __shfl_sync(group, t.dy, src),
+                    D == 3 ? __shfl_sync(group, t.dz, src) : 0.0f};
+    }
+    static __device__ __forceinline__ void add(Acc& a, const Term& t) {
+        a.x = __fmaf_rn(t.f, t.dx, a.x);
+        a.y = __fmaf_rn(t.f, t.dy, a.y);
+        if (D == 3) a.z = __fmaf_rn(t.f, t.dz, a.z);
+    }
+};
+
+// 3D momentum sums four interleaved partials (every size takes the same form: there are no 3D batches).
+template <int D, class Act>
+constexpr bool kListInter = D == 3 && Act::NC == 3;
+
+// A pair action over the neighbour lists written by the last search pass (same positions, cells and
+// criterion).  L lanes share a particle, lane g takes entries k = g mod L.
+//   L = 1        one thread per particle, terms added in list order
+//   L = 4        every lane of the group adds a round's four terms in list order: the bits of L = 1
+//                (a 2D batch and its instances alone may differ in L)
+//   L = 4 INTER  (3D momentum) four partial sums, one a lane, folded as (0 + 1) + (2 + 3)
+// What bounds it: the wavefronts its neighbour gathers take in the L1 (84-91% of peak in 3D) and, with
+// few warps in flight, one thread's serial walk.  Lanes that share a particle gather consecutive
+// entries, whose records share cache lines: 3D momentum, 955,668 particles, 308 us with L = 1 and 271
+// with L = 4 (three 16-byte gathers each way; one 32-byte record for x, v made it no faster, as half as
+// many particles share a line).  In 2D a neighbour's record fits one 32-byte load: momentum 79 -> 68 us
+// at 515,018 particles.
+// EPI: fused momentum step (integrate + bin for every particle, dead bin included; block 0 clears the
+// scan state).
+template <int D, class Act, bool EPI, int L>
+__global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 blocks (56 registers) beat 7, 8 and 10
     k_list(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M, const int* ncount,
            const __grid_constant__ Act act, unsigned long long* scan_state, int n_scan_words) {
+    using T = ListTerm<D, Act>;
+    constexpr bool ROW = ListConf<D>::ROW;
+    constexpr bool INTER = kListInter<D, Act> && L > 1;
     if (EPI && blockIdx.x == 0)
         for (int t = threadIdx.x; t < n_scan_words; t += blockDim.x) scan_state[t] = 0ull;
     const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(tid / L), g = (int)(tid % L);
     if (i < n_alive) {
         const float4 xi = A.s.xh[i];
         const int ti = tag_of(A.s.tagm[i]);
         if (ti < 1 || ti > A.n_tags || !act.wants(ti)) {
-            act.end_idle(i, ti);
-        } else {
-            const TargetConst tc = target_const<D>(xi.w);
-            const int cnt = ncount[i];
-            float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            int got = cnt;
-            if (cnt <= ListConf<D>::LCAP) {
-                const typename Act::Self me = act.self(i);
-                ListReader<D> lr;
-                lr.start(M, i, cnt);
-                if (D == 2) {   // 2D: a second neighbour record in flight costs more than it hides
-                    for (int k = 0; k < cnt; ++k) {
-                        const int e = lr.next(k);
-                        const int j = entry_index(e);
-                        EPP_CHECK(j < A.n_max, 16, j);
-                        const int tj = entry_tag(e);
-                        const float4 xj = __ldg(&A.s.xh[j]);
-                        const float4 t =
-                            act.term(me, act.fetch(j, ti, tj), ti, tj, xj, geometry<D>(xi, xj), tc);
-                        sum.x += t.x;
-                        sum.y += t.y;
-                        sum.z += t.z;
-                    }
-                    act.end(i, ti, sum, got);
-                    return;
-                }
-                // 3D: software pipeline, neighbour k + 1's loads in flight while k's term runs
-                // the row is read four entries (16 bytes) at a time, two groups ahead; inside a
-                // group the entry is picked at compile time
-                const int4* row = reinterpret_cast<const int4*>(lr.base);
-                int4 q = lr.q, qn = lr.qn;
-                int en = cnt > 0 ? q.x : list_entry(0, 1);
-                int jn = entry_index(en);
-                EPP_CHECK(jn < A.n_max, 16, jn);
-                float4 xn = cnt > 0 ? __ldg(&A.s.xh[jn]) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-                typename Act::Nb nn = act.fetch(jn, ti, entry_tag(en));
-                for (int k0 = 0; k0 < cnt; k0 += 4) {
-                    const int4 q2 = k0 + 8 < cnt ? row[(k0 >> 2) + 2] : make_int4(0, 0, 0, 0);
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int k = k0 + u;
-                        if (k >= cnt) break;
-                        const int tj = entry_tag(en);
-                        const float4 xj = xn;
-                        const typename Act::Nb nb = nn;
-                        if (k + 1 < cnt) {
-                            en = u == 0 ? q.y : u == 1 ? q.z : u == 2 ? q.w : qn.x;
-                            jn = entry_index(en);
-                            EPP_CHECK(jn < A.n_max, 16, jn);
-                            xn = __ldg(&A.s.xh[jn]);
-                            nn = act.fetch(jn, ti, entry_tag(en));
-                        }
-                        const float4 t = act.term(me, nb, ti, tj, xj, geometry<D>(xi, xj), tc);
-                        sum.x += t.x;
-                        sum.y += t.y;
-                        sum.z += t.z;
-                    }
-                    q = qn;
-                    qn = q2;
-                }
-            } else {
-                sum = neighbours_by_stencil<D>(A, i, xi, ti, tc, act);
-                got = (int)sum.w;
-                sum.w = 0.0f;
-            }
-            act.end(i, ti, sum, got);
+            if (g == 0) act.end_idle(i, ti);
+            return;
         }
-    } else if (EPI && i < A.n_max) {
+        const int cnt = ncount[i];
+        if (cnt > ListConf<D>::LCAP) {   // more neighbours than the list keeps
+            if (g == 0) {
+                const TargetConst tc = target_const<D>(xi.w);
+                float4 sum = neighbours_by_stencil<D>(A, i, xi, ti, tc, act);
+                const int got = (int)sum.w;
+                sum.w = 0.0f;
+                act.end(i, ti, sum, got);
+            }
+            return;
+        }
+        const typename T::Me me = T::me(act, i, xi, ti);
+        typename T::Acc acc{};
+        if constexpr (L == 1 && ROW) {
+            // software pipeline, neighbour k + 1's loads in flight while k's term runs; the row is
+            // read four entries (16 bytes) at a time, two groups ahead (ordinary loads: a row's next
+            // group shares its line), inside a group the entry is picked at compile time
+            const int4* row = reinterpret_cast<const int4*>(M.list + (size_t)i * ListConf<D>::LCAP);
+            int4 q = cnt > 0 ? row[0] : make_int4(0, 0, 0, 0);
+            int4 qn = cnt > 4 ? row[1] : make_int4(0, 0, 0, 0);
+            int en = cnt > 0 ? q.x : list_entry(0, 1);
+            EPP_CHECK(entry_index(en) < A.n_max, 16, entry_index(en));
+            typename T::Rec rn = T::load(A, act, me, entry_index(en), entry_tag(en));
+            for (int k0 = 0; k0 < cnt; k0 += 4) {
+                const int4 q2 = k0 + 8 < cnt ? row[(k0 >> 2) + 2] : make_int4(0, 0, 0, 0);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int k = k0 + u;
+                    if (k >= cnt) break;
+                    const int tj = entry_tag(en);
+                    const typename T::Rec r = rn;
+                    if (k + 1 < cnt) {
+                        en = u == 0 ? q.y : u == 1 ? q.z : u == 2 ? q.w : qn.x;
+                        EPP_CHECK(entry_index(en) < A.n_max, 16, entry_index(en));
+                        rn = T::load(A, act, me, entry_index(en), entry_tag(en));
+                    }
+                    T::add(acc, T::term(act, me, r, tj));
+                }
+                q = qn;
+                qn = q2;
+            }
+        } else {
+            // the lane's next entry is read ahead.  2D lists are column-major and read once each:
+            // streaming loads keep the L1 for the records.
+            const int* list = ROW ? M.list + (size_t)i * ListConf<D>::LCAP + g : M.list + i + (size_t)g * M.cap;
+            const size_t stride = ROW ? L : (size_t)L * M.cap;
+            const int first = (int)(threadIdx.x & 31u & ~(unsigned)(L - 1));
+            const unsigned group = L == 1 ? 0u : ((1u << L) - 1u) << first;
+            int en = g < cnt ? (ROW ? *list : __ldcs(list)) : 0;
+            for (int k0 = 0; k0 < cnt; k0 += L) {
+                typename T::Term t{};
+                if (k0 + g < cnt) {
+                    const int j = entry_index(en), tj = entry_tag(en);
+                    EPP_CHECK(j < A.n_max, 16, j);
+                    const typename T::Rec r = T::load(A, act, me, j, tj);
+                    if (k0 + L + g < cnt) {
+                        list += stride;
+                        en = ROW ? *list : __ldcs(list);
+                    }
+                    t = T::term(act, me, r, tj);
+                    if (L == 1 || INTER) T::add(acc, t);
+                }
+                if constexpr (L > 1 && !INTER) {
+#pragma unroll
+                    for (int u = 0; u < L; ++u) {
+                        const typename T::Term tu = T::from(group, t, first + u);
+                        if (k0 + u < cnt) T::add(acc, tu);
+                    }
+                }
+            }
+            if constexpr (INTER) {
+#pragma unroll
+                for (int o = 1; o < L; o <<= 1) {
+                    acc.x = __fadd_rn(acc.x, __shfl_xor_sync(group, acc.x, o));
+                    if (Act::NC > 1) acc.y = __fadd_rn(acc.y, __shfl_xor_sync(group, acc.y, o));
+                    if (Act::NC > 2) acc.z = __fadd_rn(acc.z, __shfl_xor_sync(group, acc.z, o));
+                }
+            }
+        }
+        if (g == 0) act.end(i, ti, make_float4(acc.x, acc.y, acc.z, 0.0f), cnt);
+    } else if (EPI && i < A.n_max && g == 0) {
         act.end_idle(i, tag_of(A.s.tagm[i]));
     }
 }
