@@ -147,8 +147,11 @@ struct CPCont {
         // every operation rounded on its own (no contraction into fused multiply-adds), so the term
         // is the same bit for bit wherever a pass evaluates it
         const float r = root(g.dr2);
-        float hinv, kdw, hh;
-        pair_consts<D>(tc, xj.w, hinv, kdw, hh);
+        float hinv = tc.hinv, kdw = tc.kdw;
+        if (xj.w != tc.h) {
+            hinv = invharmonic_exact(tc.h, xj.w);
+            kdw = wc2_kdw<D>(hinv);
+        }
         const float dwr = pair_dwr<D, GEN>(P.kernel, __fmul_rn(r, hinv), hinv, kdw);
         if (dwr == 0.0f) return out;
         float vdx = __fmul_rn(g.dx, __fsub_rn(me.v.x, nb.v.x));
@@ -157,6 +160,25 @@ struct CPCont {
         if (ff) out.x = __fmul_rn(__fmul_rn(nb.v.w, vdx), dwr);                              // iClassicContinuity!
         else out.x = __fmul_rn(__fmul_rn(__fmul_rn(me.rho, vol_of(nb)), vdx), dwr);         // iBalancedContinuity!
         return out;
+    }
+    // term() of a 2D fluid-fluid pair of equal h, the same bits: vectors on the packed pipe, and under
+    // the benchmark kernel the support's edge as a clamp (a zero factor) in place of a branch
+    static constexpr bool FAST = D == 2;
+    __device__ __forceinline__ float fluid_term(f32x2 xi, f32x2 vi, float4 xj, float4 nb, const TargetConst& tc) const {
+        const f32x2 d = f2_sub(xi, f2_pack(xj.x, xj.y));
+        float ex, ey, vx, vy;
+        f2_unpack(f2_mul(d, d), ex, ey);
+        f2_unpack(f2_mul(d, f2_sub(vi, f2_pack(nb.x, nb.y))), vx, vy);
+        const float q = __fmul_rn(root(__fadd_rn(ex, ey)), tc.hinv);
+        float dwr;
+        if constexpr (GEN) {
+            dwr = pair_dwr<D, GEN>(P.kernel, q, tc.hinv, tc.kdw);
+            if (dwr == 0.0f) return 0.0f;
+        } else {
+            const float u = fmaxf(__fsub_rn(2.0f, q), 0.0f);
+            dwr = __fmul_rn(tc.kdw, __fmul_rn(__fmul_rn(u, u), u));
+        }
+        return __fmul_rn(__fmul_rn(nb.w, __fadd_rn(vx, vy)), dwr);
     }
     __device__ __forceinline__ float4 contrib(int i, int j, int ti, int tj, float4 xi, float4 xj,
                                               const PairGeo& g, const TargetConst& tc) const {
@@ -182,6 +204,7 @@ struct CPCont {
 template <int D>
 struct CPCount {
     int* ncount;
+    static constexpr bool FAST = false;
     static constexpr int NC = 0;
     struct Self {};
     struct Nb {};

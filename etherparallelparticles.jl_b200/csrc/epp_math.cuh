@@ -17,6 +17,27 @@ namespace epp {
 
 constexpr int kMaxTags = EPP_MAX_TAGS;
 
+// Division of 0 <= v < 2^31 by a fixed d >= 1 as a multiplication (round-up method, Granlund and
+// Montgomery 1994): with l = ceil(log2 d) and m = floor(2^(31 + l) / d) + 1, v / d = (v m) >> (31 + l);
+// m < 2^32 for d >= 2, and d = 1 is kept apart (m = 0).
+struct FastDiv {
+    unsigned m;
+    int s;
+    __host__ void set(int d) {
+        int l = 0;
+        while ((1ll << l) < d) ++l;
+        m = d <= 1 ? 0u : (unsigned)((1ull << (31 + l)) / (unsigned)d + 1ull);
+        s = l > 0 ? l - 1 : 0;
+    }
+    __host__ __device__ int div(int v) const {
+#ifdef __CUDA_ARCH__
+        return m ? (int)(__umulhi((unsigned)v, m) >> s) : v;
+#else
+        return m ? (int)((unsigned)(((unsigned long long)(unsigned)v * m) >> 32) >> s) : v;
+#endif
+    }
+};
+
 // Domain in FP32 (as Domain2D{Int32, Float32}); n[a] cells per axis, x fastest.
 struct DevDomain {
     int dim;
@@ -26,6 +47,7 @@ struct DevDomain {
     int n_inst;           // instances stacked as independent layers (2D only)
     float gap_square;
     float first[3], last[3], gap_inv[3];
+    FastDiv by[2];        // division by n[0] and n[1]: the coordinates of a linear cell index
 };
 
 // Per-instance constants of a batch (each instance has its own column height, so its own c0
@@ -238,6 +260,31 @@ __device__ __forceinline__ Rec8 load_rec(const float4* rec, int j) {
     return r;
 }
 
+// Pairs of FP32 values in one 64-bit register: Blackwell's f32x2 arithmetic performs two IEEE
+// round-to-nearest operations per instruction.  Packed sub and mul match __fsub_rn / __fmul_rn
+// bit for bit (checked on B200 over 8M random pairs); a packed add fed directly by a packed
+// multiply was measured to round like a fused multiply-add, so sums stay scalar __fadd_rn.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_unpack(f32x2 v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+
 // Square root by Newton's iteration on 1 / sqrt(x) from the approximate reciprocal root, the last
 // step on the residual x - s^2: no branch for special operands.  Equal to the IEEE square root for
 // every mantissa (both binades of 1, 2^-20, 2^-40, 2^20 and 2^-93 compared with __fsqrt_rn on
@@ -291,6 +338,7 @@ inline int plan_domain(const epp_domain& in, int n_inst, long long max_cells, De
         if (ncell > max_cells) return EPP_ERR_CAPACITY;
     }
     if (ncell * n_inst > max_cells) return EPP_ERR_CAPACITY;   // <= 2^30 * 2^22
+    for (int a = 0; a < 2; ++a) d.by[a].set(d.n[a]);
     d.cells_per_inst = (int)ncell;
     d.n_inst = n_inst;
     d.n_cells = (int)(ncell * n_inst);

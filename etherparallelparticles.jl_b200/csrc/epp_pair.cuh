@@ -79,10 +79,8 @@ __device__ __forceinline__ void traverse(const PairArgs& A, int i, float4 xi, in
 
 // Adds the per-thread neighbour counts of a block's warps to *counter (all lanes take part).
 __device__ __forceinline__ void count_pairs(unsigned long long* counter, int cnt) {
-    unsigned long long c = (unsigned long long)cnt;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0 && counter && c) atomicAdd(counter, c);
+    const int c = __reduce_add_sync(0xffffffffu, cnt);   // 32 counts of at most 2^26 candidates each
+    if ((threadIdx.x & 31) == 0 && counter && c) atomicAdd(counter, (unsigned long long)c);
 }
 
 template <int D, class Act>

@@ -68,31 +68,6 @@ __device__ __forceinline__ PairGeo geometry(float4 xi, float4 xj) {
     return g;
 }
 
-// Pairs of FP32 values in one 64-bit register: Blackwell's f32x2 arithmetic performs two IEEE
-// round-to-nearest operations per instruction.  Packed sub and mul match __fsub_rn / __fmul_rn
-// bit for bit (checked on B200 over 8M random pairs); a packed add fed directly by a packed
-// multiply was measured to round like a fused multiply-add, so sums stay scalar __fadd_rn.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 f2_pack(float a, float b) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void f2_unpack(f32x2 v, float& a, float& b) {
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ f32x2 f2_sub(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-
-
 template <int D>
 struct TileConf {
     static constexpr int NRMAX = D == 2 ? 3 : 9;   // stencil rows: ranges of a tile or of one particle

@@ -7,19 +7,23 @@
 // the warp's union of stencils against every lane -- about 190 per particle; here each lane tests
 // only its own window, 81 candidates.
 //
-// A warp takes 32 consecutive particles in cell order.  When their cells lie in one cell row, the
-// union of their windows in a stencil row is one contiguous range; the warp stages the three union
-// rows (up to 64 candidates each) in shared memory in one round -- position and h, the list entry
-// (index and tag) in the unused z lane, and the search action's neighbour record -- and every lane
-// reads its own window from there.  The lane builds one acceptance word per stencil row with the
-// reference's IEEE criterion (and the active-pair matrix, applied from per-row tag bitmaps), then
-// walks the set bits of the three words in list order, in one loop: it appends the neighbour to
-// its list (the lists the momentum, filter and extrapolation passes read; same layout and order as
-// k_build's: stencil rows, then cell order, then id order inside a cell) and adds the search
-// action's term -- the continuity rate -- from the staged record, so no separate continuity pass
-// walks the neighbours again.  Windows beyond 32 candidates (dense neighbourhoods) go row by row
-// in 32-candidate chunks.  A warp that crosses a cell-row end takes one such round per cell
-// row of its particles; union rows longer than 64 are read from global memory instead.
+// A warp takes 32 consecutive particles in cell order.  Those of one cell row (without a gap) form a
+// part: the union of their windows in a stencil row is one contiguous range, from the first lane's
+// window to the last lane's.  The warp stages the three ranges of each part in shared memory, packed one after the other
+// -- position and h, the list entry (index and tag) in the unused z lane, and the search action's
+// neighbour record -- and every lane reads its own windows from there.  The staging area holds both
+// parts of a warp that crosses a cell-row end; what does not fit (a free surface, whose warps span
+// many cells over a dense row; dense neighbourhoods) is split into passes over fewer lanes.  The lane
+// builds one acceptance word per stencil row with the reference's IEEE criterion and the active-pair
+// matrix, then walks the set bits of the three words in list order, in one loop: it appends the
+// neighbour to its list (the lists the momentum, filter and extrapolation passes read; same layout
+// and order as k_build's: stencil rows, then cell order, then id order inside a cell) and adds the
+// search action's term -- the continuity rate -- from the staged record, so no separate continuity
+// pass walks the neighbours again.
+//
+// What bounds it: instruction issue at large sizes (bulk warps -- one h, one tag, fluid -- take a
+// specialised test and walk), and at middle sizes the slowest warp, hence one pass for all parts and
+// no dependent global reads in it.
 #pragma once
 #include "epp_tile.cuh"
 
@@ -52,63 +56,31 @@ __device__ __forceinline__ RowWin row_range(const PairArgs& A, int row, int xa, 
     return w;
 }
 
+constexpr int kStage2 = 240;   // staged candidates per warp: 7 blocks of 128 threads still fit an SM
+
 template <class Act>
 struct Stage2 {
-    float4 x[3 * 64];                 // (x, y, list entry as bits, h)
-    typename Act::Nb nb[3 * 64];
+    float4 x[kStage2];                 // (x, y, list entry as bits, h)
+    typename Act::Nb nb[kStage2];
 };
 
-// Stages union rows u[0..2] (each at most 64 candidates) and records, per row, the union slots
-// whose tag this lane's row of the active-pair matrix allows and whether every candidate of the
-// row has one h (one_h, h0).  A tag outside 1..n_tags sets EPP_STATUS_BAD_TAG.  Warp-collective.
-template <class Act, bool FETCH>
-__device__ __forceinline__ void stage_rows2(const PairArgs& A, const Act& act, Stage2<Act>& S, const RowWin (&u)[3],
-                                            unsigned amask, int lane, unsigned& st, unsigned long long (&allowed)[3],
-                                            bool (&one_h)[3], float (&h0)[3]) {
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-        allowed[r] = 0ull;
-        one_h[r] = true;
-        h0[r] = 0.0f;
-#pragma unroll
-        for (int part = 0; part < 2; ++part) {
-            if (u[r].lo + part * 32 >= u[r].hi) break;   // warp-uniform: nothing left in this row
-            const int k = part * 32 + lane;
-            const int j = u[r].lo + k;
-            const bool real = j < u[r].hi;
-            const float4 xj = real ? A.s.xh[j] : make_float4(1e30f, 1e30f, 0.0f, 0.0f);
-            const int tj = real ? tag_of(A.s.tagm[j]) : 0;
-            S.x[64 * r + k] = make_float4(xj.x, xj.y, __int_as_float(list_entry(j, tj >= 1 ? tj : 1)), xj.w);
-            if (FETCH && real) S.nb[64 * r + k] = act.fetch(j, 0, tj);
-            if (__ballot_sync(0xffffffffu, real && (tj < 1 || tj > A.n_tags))) st |= EPP_STATUS_BAD_TAG;
-            for (int t = 1; t <= A.n_tags; ++t) {
-                const unsigned b = __ballot_sync(0xffffffffu, real && tj == t);
-                if ((amask >> (t - 1)) & 1u) allowed[r] |= (unsigned long long)b << (part * 32);
-            }
-            const float hf = __shfl_sync(0xffffffffu, xj.w, 0);
-            if (part == 0) h0[r] = hf;
-            one_h[r] = __all_sync(0xffffffffu, !real || xj.w == h0[r]) && one_h[r];
-        }
-    }
-    __syncwarp();
-}
-
-// Acceptance bits of staged candidates [k0, k1) (k1 - k0 <= 32) of a lane's window starting at
-// slot `off`: bit k - k0 set when candidate k is within the criterion's radius, by the reference's
-// IEEE arithmetic.  `uniform`: every candidate has the lane's h (or the default criterion), so one
-// exact bound `r2u` serves; otherwise the bound is looked up per candidate.
-__device__ __forceinline__ unsigned window_bits(const float4* sx, int off, int k0, int k1, float4 xi, bool uniform,
-                                                float r2u, float h2sq, bool dflt, float gap_square) {
+// Acceptance bits of a lane's window of `len` <= 32 candidates from slot `off`: bit k set when
+// candidate k passes the criterion by the reference's IEEE arithmetic.  `one`: every candidate has the
+// lane's h (or the default criterion), so one exact bound serves; otherwise it is looked up per
+// candidate.  Cells hold their fluid before their walls, so h alternates along a row between the
+// lane's own and a wall's: the last other h and its bound (a division) are kept in (ho, ro).
+__device__ __forceinline__ unsigned window_bits(const float4* sx, int off, int len, float4 xi, bool one, float own, bool dflt,
+                                                float& ho, float& ro) {
     // (dx, dy) and (dx^2, dy^2) on the packed f32x2 pipe (each half rounds like __fsub_rn /
     // __fmul_rn), the sum scalar
     const f32x2 XY = f2_pack(xi.x, xi.y);
     unsigned word = 0u;
-    if (uniform) {
+    if (one) {
         // dr2 <= R2 as integers: non-negative floats order like their bit patterns, so
         // bits(dr2) - bits(R2) - 1 is negative exactly for the accepted candidates
-        const int nR2 = -__float_as_int(r2u) - 1;
-        for (int k = k1 - 1; k >= k0; --k) {
+        const int nR2 = -__float_as_int(own) - 1;
+#pragma unroll 4
+        for (int k = len - 1; k >= 0; --k) {
             const f32x2 d = f2_sub(XY, *reinterpret_cast<const f32x2*>(&sx[off + k]));
             float dx2, dy2;
             f2_unpack(f2_mul(d, d), dx2, dy2);
@@ -116,17 +88,17 @@ __device__ __forceinline__ unsigned window_bits(const float4* sx, int off, int k
         }
         return word;
     }
-    float hc = xi.w, rc = dflt ? gap_square : h2sq;
-    for (int k = k1 - 1; k >= k0; --k) {
+#pragma unroll 4
+    for (int k = len - 1; k >= 0; --k) {
         const float hj = sx[off + k].w;
         const f32x2 d = f2_sub(XY, *reinterpret_cast<const f32x2*>(&sx[off + k]));
         float dx2, dy2;
         f2_unpack(f2_mul(d, d), dx2, dy2);
-        if (hj != hc) {
-            hc = hj;
-            rc = dflt ? gap_square : (hc == xi.w ? h2sq : pair_r2(xi.w, hc));
+        if (hj != xi.w && hj != ho) {
+            ho = hj;
+            ro = dflt ? own : pair_r2(xi.w, ho);
         }
-        word = (word << 1) | (__fadd_rn(dx2, dy2) <= rc ? 1u : 0u);
+        word = (word << 1) | (__fadd_rn(dx2, dy2) <= (hj == xi.w ? own : ro) ? 1u : 0u);
     }
     return word;
 }
@@ -135,79 +107,39 @@ __device__ __forceinline__ unsigned window_bits(const float4* sx, int off, int k
 struct WinOut {
     int cnt;
     float sx, sy;
-    unsigned st;
 };
 
-// The per-lane search of the 2D search pass in its general form: windows of any length, row by
-// row 32 candidates at a time, from the staged union rows u[] or, when `staged` is false, from
-// global memory.  Only dense neighbourhoods (a window beyond 32 candidates) and union rows beyond
-// the staging area come here.  Inlined: as an out-of-line call it cost the kernel registers (the
-// values live across the call) and 13% of its time.
-// uniform_rows: bit r set when every candidate of staged row r has the lane's h (or the default
-// criterion), so one exact bound serves the row.
+// The per-lane search in its general form, candidate by candidate from global memory: dense
+// neighbourhoods only (a window beyond 32 candidates, or windows beyond the staging area).  Inlined:
+// as an out-of-line call it cost the kernel registers (the values live across the call) and 13% of
+// its time.
 template <class Act>
-__device__ __forceinline__ WinOut win_lane_general(const PairArgs& A, const TileMask& M, const Act& act,
-                                                const Stage2<Act>& S, bool staged, RowWin u0, RowWin u1, RowWin u2,
-                                                unsigned long long al0, unsigned long long al1, unsigned long long al2,
-                                                unsigned uniform_rows, int i, int ti, float4 xi, unsigned amask,
-                                                int rid, int cx) {
+__device__ __forceinline__ WinOut win_lane_general(const PairArgs& A, const TileMask& M, const Act& act, RowWin w0, RowWin w1,
+                                                RowWin w2, int i, int ti, float4 xi, unsigned amask) {
     const TargetConst tc = target_const<2>(xi.w);
     const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
     typename Act::Self me = act.self(i);
     ListWriter<2> L = list_writer<2>(M, i);
-    WinOut o{0, 0.0f, 0.0f, 0u};
-#pragma unroll
+    WinOut o{0, 0.0f, 0.0f};
+    float ho = xi.w, ro = dflt ? A.dom.gap_square : tc.h2sq;
+#pragma unroll 1
     for (int r = 0; r < 3; ++r) {
-        const RowWin win = row_range(A, stencil_row2(A, rid, rid % A.dom.n[1], r), cx - 1, cx + 1);
-        const RowWin u = r == 0 ? u0 : (r == 1 ? u1 : u2);
-        const unsigned long long allowed = r == 0 ? al0 : (r == 1 ? al1 : al2);
-        const int len = win.hi - win.lo;
-        const int woff = win.lo - u.lo;
-        const bool uniform = staged && ((uniform_rows >> r) & 1u);
-        for (int k0 = 0; k0 < len; k0 += 32) {
-            const int k1 = min(len, k0 + 32);
-            unsigned word;
-            if (staged) {
-                word = window_bits(S.x, 64 * r + woff, k0, k1, xi, uniform, dflt ? A.dom.gap_square : tc.h2sq,
-                                   tc.h2sq, dflt, A.dom.gap_square);
-                word &= (unsigned)(allowed >> (woff + k0));
-            } else {
-                word = 0u;
-                for (int k = k1 - 1; k >= k0; --k) {
-                    const int j = win.lo + k;
-                    word = (word << 1) | (accept<2>(A, i, xi, amask, tc.h2sq, j, A.s.xh[j], o.st) ? 1u : 0u);
-                }
+        const int lo = r == 0 ? w0.lo : r == 1 ? w1.lo : w2.lo, hi = r == 0 ? w0.hi : r == 1 ? w1.hi : w2.hi;
+#pragma unroll 1
+        for (int j = lo; j < hi; ++j) {
+            const float4 xj = A.s.xh[j];
+            const int tj = tag_of(A.s.tagm[j]);
+            const PairGeo g = geometry<2>(xi, xj);
+            if (xj.w != ho) {
+                ho = xj.w;
+                ro = dflt ? A.dom.gap_square : ho == xi.w ? tc.h2sq : pair_r2(xi.w, ho);
             }
-            if (k1 - k0 < 32) word &= (1u << (k1 - k0)) - 1u;
-            if (r == 1) {   // not its own neighbour
-                const int ks = i - win.lo - k0;
-                if (ks >= 0 && ks < 32) word &= ~(1u << ks);
-            }
-            while (word) {   // append and run the search action, in list order
-                const int k = k0 + __ffs(word) - 1;
-                word &= word - 1u;
-                float4 xj;
-                int e, tj;
-                typename Act::Nb nb;
-                if (staged) {
-                    const float4 xs = S.x[64 * r + woff + k];
-                    e = __float_as_int(xs.z);
-                    xj = make_float4(xs.x, xs.y, 0.0f, xs.w);
-                    tj = entry_tag(e);
-                    if (Act::NC != 0) nb = S.nb[64 * r + woff + k];
-                } else {
-                    const int j = win.lo + k;
-                    xj = A.s.xh[j];
-                    tj = tag_of(A.s.tagm[j]);
-                    e = list_entry(j, tj);
-                    if (Act::NC != 0) nb = act.fetch(j, ti, tj);
-                }
-                L.put(o.cnt++, e);
-                if (Act::NC != 0) {
-                    const float4 t = act.term(me, nb, ti, tj, xj, geometry<2>(xi, xj), tc);
-                    o.sx = __fadd_rn(o.sx, t.x);
-                    o.sy = __fadd_rn(o.sy, t.y);
-                }
+            if (!(g.dr2 <= ro) || j == i || !(__funnelshift_rc(amask, 0u, (unsigned)(tj - 1)) & 1u)) continue;
+            L.put(o.cnt++, list_entry(j, tj));
+            if (Act::NC != 0) {
+                const float4 t = act.term(me, act.fetch(j, ti, tj), ti, tj, xj, g, tc);
+                o.sx = __fadd_rn(o.sx, t.x);
+                o.sy = __fadd_rn(o.sy, t.y);
             }
         }
     }
@@ -223,6 +155,7 @@ template <class Act>
 __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M,
                                                    const __grid_constant__ Act act, unsigned long long* pairs) {
     __shared__ Stage2<Act> stage[4];
+    constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     Stage2<Act>& S = stage[threadIdx.x >> 5];
     const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
@@ -231,112 +164,274 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
     int cnt = 0;
     if (w0 < n_alive) {   // warp-uniform
         const bool on = i < n_alive;
-        const int n0 = A.dom.n[0];
         const int c = A.s.cell[min(i, n_alive - 1)];
-        EPP_CHECK(!__any_sync(0xffffffffu, c < 0 || c >= A.dom.n_cells), 34, c);
-        const int rid = c / n0, cx = c - rid * n0;
-        const int y = rid % A.dom.n[1];
+        EPP_CHECK(!__any_sync(FULL, c < 0 || c >= A.dom.n_cells), 34, c);
+        const int rid = A.dom.by[0].div(max(c, 0)), cx = c - rid * A.dom.n[0];
+        const int y = rid - A.dom.by[1].div(rid) * A.dom.n[1];
         const float4 xi = on ? A.s.xh[i] : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
         const int ti = on ? tag_of(A.s.tagm[i]) : 0;
         const bool valid = on && ti >= 1 && ti <= A.n_tags;
-        unsigned st = (on && !valid) ? EPP_STATUS_BAD_TAG : 0u;
-        const unsigned amask = valid ? A.adj[ti - 1] : 0u;
+        const unsigned amask = valid ? A.adj[ti - 1] : 0u;   // bits of valid tags only
+        const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
+        RowWin win[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) win[r] = row_range(A, stencil_row2(A, rid, y, r), cx - 1, cx + 1);
+        // a part ends at the end of a cell row and where the next lane's windows do not meet this one's:
+        // what lies between (the floor under a gap of the fluid) is nobody's candidate
+        const int rid_p = __shfl_up_sync(FULL, rid, 1), cx_p = __shfl_up_sync(FULL, cx, 1);
+        const unsigned starts = __ballot_sync(FULL, lane == 0 || rid != rid_p || cx - cx_p > 3);
         float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        // One round per cell row among the warp's particles (cell order keeps each row's lanes
-        // contiguous): a warp inside one cell row -- all but about 2% -- takes one round; a warp
-        // that crosses a row end stages the union rows of each part in turn instead of reading
-        // candidates from global memory one dependent load at a time.
-        unsigned pending = __ballot_sync(0xffffffffu, on);
-        while (pending) {   // warp-uniform
-            const int lead = __ffs(pending) - 1;
-            const int rid_g = __shfl_sync(0xffffffffu, rid, lead);
-            const int y_g = __shfl_sync(0xffffffffu, y, lead);
-            const bool mine = ((pending >> lane) & 1u) && rid == rid_g;
-            const unsigned members = __ballot_sync(0xffffffffu, mine);
-            const int xa = __shfl_sync(0xffffffffu, cx, lead) - 1;
-            const int xb = __shfl_sync(0xffffffffu, cx, 31 - __clz(members)) + 1;
-            pending &= ~members;
-            RowWin u[3];
-            bool staged = true;
+        unsigned pending = __ballot_sync(FULL, on);
+        while (pending) {   // warp-uniform: a pass over as many parts as the staging area holds
+            const int head = __ffs(pending) - 1;
+            const float hw = __shfl_sync(FULL, xi.w, head);   // the pass is plain when every candidate has
+            const int tw = __shfl_sync(FULL, ti, head);       // the first lane's h and tag
+            bool same_h = true, same_t = true, staged = false;
+            int used = 0, off[3] = {0, 0, 0};
+            unsigned taken = 0u;
+            __syncwarp();
+            while (pending) {
+                const int lead = __ffs(pending) - 1;
+                const unsigned after = starts & ~((2u << lead) - 1u);   // part starts behind the lead
+                int last = min(after ? __ffs(after) - 2 : 31, 31 - __clz(pending));
+                int lo[3], len[3], total;
+                for (;;) {
+                    total = 0;
 #pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                u[r] = row_range(A, stencil_row2(A, rid_g, y_g, r), xa, xb);
-                staged = staged && u[r].hi - u[r].lo <= 64;   // warp-uniform
+                    for (int r = 0; r < 3; ++r) {
+                        lo[r] = __shfl_sync(FULL, win[r].lo, lead);
+                        len[r] = max(__shfl_sync(FULL, win[r].hi, last) - lo[r], 0);
+                        total += len[r];
+                    }
+                    if (total <= kStage2 - used || used > 0 || last == lead) break;
+                    last = lead + (last - lead) / 2;
+                }
+                if (total > kStage2 - used) {
+                    if (used > 0) break;   // next pass
+                    taken = 1u << lead;    // one lane's windows are too long: read from global memory
+                    pending &= ~taken;
+                    break;
+                }
+                for (int k = lane; k < total; k += 32) {
+                    const int j = k < len[0] ? lo[0] + k : k < len[0] + len[1] ? lo[1] + (k - len[0]) : lo[2] + (k - len[0] - len[1]);
+                    const float4 xj = A.s.xh[j];
+                    const int tj = tag_of(A.s.tagm[j]);
+                    const bool bad = tj < 1 || tj > A.n_tags;   // never a neighbour: fails every test (its own lane reports it)
+                    S.x[used + k] = make_float4(bad ? __int_as_float(0x7fffffff) : xj.x, xj.y,
+                                                __int_as_float(list_entry(j, bad ? 1 : tj)), xj.w);
+                    if (Act::NC != 0) S.nb[used + k] = act.fetch(j, 0, tj);
+                    same_h = same_h && xj.w == hw;
+                    same_t = same_t && tj == tw;
+                }
+                const unsigned part = ((2u << last) - 1u) & ~((1u << lead) - 1u);
+                if ((part >> lane) & 1u) {
+                    staged = true;
+                    off[0] = used + win[0].lo - lo[0];
+                    off[1] = used + len[0] + win[1].lo - lo[1];
+                    off[2] = used + len[0] + len[1] + win[2].lo - lo[2];
+                }
+                used += total;
+                taken |= part;
+                pending &= ~part;
             }
-            unsigned long long allowed[3] = {0ull, 0ull, 0ull};
-            bool one_h[3] = {false, false, false};
-            float h0[3] = {0.0f, 0.0f, 0.0f};
-            if (staged) stage_rows2<Act, Act::NC != 0>(A, act, S, u, amask, lane, st, allowed, one_h, h0);
-            if (!(mine && valid)) continue;
-            const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
-            RowWin win[3];
-#pragma unroll
-            for (int r = 0; r < 3; ++r) win[r] = row_range(A, stencil_row2(A, rid, y, r), cx - 1, cx + 1);
-            unsigned uniform_rows = 0u;
-#pragma unroll
-            for (int r = 0; r < 3; ++r)
-                if (one_h[r] && (dflt || h0[r] == xi.w)) uniform_rows |= 1u << r;
-            if (!staged || win[0].hi - win[0].lo > 32 || win[1].hi - win[1].lo > 32 || win[2].hi - win[2].lo > 32) {
-                const WinOut o = win_lane_general<Act>(A, M, act, S, staged, u[0], u[1], u[2], allowed[0], allowed[1],
-                                                       allowed[2], uniform_rows, i, ti, xi, amask, rid, cx);
+            same_h = __all_sync(FULL, same_h);   // (also orders the staging before its use)
+            same_t = __all_sync(FULL, same_t);
+            __syncwarp();
+            if (!(((taken >> lane) & 1u) && valid)) continue;
+            const int l0 = win[0].hi - win[0].lo, l1 = win[1].hi - win[1].lo, l2 = win[2].hi - win[2].lo;
+            const int longest = max(l0, max(l1, l2));
+            // cells of four particle rows or columns (where the lattice and the cells drift apart) make
+            // windows of up to 40: the lanes of the pass then take each row in two words, one after the other
+            const bool two = __any_sync(__activemask(), staged && longest > 32);
+            if (!staged || longest > 64) {
+                const WinOut o = win_lane_general<Act>(A, M, act, win[0], win[1], win[2], i, ti, xi, amask);
                 cnt = o.cnt;
                 sum.x = o.sx;
                 sum.y = o.sy;
-                st |= o.st;
                 continue;
             }
-            // every window in one word: the three words first, then one walk over all of them, so
-            // a warp iterates as often as its busiest lane's neighbour count (not the sum over rows
-            // of each row's busiest lane)
             const TargetConst tc = target_const<2>(xi.w);
-            unsigned w[3];
-            int off[3];
-#pragma unroll
-            for (int r = 0; r < 3; ++r) {
-                const int len = win[r].hi - win[r].lo;
-                const int woff = win[r].lo - u[r].lo;   // the window's first slot in its staged row
-                off[r] = 64 * r + woff;
-                unsigned word = 0u;
-                if (len > 0) {
-                    word = window_bits(S.x, off[r], 0, len, xi, (uniform_rows >> r) & 1u,
-                                       dflt ? A.dom.gap_square : tc.h2sq, tc.h2sq, dflt, A.dom.gap_square);
-                    word &= (unsigned)(allowed[r] >> woff);
-                    if (len < 32) word &= (1u << len) - 1u;
-                }
-                if (r == 1) word &= ~(1u << (i - win[1].lo));   // not its own neighbour
-                w[r] = word;
-            }
+            if (same_t && !((amask >> (tw - 1)) & 1u)) continue;   // nothing the lane may see: walls among walls
+            const bool one = dflt || (same_h && xi.w == hw);
+            const float own = dflt ? A.dom.gap_square : tc.h2sq;
+            float ho = xi.w, ro = own;   // the last other h and its bound
             typename Act::Self me = act.self(i);
             ListWriter<2> L = list_writer<2>(M, i);
-            unsigned a = w[0], b = w[1], c2 = w[2];
-            while (a | b | c2) {   // append and run the search action, in list order
-                const int r = a ? 0 : (b ? 1 : 2);
-                const unsigned cur = a ? a : (b ? b : c2);
-                const int slot = (r == 0 ? off[0] : (r == 1 ? off[1] : off[2])) + __ffs(cur) - 1;
-                const unsigned rest = cur & (cur - 1u);
-                if (r == 0) a = rest;
-                else if (r == 1) b = rest;
-                else c2 = rest;
-                const float4 xs = S.x[slot];
-                const int e = __float_as_int(xs.z);
-                L.put(cnt++, e);
-                if (Act::NC != 0) {
-                    const int tj = entry_tag(e);
-                    const float4 xj = make_float4(xs.x, xs.y, 0.0f, xs.w);
-                    const float4 t = act.term(me, S.nb[slot], ti, tj, xj, geometry<2>(xi, xj), tc);
-                    sum.x = __fadd_rn(sum.x, t.x);
-                    sum.y = __fadd_rn(sum.y, t.y);
+            const f32x2 XI = f2_pack(xi.x, xi.y);
+            bool bulk = false;   // the bulk of the fluid: fluid candidates of the lane's h around a fluid lane
+            if constexpr (Act::FAST) bulk = same_t && one && !dflt && tw == act.P.fluid && ti == tw;
+            for (int q = 0; q < (two ? 6 : 1); ++q) {
+                unsigned a, b = 0u, c2 = 0u;
+                int o0 = off[0], o1 = off[1], o2 = off[2];
+                if (!two) {
+                    // the three words first, then one walk over all of them, so a warp iterates as often as
+                    // its busiest lane's neighbour count (not the sum over rows of each row's busiest lane)
+                    a = window_bits(S.x, o0, l0, xi, one, own, dflt, ho, ro);
+                    b = window_bits(S.x, o1, l1, xi, one, own, dflt, ho, ro);
+                    c2 = window_bits(S.x, o2, l2, xi, one, own, dflt, ho, ro);
+                    b &= ~(1u << (i - win[1].lo));   // not its own neighbour
+                    if (!b) b = c2, o1 = o2, c2 = 0u;   // empty rows last: one word is current, the next follows
+                    if (!a) a = b, o0 = o1, b = c2, o1 = o2, c2 = 0u;
+                } else {
+                    const int r = q >> 1, k0 = (q & 1) * 32;
+                    o0 = (r == 0 ? off[0] : r == 1 ? off[1] : off[2]) + k0;
+                    a = window_bits(S.x, o0, min((r == 0 ? l0 : r == 1 ? l1 : l2) - k0, 32), xi, one, own, dflt, ho, ro);
+                    const int self = i - win[1].lo - k0;
+                    if (r == 1 && self >= 0 && self < 32) a &= ~(1u << self);
+                }
+                if (bulk) {
+                    if constexpr (Act::FAST) {
+                        const f32x2 VI = f2_pack(me.v.x, me.v.y);
+                        while (a) {
+                            const int slot = o0 + __ffs(a) - 1;
+                            a &= a - 1u;
+                            if (!a) a = b, o0 = o1, b = c2, o1 = o2, c2 = 0u;
+                            const float4 xs = S.x[slot];
+                            L.put(cnt++, __float_as_int(xs.z));
+                            sum.x = __fadd_rn(sum.x, act.fluid_term(XI, VI, xs, S.nb[slot].v, tc));
+                        }
+                    }
+                } else {
+                    while (a) {   // append and run the search action, in list order
+                        const int slot = o0 + __ffs(a) - 1;
+                        a &= a - 1u;
+                        if (!a) a = b, o0 = o1, b = c2, o1 = o2, c2 = 0u;
+                        const float4 xs = S.x[slot];
+                        const int e = __float_as_int(xs.z);
+                        if (!((amask >> (entry_tag(e) - 1)) & 1u)) continue;   // the active-pair matrix
+                        L.put(cnt++, e);
+                        if (Act::NC != 0) {
+                            const int tj = entry_tag(e);
+                            const float4 xj = make_float4(xs.x, xs.y, 0.0f, xs.w);
+                            const float4 t = act.term(me, S.nb[slot], ti, tj, xj, geometry<2>(xi, xj), tc);
+                            sum.x = __fadd_rn(sum.x, t.x);
+                            sum.y = __fadd_rn(sum.y, t.y);
+                        }
+                    }
                 }
             }
             L.flush(cnt);
         }
         if (on) {
-            if (!valid) act.end_idle(i, ti);
-            else act.end(i, ti, sum, cnt);
+            if (!valid) {
+                act.end_idle(i, ti);
+                atomicOr(A.status, EPP_STATUS_BAD_TAG);
+            } else {
+                act.end(i, ti, sum, cnt);
+            }
         }
-        if (st) atomicOr(A.status, st);
     }
     count_pairs(pairs, cnt);
+}
+
+// The same pass for small systems: L lanes per particle, candidates straight from global memory, so a
+// particle's walk is L times shorter.  Lane g tests candidates g, g + L, ... of each window (four loads
+// in flight); a ballot of the group gives each accepted one its place in the list, kept in shared
+// memory; then lane g writes entries g, g + L, ... out and evaluates the action's terms for them, and
+// the first lane adds the terms in list order: lists, counts and sums have the bits of k_win_build.  A
+// particle with more neighbours than a list keeps goes through the general per-lane search.  It issues
+// four times k_win_build's instructions per particle (383 against 93) but a fifth of them one after
+// the other: 12 us against 25 at 1,418 particles, 22 each at 22,279.
+template <class Act, int L>
+__global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M,
+                                                   const __grid_constant__ Act act, unsigned long long* pairs) {
+    constexpr int P = 128 / L, CAP = ListConf<2>::LCAP;
+    __shared__ int s_e[P][CAP + 1];                           // accepted entries (odd rows: no bank conflicts)
+    __shared__ float s_t[Act::NC != 0 ? P : 1][CAP + 1];      // their terms
+    const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
+    const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / L);
+    const int g = threadIdx.x % L, p = threadIdx.x / L;
+    const int first = (int)(threadIdx.x & 31u & ~(unsigned)(L - 1));
+    const unsigned group = ((1u << L) - 1u) << first;
+    int cnt = 0;
+    if (i < n_alive) {
+        const float4 xi = A.s.xh[i];
+        const int ti = tag_of(A.s.tagm[i]);
+        const int c = A.s.cell[i];
+        if (ti < 1 || ti > A.n_tags) {
+            if (g == 0) {
+                act.end_idle(i, ti);
+                atomicOr(A.status, EPP_STATUS_BAD_TAG);
+            }
+        } else {
+            EPP_CHECK(c >= 0 && c < A.dom.n_cells, 35, c);
+            const int rid = A.dom.by[0].div(c), cx = c - rid * A.dom.n[0];
+            const int y = rid - A.dom.by[1].div(rid) * A.dom.n[1];
+            RowWin win[3];
+#pragma unroll
+            for (int r = 0; r < 3; ++r) win[r] = row_range(A, stencil_row2(A, rid, y, r), cx - 1, cx + 1);
+            const unsigned amask = A.adj[ti - 1];   // bits of valid tags only
+            const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
+            const TargetConst tc = target_const<2>(xi.w);
+            const float r2own = dflt ? A.dom.gap_square : tc.h2sq;
+            const f32x2 XI = f2_pack(xi.x, xi.y);
+            float ho = xi.w, ro = r2own;   // the bound of the last h_j seen
+#pragma unroll
+            for (int r = 0; r < 3; ++r) {
+                for (int j0 = win[r].lo; j0 < win[r].hi; j0 += 4 * L) {
+                    float4 xj[4];
+                    int tm[4];
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        const int j = j0 + q * L + g;
+                        xj[q] = make_float4(0.0f, 0.0f, 0.0f, xi.w);
+                        tm[q] = 0;
+                        if (j < win[r].hi && j != i) {
+                            xj[q] = A.s.xh[j];
+                            tm[q] = tag_of(A.s.tagm[j]);
+                        }
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) {
+                        if (j0 + q * L >= win[r].hi) break;   // uniform in the group
+                        // the reference's IEEE criterion and the active-pair matrix (tag 0: none)
+                        float ex, ey;
+                        const f32x2 d = f2_sub(XI, f2_pack(xj[q].x, xj[q].y));
+                        f2_unpack(f2_mul(d, d), ex, ey);
+                        if (xj[q].w != ho) {
+                            ho = xj[q].w;
+                            ro = dflt || ho == xi.w ? r2own : pair_r2(xi.w, ho);
+                        }
+                        const bool ok = __fadd_rn(ex, ey) <= ro && (__funnelshift_rc(amask, 0u, (unsigned)(tm[q] - 1)) & 1u);
+                        const unsigned hits = (__ballot_sync(group, ok) >> first) & ((1u << L) - 1u);
+                        const int at = cnt + __popc(hits & ((1u << g) - 1u));
+                        if (ok && at < CAP) s_e[p][at] = list_entry(j0 + q * L + g, tm[q]);
+                        cnt += __popc(hits);
+                    }
+                }
+            }
+            float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (cnt > CAP) {
+                if (g == 0) {
+                    const WinOut o = win_lane_general<Act>(A, M, act, win[0], win[1], win[2], i, ti, xi, amask);
+                    sum.x = o.sx;
+                    sum.y = o.sy;
+                }
+            } else {
+                __syncwarp(group);
+                const typename Act::Self me = act.self(i);
+#pragma unroll 2
+                for (int k = g; k < cnt; k += L) {
+                    const int e = s_e[p][k], j = entry_index(e), tj = entry_tag(e);
+                    M.list[(size_t)k * M.cap + i] = e;
+                    if constexpr (Act::NC != 0) {
+                        const float4 xj = A.s.xh[j];
+                        const typename Act::Nb nb = act.fetch(j, ti, tj);
+                        s_t[p][k] = act.term(me, nb, ti, tj, xj, geometry<2>(xi, xj), tc).x;
+                    }
+                }
+                if constexpr (Act::NC != 0) {
+                    __syncwarp(group);
+                    if (g == 0) {
+#pragma unroll 4
+                        for (int k = 0; k < cnt; ++k) sum.x = __fadd_rn(sum.x, s_t[p][k]);
+                    }
+                }
+            }
+            if (g == 0) act.end(i, ti, sum, cnt);
+        }
+    }
+    count_pairs(pairs, g == 0 ? cnt : 0);
 }
 
 }  // namespace epp

@@ -92,3 +92,59 @@ def test_batch_beyond_the_lane_rules_equals_its_instances(threads):
         for name, v in alone.items():
             assert np.array_equal(d.host[name][r0:r1], v), (k, name)
     d.close()
+
+
+# The eight-lane search (up to 20,000 particles) against the staged one (beyond), on windows of every
+# kind: lattices that drift against the cells (windows beyond 32 candidates), fluid and walls of
+# different h, sparse rows, and lists beyond their capacity (h = 3 dx).  The 20-instance batch takes the
+# staged search, each instance alone the eight-lane one.
+@pytest.mark.gpu
+@pytest.mark.parametrize("dx,h_factor,jitter,physics", [(0.0231, 1.5, 0.1, "benchmark"), (0.03, 1.5, 0.4, "benchmark"),
+                                                        (0.045, 3.0, 0.1, "benchmark"), (0.0231, 1.5, 0.1, "example")])
+def test_eight_lane_search_equals_the_staged_search(dx, h_factor, jitter, physics):
+    n_inst = 24
+    columns = [(0.5 + 0.03 * k, 1.0 + 0.05 * k) for k in range(n_inst)]
+    b = casegen.dam_break_batch(columns=columns, dx=dx, h_factor=h_factor)
+    if physics == "example":   # any kernel but the specialised one
+        b.physics.kernel = abi.EPP_KERNEL_CUBIC_SPLINE
+    stir(b, 7, jitter=jitter)
+    assert b.n > 20000
+    d = device(b, n_inst)
+    d.ctx.search(SYM, CONT, b.physics, 0)
+    d.ctx.synchronize()
+    d.asyncto()
+    cnt, ids = d.ctx.neighbour_lists(b.n, 64)
+    for k in (0, 11, 23):
+        r0, r1 = b.rows[k]
+        c = casegen.dam_break_2d(dx=dx, column=columns[k], h_factor=h_factor, max_neighbour_number=1)
+        for name in ("PositionVec", "VelocityVec"):
+            c.ps[name] = d.host[name][r0:r1]
+        c.physics.kernel = b.physics.kernel
+        assert c.n <= 20000
+        a = device(c)
+        a.ctx.search(SYM, CONT, c.physics, 0)
+        a.ctx.synchronize()
+        a.asyncto()
+        acnt, aids = a.ctx.neighbour_lists(c.n, 64)
+        assert np.array_equal(acnt, cnt[r0:r1])
+        assert np.array_equal(np.where(aids > 0, aids + r0, 0), ids[r0:r1])
+        for name in ("dDensity", "nCount"):
+            assert np.array_equal(a.host[name], d.host[name][r0:r1]), (k, name)
+        a.close()
+    d.close()
+
+
+# v / d by multiplication, on the CPU: the same arithmetic as csrc/epp_math.cuh FastDiv
+@pytest.mark.parametrize("d", [1, 2, 3, 7, 64, 1000, 1367, 65535, 65537, (1 << 22) + 1, (1 << 30) - 1, 1 << 30])
+def test_fast_division(d):
+    length = 0
+    while (1 << length) < d:
+        length += 1
+    m, s = (0, 0) if d <= 1 else ((1 << (31 + length)) // d + 1, length - 1)
+    assert m < 1 << 32
+    rng = np.random.default_rng(d)
+    v = np.concatenate([rng.integers(0, 1 << 31, 20000), np.arange(0, min(20 * d, 1 << 31), max(1, d))[:2000],
+                        np.arange(d - 1, min(20 * d, (1 << 31) - 1), d)[:2000], [0, (1 << 31) - 1]])
+    for x in (int(x) for x in v):
+        q = x if m == 0 else ((x * m) >> 32) >> s
+        assert q == x // d, (x, d)
