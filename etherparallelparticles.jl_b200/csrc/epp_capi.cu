@@ -396,18 +396,19 @@ bool generic_physics(const epp_physics* p) {
 // continuity pass (epp_set_tuning EPP_TUNING_LISTS); 3D always uses the latter.
 bool uses_windows(const epp_ctx* ctx) { return ctx->D == 2 && ctx->store != EPP_TUNING_LISTS; }
 
-// Largest particle count at which the 2D search pass takes eight lanes per particle: measured, us with
-// eight lanes and with one, 12 / 25 at 1,418 particles, 14 / 23 at 6,518, 22 / 22 at 22,279, 33 / 27 at
-// 45,203.
-constexpr int kWinLanesMax = 20000;
+// Largest particle count at which the search pass takes eight lanes per particle: measured, us with
+// eight lanes and with one, 2D 12 / 25 at 1,418 particles, 14 / 23 at 6,518, 22 / 22 at 22,279, 33 / 27
+// at 45,203; 3D 52 / 88 at 33,123, 83 / 82 at 62,721, 216 / 119 at 165,888.
+template <int D>
+constexpr int kWinLanesMax = D == 2 ? 20000 : 60000;
 
 // The 2D window search pass with search action `act` (CPCount: lists and nCount only).
 template <class Act>
 int launch_win_build(epp_ctx* ctx, int set, int crit, const Act& act, unsigned long long* pairs) {
     PairArgs A = pair_args(ctx, set, crit);
     TileMask M{ctx->cap, ctx->nlist};
-    if (ctx->n <= kWinLanesMax)
-        k_win_lanes<Act, 8><<<blocks_for((long long)ctx->n * 8, ctx->pass_threads), ctx->pass_threads, 0, ctx->stream>>>(
+    if (ctx->n <= kWinLanesMax<2>)
+        k_win_lanes<2, Act, 8><<<blocks_for((long long)ctx->n * 8, ctx->pass_threads), ctx->pass_threads, 0, ctx->stream>>>(
             A, M, act, pairs);
     else
         k_win_build<Act><<<blocks_for(ctx->n, ctx->pass_threads), ctx->pass_threads, 0, ctx->stream>>>(A, M, act, pairs);
@@ -423,7 +424,15 @@ int launch_build(epp_ctx* ctx, int set, int crit, unsigned long long* pairs) {
     }
     PairArgs A = pair_args(ctx, set, crit);
     TileMask M{ctx->cap, ctx->nlist};
-    k_build<D><<<blocks_for(ctx->n, ctx->pass_threads), ctx->pass_threads, 0, ctx->stream>>>(A, M, ctx->ncnt[set], pairs);
+    const int T = ctx->pass_threads;
+    if constexpr (D == 2) {
+        k_build<<<blocks_for(ctx->n, T), T, 0, ctx->stream>>>(A, M, ctx->ncnt[set], pairs);
+    } else if (ctx->n <= kWinLanesMax<3>) {
+        k_win_lanes<3, CPCount<3>, 8><<<blocks_for((long long)ctx->n * 8, T), T, 0, ctx->stream>>>(
+            A, M, CPCount<3>{ctx->ncnt[set]}, pairs);
+    } else {
+        k_win_build3<<<blocks_for(ctx->n, T), T, 0, ctx->stream>>>(A, M, ctx->ncnt[set], pairs);
+    }
     CK_LAUNCH();
     return EPP_OK;
 }

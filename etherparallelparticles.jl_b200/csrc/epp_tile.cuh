@@ -102,7 +102,9 @@ struct ListWriter {
     int cap;
     int b0, b1, b2;
     __device__ __forceinline__ void put(int cnt, int j) {
-        if (cnt >= ListConf<D>::LCAP) return;
+        if (cnt < ListConf<D>::LCAP) put_room(cnt, j);
+    }
+    __device__ __forceinline__ void put_room(int cnt, int j) {   // cnt < LCAP
         if (!ListConf<D>::ROW) {   // column-major: base advances one column per entry
             *base = j;
             base += cap;
@@ -232,7 +234,7 @@ __device__ __forceinline__ int lane_stencil_list(const PairArgs& A, ListWriter<D
     return cnt;
 }
 
-// The search pass: neighbour lists and nCount.  Each chunk of 32 candidates of the warp's union
+// The 2D search pass of EPP_TUNING_LISTS: neighbour lists and nCount.  Each chunk of 32 candidates of the warp's union
 // is staged in shared memory (position and index, one coalesced load per lane; the next chunk's
 // loads are issued before the current chunk is tested); every lane tests all 32 against its own
 // particle in lockstep with the reference's IEEE criterion.  A chunk whose candidates share one
@@ -240,11 +242,10 @@ __device__ __forceinline__ int lane_stencil_list(const PairArgs& A, ListWriter<D
 // other chunks look the bound up per candidate.  One ballot per tag gives the chunk's candidates
 // of each tag, so a lane keeps only the pairs its row of the active-pair matrix allows, then
 // appends them to its list in candidate order.
-template <int D>
-__global__ void __launch_bounds__(128, D == 2 ? 8 : 6)
+__global__ void __launch_bounds__(128, 8)
     k_build(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M, int* ncount,
             unsigned long long* pairs) {
-    __shared__ __align__(16) float s_p[4][4][32];   // staged x, y, z, h of a chunk (per warp)
+    __shared__ __align__(16) float s_p[4][3][32];   // staged x, y, h of a chunk (per warp)
     __shared__ int s_j[4][32];
     const int lane = threadIdx.x & 31;
     const int wib = threadIdx.x >> 5;
@@ -262,7 +263,7 @@ __global__ void __launch_bounds__(128, D == 2 ? 8 : 6)
         // tile mode: the warp's cells lie in one cell row (all but the ~2% of warps that cross
         // a row end); otherwise every lane uses its own stencil
         const bool tiled = r1 == r0;
-        TileRanges<D> R;
+        TileRanges<2> R;
         R.n = 0;
         R.total = 0;
         if (tiled) {
@@ -276,18 +277,18 @@ __global__ void __launch_bounds__(128, D == 2 ? 8 : 6)
         const bool valid = on && ti >= 1 && ti <= A.n_tags;
         unsigned st = 0;
         if (on && !valid) st |= EPP_STATUS_BAD_TAG;
-        const TargetConst tc = target_const<D>(on ? xi.w : 1.0f);
+        const TargetConst tc = target_const<2>(on ? xi.w : 1.0f);
         const unsigned amask = valid ? A.adj[ti - 1] : 0u;
-        ListWriter<D> L = list_writer<D>(M, min(i, n_alive - 1));
+        ListWriter<2> L = list_writer<2>(M, min(i, n_alive - 1));
         if (!tiled) {
-            if (valid) cnt = lane_stencil_list<D>(A, L, R, i, xi, ti, tc.h2sq, st);
+            if (valid) cnt = lane_stencil_list<2>(A, L, R, i, xi, ti, tc.h2sq, st);
         } else {
             const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
             float hc_h = xi.w;   // exact bound of the last h_j seen
             float hc_r2 = dflt ? A.dom.gap_square : tc.h2sq;
             const int nchunk = (R.total + 31) >> 5;
             // this lane's own particle in the union: the middle stencil row holds it
-            constexpr int RMID = D == 3 ? 4 : 1;
+            constexpr int RMID = 1;
             const int k_self = on ? R.cum[RMID] + (i - R.lo[RMID]) : -1;
             // chunk 0 in flight
             bool real = lane < R.total;
@@ -299,8 +300,7 @@ __global__ void __launch_bounds__(128, D == 2 ? 8 : 6)
                 // padding past the last candidate is far away: it fails every test
                 s_p[wib][0][lane] = xn.x;
                 s_p[wib][1][lane] = xn.y;
-                s_p[wib][2][lane] = xn.z;
-                s_p[wib][3][lane] = xn.w;
+                s_p[wib][2][lane] = xn.w;
                 s_j[wib][lane] = list_entry(jn, tn);   // appended as is (a real, allowed tag)
                 const int tj = tn;
                 const bool real_c = real;
@@ -334,11 +334,10 @@ __global__ void __launch_bounds__(128, D == 2 ? 8 : 6)
                     // a funnel shift moves that sign bit into the chunk's word (candidate 0 ends in
                     // the top bit, where the append loop below starts)
                     const int nR2 = -__float_as_int(hc_r2) - 1;
-                    // two candidates per packed sub / mul; dr2 = (dx dx + dy dy) + dz dz, IEEE
-                    const f32x2 XI = f2_pack(xi.x, xi.x), YI = f2_pack(xi.y, xi.y), ZI = f2_pack(xi.z, xi.z);
+                    // two candidates per packed sub / mul; dr2 = dx dx + dy dy, IEEE
+                    const f32x2 XI = f2_pack(xi.x, xi.x), YI = f2_pack(xi.y, xi.y);
                     const f32x2* px = reinterpret_cast<const f32x2*>(s_p[wib][0]);
                     const f32x2* py = reinterpret_cast<const f32x2*>(s_p[wib][1]);
-                    const f32x2* pz = reinterpret_cast<const f32x2*>(s_p[wib][2]);
 #pragma unroll
                     for (int b = 0; b < 16; ++b) {
                         const f32x2 dx = f2_sub(XI, px[b]);
@@ -347,27 +346,16 @@ __global__ void __launch_bounds__(128, D == 2 ? 8 : 6)
                         f2_unpack(f2_mul(dx, dx), x0, x1);
                         f2_unpack(f2_mul(dy, dy), y0, y1);
                         float d0 = __fadd_rn(x0, y0), d1 = __fadd_rn(x1, y1);
-                        if (D == 3) {
-                            const f32x2 dz = f2_sub(ZI, pz[b]);
-                            float z0, z1;
-                            f2_unpack(f2_mul(dz, dz), z0, z1);
-                            d0 = __fadd_rn(d0, z0);
-                            d1 = __fadd_rn(d1, z1);
-                        }
                         word = __funnelshift_l((unsigned)(__float_as_int(d0) + nR2), word, 1);
                         word = __funnelshift_l((unsigned)(__float_as_int(d1) + nR2), word, 1);
                     }
                 } else {
 #pragma unroll 8
                     for (int b = 0; b < 32; ++b) {
-                        const float4 xj = make_float4(s_p[wib][0][b], s_p[wib][1][b], s_p[wib][2][b], s_p[wib][3][b]);
+                        const float4 xj = make_float4(s_p[wib][0][b], s_p[wib][1][b], 0.0f, s_p[wib][2][b]);
                         const float dx = __fsub_rn(xi.x, xj.x);
                         const float dy = __fsub_rn(xi.y, xj.y);
                         float dr2 = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-                        if (D == 3) {
-                            const float dz = __fsub_rn(xi.z, xj.z);
-                            dr2 = __fadd_rn(dr2, __fmul_rn(dz, dz));
-                        }
                         if (xj.w != hc_h) {
                             hc_h = xj.w;
                             hc_r2 = dflt ? A.dom.gap_square : xj.w == xi.w ? tc.h2sq : pair_r2(xi.w, xj.w);

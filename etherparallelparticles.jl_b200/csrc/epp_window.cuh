@@ -29,16 +29,22 @@
 
 namespace epp {
 
+// A bound b on dr2 for the integer test bits(dr2) + accept_bias(b) < 0 <=> dr2 <= b: non-negative
+// floats order like their bit patterns.  A NaN bound accepts nothing.
+__device__ __forceinline__ int accept_bias(float b) { return b >= 0.0f ? -__float_as_int(b) - 1 : 0; }
+
 struct RowWin {
     int lo, hi;   // candidate range [lo, hi) in cell order
 };
 
-// Linear cell row of stencil row r (0, 1, 2 for dy = -1, 0, +1) of the cell row `rid` = y + n1 k
-// (k is the instance of a batch; the caller passes y = rid mod n1), or -1 when y + dy is outside
-// the grid.
-__device__ __forceinline__ int stencil_row2(const PairArgs& A, int rid, int y, int r) {
-    const int yy = y + r - 1;
-    return (yy >= 0 && yy < A.dom.n[1]) ? rid + r - 1 : -1;
+// Linear cell row of stencil row r of the cell row rid = y + n1 z, or -1 outside the grid.  2D: r =
+// 0, 1, 2 for dy = -1, 0, +1 (z is the instance of a batch, never crossed); 3D: r = 3 (dz + 1) + dy + 1.
+template <int D>
+__device__ __forceinline__ int stencil_row(const PairArgs& A, int rid, int y, int z, int r) {
+    const int yy = y + (D == 3 ? r % 3 : r) - 1, dz = D == 3 ? r / 3 - 1 : 0;
+    if (yy < 0 || yy >= A.dom.n[1]) return -1;
+    if (D == 3 && (z + dz < 0 || z + dz >= A.dom.n[2])) return -1;
+    return rid + yy - y + (D == 3 ? A.dom.n[1] * dz : 0);
 }
 
 // Candidates of cells xa .. xb (clamped to the grid) of linear cell row `row` (-1: none).
@@ -76,9 +82,7 @@ __device__ __forceinline__ unsigned window_bits(const float4* sx, int off, int l
     const f32x2 XY = f2_pack(xi.x, xi.y);
     unsigned word = 0u;
     if (one) {
-        // dr2 <= R2 as integers: non-negative floats order like their bit patterns, so
-        // bits(dr2) - bits(R2) - 1 is negative exactly for the accepted candidates
-        const int nR2 = -__float_as_int(own) - 1;
+        const int nR2 = accept_bias(own);
 #pragma unroll 4
         for (int k = len - 1; k >= 0; --k) {
             const f32x2 d = f2_sub(XY, *reinterpret_cast<const f32x2*>(&sx[off + k]));
@@ -113,23 +117,26 @@ struct WinOut {
 // neighbourhoods only (a window beyond 32 candidates, or windows beyond the staging area).  Inlined:
 // as an out-of-line call it cost the kernel registers (the values live across the call) and 13% of
 // its time.
-template <class Act>
-__device__ __forceinline__ WinOut win_lane_general(const PairArgs& A, const TileMask& M, const Act& act, RowWin w0, RowWin w1,
-                                                RowWin w2, int i, int ti, float4 xi, unsigned amask) {
-    const TargetConst tc = target_const<2>(xi.w);
+template <int D, class Act>
+__device__ __forceinline__ WinOut win_lane_general(const PairArgs& A, const TileMask& M, const Act& act,
+                                                const RowWin (&win)[D == 3 ? 9 : 3], int i, int ti, float4 xi, unsigned amask) {
+    const TargetConst tc = target_const<D>(xi.w);
     const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
     typename Act::Self me = act.self(i);
-    ListWriter<2> L = list_writer<2>(M, i);
+    ListWriter<D> L = list_writer<D>(M, i);
     WinOut o{0, 0.0f, 0.0f};
     float ho = xi.w, ro = dflt ? A.dom.gap_square : tc.h2sq;
 #pragma unroll 1
-    for (int r = 0; r < 3; ++r) {
-        const int lo = r == 0 ? w0.lo : r == 1 ? w1.lo : w2.lo, hi = r == 0 ? w0.hi : r == 1 ? w1.hi : w2.hi;
+    for (int r = 0; r < (D == 3 ? 9 : 3); ++r) {
+        int lo = 0, hi = 0;
+#pragma unroll
+        for (int q = 0; q < (D == 3 ? 9 : 3); ++q)
+            if (q == r) lo = win[q].lo, hi = win[q].hi;
 #pragma unroll 1
         for (int j = lo; j < hi; ++j) {
             const float4 xj = A.s.xh[j];
             const int tj = tag_of(A.s.tagm[j]);
-            const PairGeo g = geometry<2>(xi, xj);
+            const PairGeo g = geometry<D>(xi, xj);
             if (xj.w != ho) {
                 ho = xj.w;
                 ro = dflt ? A.dom.gap_square : ho == xi.w ? tc.h2sq : pair_r2(xi.w, ho);
@@ -167,7 +174,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
         const int c = A.s.cell[min(i, n_alive - 1)];
         EPP_CHECK(!__any_sync(FULL, c < 0 || c >= A.dom.n_cells), 34, c);
         const int rid = A.dom.by[0].div(max(c, 0)), cx = c - rid * A.dom.n[0];
-        const int y = rid - A.dom.by[1].div(rid) * A.dom.n[1];
+        const int z = A.dom.by[1].div(rid), y = rid - z * A.dom.n[1];
         const float4 xi = on ? A.s.xh[i] : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
         const int ti = on ? tag_of(A.s.tagm[i]) : 0;
         const bool valid = on && ti >= 1 && ti <= A.n_tags;
@@ -175,7 +182,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
         const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
         RowWin win[3];
 #pragma unroll
-        for (int r = 0; r < 3; ++r) win[r] = row_range(A, stencil_row2(A, rid, y, r), cx - 1, cx + 1);
+        for (int r = 0; r < 3; ++r) win[r] = row_range(A, stencil_row<2>(A, rid, y, z, r), cx - 1, cx + 1);
         // a part ends at the end of a cell row and where the next lane's windows do not meet this one's:
         // what lies between (the floor under a gap of the fluid) is nobody's candidate
         const int rid_p = __shfl_up_sync(FULL, rid, 1), cx_p = __shfl_up_sync(FULL, cx, 1);
@@ -244,7 +251,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
             // windows of up to 40: the lanes of the pass then take each row in two words, one after the other
             const bool two = __any_sync(__activemask(), staged && longest > 32);
             if (!staged || longest > 64) {
-                const WinOut o = win_lane_general<Act>(A, M, act, win[0], win[1], win[2], i, ti, xi, amask);
+                const WinOut o = win_lane_general<2, Act>(A, M, act, win, i, ti, xi, amask);
                 cnt = o.cnt;
                 sum.x = o.sx;
                 sum.y = o.sy;
@@ -324,6 +331,215 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
     count_pairs(pairs, cnt);
 }
 
+// The 3D search pass: neighbour lists and nCount.  Windows as in 2D, nine stencil rows of about 53
+// candidates at h = 1.3 dx, one plane (three rows) staged at a time; a particle's 480 candidates are
+// tested by its own lane.  It replaces a lockstep search of the warp's whole union of stencils (about
+// 700 candidates, 32 at a time, with a divergent append after each chunk): 574 -> 387 us at 955,668
+// particles, 182 -> 119 at 165,888.  Issue-bound (79% of the slots): about half on the tests, 40% on the
+// walk over their bits, which is why a word whose candidates have one tag computes its entries and
+// checks the list's capacity once.  Warps near walls stage two h's and take the two bounds by a select.
+// When one particle's plane is longer than the staging area (dense neighbourhoods) the rows go one by
+// one, and a row beyond it is read from global memory.  One warp per cell, its lanes on the candidates
+// and ballots in place of the walk, measured 528 us: two POPC per target and chunk, no fewer
+// instructions.
+constexpr int kStage3 = 320;   // staged candidates per warp: 7 blocks of 128 threads fit an SM
+
+struct Stage3 {
+    float4 x[kStage3];   // (x, y, z, h)
+    int e[kStage3];      // list entry (index and tag)
+};
+
+// Acceptance bits of `len` <= 32 staged candidates from slot `off`, candidate 0 in the top bit; see
+// window_bits.  HS = 1: one exact bound (its bias nA) for all; 2: candidates of h == hA take nA, the
+// others, all of one other h, nB (fluid and walls); 3: any h, nO for the lane's own, the bias of the
+// last other one kept in (ho, no).
+template <int HS>
+__device__ __forceinline__ unsigned window_bits3(const float4* sx, int off, int len, float4 xi, int nA, float hA, int nB,
+                                                 int nO, float& ho, int& no) {
+    const f32x2 XY = f2_pack(xi.x, xi.y);
+    unsigned word = 0u;
+#pragma unroll 4
+    for (int k = 0; k < len; ++k) {
+        const float4 c = sx[off + k];
+        const f32x2 d = f2_sub(XY, f2_pack(c.x, c.y));
+        float ex, ey;
+        f2_unpack(f2_mul(d, d), ex, ey);
+        const float dz = __fsub_rn(xi.z, c.z);
+        const float dr2 = __fadd_rn(__fadd_rn(ex, ey), __fmul_rn(dz, dz));
+        int n = nA;
+        if (HS == 2) n = c.w == hA ? nA : nB;
+        if (HS == 3) {
+            if (c.w != ho) {
+                ho = c.w;
+                no = ho == xi.w ? nO : accept_bias(pair_r2(xi.w, ho));
+            }
+            n = no;
+        }
+        word = __funnelshift_l((unsigned)(__float_as_int(dr2) + n), word, 1);
+    }
+    return len < 32 ? word << (32 - len) : word;
+}
+
+__global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M,
+                                                       int* ncount, unsigned long long* pairs) {
+    __shared__ Stage3 stage[4];
+    constexpr unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    Stage3& S = stage[threadIdx.x >> 5];
+    const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int w0 = i - lane;
+    int cnt = 0;
+    if (w0 < n_alive) {   // warp-uniform
+        const bool on = i < n_alive;
+        const int c = A.s.cell[min(i, n_alive - 1)];
+        EPP_CHECK(!__any_sync(FULL, c < 0 || c >= A.dom.n_cells), 36, c);
+        const int rid = A.dom.by[0].div(max(c, 0)), cx = c - rid * A.dom.n[0];
+        const int z = A.dom.by[1].div(rid), y = rid - z * A.dom.n[1];
+        const float4 xi = on ? A.s.xh[i] : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+        const int ti = on ? tag_of(A.s.tagm[i]) : 0;
+        const bool valid = on && ti >= 1 && ti <= A.n_tags;
+        const unsigned amask = valid ? A.adj[ti - 1] : 0u;   // bits of valid tags only
+        const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
+        const float own = dflt ? A.dom.gap_square : target_const<3>(xi.w).h2sq;
+        ListWriter<3> L = list_writer<3>(M, min(i, n_alive - 1));
+        // parts as in the 2D pass: they end with a cell row and at a gap of it
+        const int rid_p = __shfl_up_sync(FULL, rid, 1), cx_p = __shfl_up_sync(FULL, cx, 1);
+        const unsigned starts = __ballot_sync(FULL, lane == 0 || rid != rid_p || cx - cx_p > 3);
+        const unsigned alive = __ballot_sync(FULL, on);
+        int rows = 3;
+        for (int r0 = 0; r0 < 9; r0 += rows) {   // warp-uniform
+            RowWin win[3];
+            int mine = 0;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                win[q] = q < rows ? row_range(A, stencil_row<3>(A, rid, y, z, r0 + q), cx - 1, cx + 1) : RowWin{0, 0};
+                mine += win[q].hi - win[q].lo;
+            }
+            if (rows == 3 && __any_sync(FULL, mine > kStage3)) {   // from here on one row at a time
+                rows = 1;
+                win[1] = win[2] = RowWin{0, 0};
+            }
+            unsigned pending = alive;
+            while (pending) {   // warp-uniform: a pass over as many parts as the staging area holds
+                const int head = __ffs(pending) - 1;
+                const float hw = __shfl_sync(FULL, xi.w, head);
+                const int tw = __shfl_sync(FULL, ti, head);
+                bool same_t = true, staged = false;
+                bool other = false, two_h = true;   // an h other than hw was staged by this lane; one such h only
+                float hb = hw;
+                int used = 0, off[3] = {0, 0, 0};
+                unsigned taken = 0u;
+                __syncwarp();
+                while (pending) {
+                    const int lead = __ffs(pending) - 1;
+                    const unsigned after = starts & ~((2u << lead) - 1u);   // part starts behind the lead
+                    int last = min(after ? __ffs(after) - 2 : 31, 31 - __clz(pending));
+                    int lo[3], len[3], total;
+                    for (;;) {
+                        total = 0;
+#pragma unroll
+                        for (int q = 0; q < 3; ++q) {
+                            lo[q] = __shfl_sync(FULL, win[q].lo, lead);
+                            len[q] = max(__shfl_sync(FULL, win[q].hi, last) - lo[q], 0);
+                            total += len[q];
+                        }
+                        if (total <= kStage3 - used || used > 0 || last == lead) break;
+                        last = lead + (last - lead) / 2;
+                    }
+                    if (total > kStage3 - used) {
+                        if (used > 0) break;   // next pass
+                        taken = 1u << lead;    // one lane's row is too long: read from global memory
+                        pending &= ~taken;
+                        break;
+                    }
+                    for (int k = lane; k < total; k += 32) {
+                        const int j = k < len[0] ? lo[0] + k
+                                                 : k < len[0] + len[1] ? lo[1] + (k - len[0]) : lo[2] + (k - len[0] - len[1]);
+                        float4 xj = A.s.xh[j];
+                        const int tj = tag_of(A.s.tagm[j]);
+                        const bool bad = tj < 1 || tj > A.n_tags;   // never a neighbour: fails every test
+                        if (bad) xj.x = __int_as_float(0x7fffffff);
+                        S.x[used + k] = xj;
+                        S.e[used + k] = list_entry(j, bad ? 1 : tj);
+                        if (xj.w != hw) {
+                            two_h = two_h && (!other || hb == xj.w);
+                            other = true;
+                            hb = xj.w;
+                        }
+                        same_t = same_t && tj == tw;
+                    }
+                    const unsigned part = ((2u << last) - 1u) & ~((1u << lead) - 1u);
+                    if ((part >> lane) & 1u) {
+                        staged = true;
+                        off[0] = used + win[0].lo - lo[0];
+                        off[1] = used + len[0] + win[1].lo - lo[1];
+                        off[2] = used + len[0] + len[1] + win[2].lo - lo[2];
+                    }
+                    used += total;
+                    taken |= part;
+                    pending &= ~part;
+                }
+                const unsigned others = __ballot_sync(FULL, other);
+                const float h2 = __shfl_sync(FULL, hb, others ? __ffs(others) - 1 : 0);   // the other h, if any
+                two_h = __all_sync(FULL, two_h && (!other || hb == h2));
+                same_t = __all_sync(FULL, same_t);
+                __syncwarp();
+                if (!(((taken >> lane) & 1u) && valid)) continue;
+                if (same_t && staged && !((amask >> (tw - 1)) & 1u)) continue;   // walls among walls
+                // exact bounds of this lane against hw and the other h, as window_bits3 takes them
+                const int hs = dflt || !others ? 1 : two_h ? 2 : 3;   // warp-uniform
+                const int nO = accept_bias(own);
+                const int nA = dflt || xi.w == hw ? nO : accept_bias(pair_r2(xi.w, hw));
+                const int nB = hs == 1 || xi.w == h2 ? nO : accept_bias(pair_r2(xi.w, h2));
+                float ho = xi.w;
+                int no = nO;
+#pragma unroll 1
+                for (int q = 0; q < rows; ++q) {
+                    const int lo = q == 0 ? win[0].lo : q == 1 ? win[1].lo : win[2].lo;
+                    const int n = (q == 0 ? win[0].hi : q == 1 ? win[1].hi : win[2].hi) - lo;
+                    const int o = q == 0 ? off[0] : q == 1 ? off[1] : off[2];
+                    const int self = r0 + q == 4 ? i - lo : -1;   // not its own neighbour
+                    if (!staged) {
+                        for (int k = 0; k < n; ++k) {
+                            const int j = lo + k;
+                            unsigned st = 0u;
+                            if (accept<3>(A, i, xi, amask, own, j, A.s.xh[j], st)) L.put(cnt++, list_entry(j, tag_of(A.s.tagm[j])));
+                        }
+                        continue;
+                    }
+                    for (int k0 = 0; k0 < n; k0 += 32) {
+                        const int len = min(n - k0, 32);
+                        unsigned word = hs == 1   ? window_bits3<1>(S.x, o + k0, len, xi, nA, hw, nB, nO, ho, no)
+                                        : hs == 2 ? window_bits3<2>(S.x, o + k0, len, xi, nA, hw, nB, nO, ho, no)
+                                                  : window_bits3<3>(S.x, o + k0, len, xi, nA, hw, nB, nO, ho, no);
+                        if ((self >> 5) == (k0 >> 5)) word &= ~(0x80000000u >> (self & 31));
+                        if (same_t && cnt + 32 <= ListConf<3>::LCAP) {   // entries from their index, room for all
+                            const int e0 = list_entry(lo + k0, tw);
+                            while (word) {
+                                const int b = __clz(word);
+                                word ^= 0x80000000u >> b;
+                                L.put_room(cnt++, e0 + b);
+                            }
+                            continue;
+                        }
+                        while (word) {
+                            const int b = __clz(word);
+                            word ^= 0x80000000u >> b;
+                            const int e = S.e[o + k0 + b];
+                            if ((amask >> (entry_tag(e) - 1)) & 1u) L.put(cnt++, e);   // the active-pair matrix
+                        }
+                    }
+                }
+            }
+        }
+        L.flush(cnt);
+        if (on) ncount[i] = cnt;
+        if (on && !valid) atomicOr(A.status, EPP_STATUS_BAD_TAG);
+    }
+    count_pairs(pairs, cnt);
+}
+
 // The same pass for small systems: L lanes per particle, candidates straight from global memory, so a
 // particle's walk is L times shorter.  Lane g tests candidates g, g + L, ... of each window (four loads
 // in flight); a ballot of the group gives each accepted one its place in the list, kept in shared
@@ -331,11 +547,11 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
 // the first lane adds the terms in list order: lists, counts and sums have the bits of k_win_build.  A
 // particle with more neighbours than a list keeps goes through the general per-lane search.  It issues
 // four times k_win_build's instructions per particle (383 against 93) but a fifth of them one after
-// the other: 12 us against 25 at 1,418 particles, 22 each at 22,279.
-template <class Act, int L>
+// the other: 12 us against 25 at 1,418 particles, 22 each at 22,279; 3D 52 against 88 at 33,123.
+template <int D, class Act, int L>
 __global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M,
                                                    const __grid_constant__ Act act, unsigned long long* pairs) {
-    constexpr int P = 128 / L, CAP = ListConf<2>::LCAP;
+    constexpr int P = 128 / L, CAP = ListConf<D>::LCAP, NR = D == 3 ? 9 : 3;
     __shared__ int s_e[P][CAP + 1];                           // accepted entries (odd rows: no bank conflicts)
     __shared__ float s_t[Act::NC != 0 ? P : 1][CAP + 1];      // their terms
     const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
@@ -356,18 +572,18 @@ __global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairA
         } else {
             EPP_CHECK(c >= 0 && c < A.dom.n_cells, 35, c);
             const int rid = A.dom.by[0].div(c), cx = c - rid * A.dom.n[0];
-            const int y = rid - A.dom.by[1].div(rid) * A.dom.n[1];
-            RowWin win[3];
+            const int z = A.dom.by[1].div(rid), y = rid - z * A.dom.n[1];
+            RowWin win[NR];
 #pragma unroll
-            for (int r = 0; r < 3; ++r) win[r] = row_range(A, stencil_row2(A, rid, y, r), cx - 1, cx + 1);
+            for (int r = 0; r < NR; ++r) win[r] = row_range(A, stencil_row<D>(A, rid, y, z, r), cx - 1, cx + 1);
             const unsigned amask = A.adj[ti - 1];   // bits of valid tags only
             const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
-            const TargetConst tc = target_const<2>(xi.w);
+            const TargetConst tc = target_const<D>(xi.w);
             const float r2own = dflt ? A.dom.gap_square : tc.h2sq;
             const f32x2 XI = f2_pack(xi.x, xi.y);
             float ho = xi.w, ro = r2own;   // the bound of the last h_j seen
 #pragma unroll
-            for (int r = 0; r < 3; ++r) {
+            for (int r = 0; r < NR; ++r) {
                 for (int j0 = win[r].lo; j0 < win[r].hi; j0 += 4 * L) {
                     float4 xj[4];
                     int tm[4];
@@ -388,11 +604,16 @@ __global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairA
                         float ex, ey;
                         const f32x2 d = f2_sub(XI, f2_pack(xj[q].x, xj[q].y));
                         f2_unpack(f2_mul(d, d), ex, ey);
+                        float dr2 = __fadd_rn(ex, ey);
+                        if (D == 3) {
+                            const float dz = __fsub_rn(xi.z, xj[q].z);
+                            dr2 = __fadd_rn(dr2, __fmul_rn(dz, dz));
+                        }
                         if (xj[q].w != ho) {
                             ho = xj[q].w;
                             ro = dflt || ho == xi.w ? r2own : pair_r2(xi.w, ho);
                         }
-                        const bool ok = __fadd_rn(ex, ey) <= ro && (__funnelshift_rc(amask, 0u, (unsigned)(tm[q] - 1)) & 1u);
+                        const bool ok = dr2 <= ro && (__funnelshift_rc(amask, 0u, (unsigned)(tm[q] - 1)) & 1u);
                         const unsigned hits = (__ballot_sync(group, ok) >> first) & ((1u << L) - 1u);
                         const int at = cnt + __popc(hits & ((1u << g) - 1u));
                         if (ok && at < CAP) s_e[p][at] = list_entry(j0 + q * L + g, tm[q]);
@@ -403,7 +624,7 @@ __global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairA
             float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             if (cnt > CAP) {
                 if (g == 0) {
-                    const WinOut o = win_lane_general<Act>(A, M, act, win[0], win[1], win[2], i, ti, xi, amask);
+                    const WinOut o = win_lane_general<D, Act>(A, M, act, win, i, ti, xi, amask);
                     sum.x = o.sx;
                     sum.y = o.sy;
                 }
@@ -413,11 +634,12 @@ __global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairA
 #pragma unroll 2
                 for (int k = g; k < cnt; k += L) {
                     const int e = s_e[p][k], j = entry_index(e), tj = entry_tag(e);
-                    M.list[(size_t)k * M.cap + i] = e;
+                    if (D == 3) M.list[(size_t)i * CAP + k] = e;
+                    else M.list[(size_t)k * M.cap + i] = e;
                     if constexpr (Act::NC != 0) {
                         const float4 xj = A.s.xh[j];
                         const typename Act::Nb nb = act.fetch(j, ti, tj);
-                        s_t[p][k] = act.term(me, nb, ti, tj, xj, geometry<2>(xi, xj), tc).x;
+                        s_t[p][k] = act.term(me, nb, ti, tj, xj, geometry<D>(xi, xj), tc).x;
                     }
                 }
                 if constexpr (Act::NC != 0) {

@@ -148,3 +148,43 @@ def test_fast_division(d):
     for x in (int(x) for x in v):
         q = x if m == 0 else ((x * m) >> 32) >> s
         assert q == x // d, (x, d)
+
+
+# 3D search: eight lanes per particle (small system) and staged planes (beyond 60,000 particles), with
+# one h, the two of fluid and walls, and three mixed at random; h = 2.5 dx takes rows one by one.  The
+# neighbour counts are the oracle's.
+@pytest.mark.gpu
+@pytest.mark.parametrize("dx,column,h_factor,kinds", [
+    (0.05, (1.0, 1.0, 0.6), 1.3, 1), (0.05, (0.93, 1.0, 0.57), 1.3, 3), (0.0262, (1.0, 1.0, 0.61), 1.3, 2),
+    (0.0262, (1.0, 1.0, 0.61), 1.3, 3), (0.03, (1.0, 1.0, 0.6), 2.5, 1)])
+def test_3d_search_variants_count_the_oracles_neighbours(dx, column, h_factor, kinds):
+    from oracle_lib import Oracle
+    c = casegen.dam_break_3d(dx=dx, column=column, h_factor=h_factor, max_neighbour_number=700)
+    stir(c, 11)
+    if kinds == 3:   # smaller h only: every neighbour stays inside the 27 cells
+        rng = np.random.default_rng(2)
+        c.ps["H"] = (c.ps["H"] * rng.choice([1.0, 0.93, 0.8], c.n)).astype(np.float32)
+    elif kinds == 2:
+        c.ps["H"] = np.where(c.ps["Tag"] == casegen.WALL_TAG, c.ps["H"] * np.float32(0.9), c.ps["H"]).astype(np.float32)
+    d = device(c, max_nb=700)
+    cfg = type(d.config).from_buffer_copy(d.config)
+    cfg.max_cell_particles = 400
+    o = Oracle(cfg, 32)
+    o.upload(c.n, c.ps.is_alive, c.ps.cell_index, c.ps.int_properties, c.ps.float_properties, d.cmap)
+    o.search(SYM, CONT, c.physics)
+    d.ctx.search(SYM, CONT, c.physics, 0)
+    d.ctx.synchronize()
+    cnt, ids = d.ctx.neighbour_lists(c.n, 160)
+    want = o.field(9, 0, c.n).astype(np.int32)
+    assert np.array_equal(cnt, want)
+    kept = cnt <= 160
+    assert np.array_equal((ids[kept] > 0).sum(1), cnt[kept])
+    x = c.ps["PositionVec"].astype(np.float64)
+    h = c.ps["H"].astype(np.float64)
+    rows = np.random.default_rng(3).choice(np.flatnonzero(kept & (cnt > 0)), 500)
+    for i in rows:   # the stored neighbours are distinct, not itself, and inside the support
+        j = ids[i][ids[i] > 0] - 1
+        assert len(set(j.tolist())) == len(j) and i not in j
+        assert np.all(np.linalg.norm(x[j] - x[i], axis=1) <= 4 * h[i] * h[j] / (h[i] + h[j]) * (1 + 1e-6))
+    assert o.status() & abi.EPP_STATUS_CELL_OVERFLOW == 0
+    d.close()
