@@ -245,6 +245,37 @@ void dev_free(epp_ctx* ctx, T*& p) {
     p = nullptr;
 }
 
+// Copies between columns of n values of the staging arrays and of the caller's matrices (4-byte
+// values, device columns n apart, host columns ld apart).  Consecutive columns whose neighbours follow
+// each other on both sides travel in one copy when the host matrix has no rows between them (ld == n):
+// a copy costs about 4 us to start, and the neighbour columns of a read-back are 350 of them.
+struct ColumnCopies {
+    cudaStream_t stream;
+    size_t n;
+    int64_t ld;
+    cudaMemcpyKind kind;
+    char* dev = nullptr;    // the pending run
+    char* host = nullptr;
+    size_t cols = 0;
+    cudaError_t err = cudaSuccess;
+    void flush() {
+        if (cols > 0 && err == cudaSuccess)
+            err = kind == cudaMemcpyHostToDevice ? cudaMemcpyAsync(dev, host, cols * n * 4, kind, stream)
+                                                 : cudaMemcpyAsync(host, dev, cols * n * 4, kind, stream);
+        cols = 0;
+    }
+    void add(const void* d, const void* h) {
+        char* dd = (char*)d;
+        char* hh = (char*)h;
+        if (cols > 0 && !((size_t)ld == n && dd == dev + cols * n * 4 && hh == host + cols * n * 4)) flush();
+        if (cols == 0) {
+            dev = dd;
+            host = hh;
+        }
+        ++cols;
+    }
+};
+
 // Cells of the grid (all instances) of a configuration: EPP_OK, or the status that rejects it.
 int plan_cells(const epp_config* cfg, DevDomain& d) {
     const int n_inst = cfg->n_instances > 1 ? cfg->n_instances : 1;
@@ -1234,26 +1265,19 @@ int32_t epp_upload(epp_ctx* ctx, int32_t n, const int32_t* is_alive, const int32
         ctx->searched = false;
         return EPP_OK;
     }
-    auto fcol = [&](int stage_col, int user_col, int width, float fill) -> int {
+    ColumnCopies fc{ctx->stream, (size_t)n, ldf, cudaMemcpyHostToDevice}, ic{ctx->stream, (size_t)n, ldi, cudaMemcpyHostToDevice};
+    auto fcol = [&](int stage_col, int user_col, int width) -> int {
         for (int k = 0; k < width; ++k) {
             float* dst = ctx->stage_f + (size_t)(stage_col + k) * n;
-            if (user_col >= 0) {
-                CK(cudaMemcpyAsync(dst, fp + (size_t)(user_col + k) * ldf, (size_t)n * 4,
-                                   cudaMemcpyHostToDevice, ctx->stream));
-            } else if (fill == 0.0f) {
-                CK(cudaMemsetAsync(dst, 0, (size_t)n * 4, ctx->stream));
-            } else {
-                std::vector<float> h(n, fill);
-                CK(cudaMemcpyAsync(dst, h.data(), (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-                CK(cudaStreamSynchronize(ctx->stream));
-            }
+            if (user_col >= 0) fc.add(dst, fp + (size_t)(user_col + k) * ldf);
+            else CK(cudaMemsetAsync(dst, 0, (size_t)n * 4, ctx->stream));
         }
         return EPP_OK;
     };
     auto icol = [&](int stage_col, const int32_t* src, int fill) -> int {
         int* dst = ctx->stage_i + (size_t)stage_col * n;
         if (src) {
-            CK(cudaMemcpyAsync(dst, src, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
+            ic.add(dst, src);
         } else if (fill == 0) {
             CK(cudaMemsetAsync(dst, 0, (size_t)n * 4, ctx->stream));
         } else {
@@ -1264,30 +1288,37 @@ int32_t epp_upload(epp_ctx* ctx, int32_t n, const int32_t* is_alive, const int32
         return EPP_OK;
     };
     int rc = 0;
-    rc |= fcol(0, m->position, D, 0.0f);
-    rc |= fcol(sf_vel(D), m->velocity, D, 0.0f);
-    rc |= fcol(sf_dvel(D), m->dvelocity, D, 0.0f);
-    rc |= fcol(sf_mass(D), m->mass, 1, 0.0f);
-    rc |= fcol(sf_vol(D), m->volume, 1, 0.0f);
-    rc |= fcol(sf_rho(D), m->density, 1, 0.0f);
-    rc |= fcol(sf_drho(D), m->ddensity, 1, 0.0f);
-    rc |= fcol(sf_p(D), m->pressure, 1, 0.0f);
-    rc |= fcol(sf_h(D), m->h, 1, 0.0f);
+    rc |= fcol(0, m->position, D);
+    rc |= fcol(sf_vel(D), m->velocity, D);
+    rc |= fcol(sf_dvel(D), m->dvelocity, D);
+    rc |= fcol(sf_mass(D), m->mass, 1);
+    rc |= fcol(sf_vol(D), m->volume, 1);
+    rc |= fcol(sf_rho(D), m->density, 1);
+    rc |= fcol(sf_drho(D), m->ddensity, 1);
+    rc |= fcol(sf_p(D), m->pressure, 1);
+    rc |= fcol(sf_h(D), m->h, 1);
+    fc.flush();
     rc |= icol(SI_TAG, ip + (size_t)m->tag * ldi, 0);
     rc |= icol(SI_MOV, m->is_movable >= 0 ? ip + (size_t)m->is_movable * ldi : nullptr, 1);
     rc |= icol(SI_NCOUNT, m->n_count >= 0 ? ip + (size_t)m->n_count * ldi : nullptr, 0);
+    ic.flush();   // the two vectors below are not columns of the matrix
     rc |= icol(SI_ALIVE, is_alive, 0);
+    ic.flush();
     rc |= icol(SI_CELL, cell_index, 0);
+    ic.flush();
     if (m->instance >= 0) {
-        const int32_t* ic = ip + (size_t)m->instance * ldi;
+        const int32_t* inst = ip + (size_t)m->instance * ldi;
         for (int k = 0; k < n; ++k)
-            if (ic[k] < 0 || ic[k] >= ctx->n_inst)
-                return fail(ctx, EPP_ERR_INVALID_ARGUMENT, "particle %d: instance %d outside 0..%d", k, ic[k],
+            if (inst[k] < 0 || inst[k] >= ctx->n_inst)
+                return fail(ctx, EPP_ERR_INVALID_ARGUMENT, "particle %d: instance %d outside 0..%d", k, inst[k],
                             ctx->n_inst - 1);
-        rc |= icol(SI_INST, ic, 0);
+        rc |= icol(SI_INST, inst, 0);
     } else {
         rc |= icol(SI_INST, nullptr, 0);
     }
+    ic.flush();
+    CK(fc.err);
+    CK(ic.err);
     {
         const int32_t* tc = ip + (size_t)m->tag * ldi;
         for (int k = 0; k < n; ++k)
@@ -1346,38 +1377,37 @@ int32_t epp_download(epp_ctx* ctx, int32_t* is_alive, int32_t* cell_index, int32
     if (D == 2) launch(std::integral_constant<int, 2>{});
     else launch(std::integral_constant<int, 3>{});
     CK_LAUNCH();
-    auto fget = [&](int stage_col, int user_col, int width) -> int {
-        if (!fp || user_col < 0) return EPP_OK;
-        for (int k = 0; k < width; ++k)
-            CK(cudaMemcpyAsync(fp + (size_t)(user_col + k) * ldf, ctx->stage_f + (size_t)(stage_col + k) * n,
-                               (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        return EPP_OK;
+    ColumnCopies fc{ctx->stream, (size_t)n, ldf, cudaMemcpyDeviceToHost}, ic{ctx->stream, (size_t)n, ldi, cudaMemcpyDeviceToHost};
+    auto fget = [&](int stage_col, int user_col, int width) {
+        if (!fp || user_col < 0) return;
+        for (int k = 0; k < width; ++k) fc.add(ctx->stage_f + (size_t)(stage_col + k) * n, fp + (size_t)(user_col + k) * ldf);
     };
-    auto iget = [&](int stage_col, int32_t* dst) -> int {
-        if (!dst) return EPP_OK;
-        CK(cudaMemcpyAsync(dst, ctx->stage_i + (size_t)stage_col * n, (size_t)n * 4, cudaMemcpyDeviceToHost,
-                           ctx->stream));
-        return EPP_OK;
+    auto iget = [&](int stage_col, int32_t* dst) {
+        if (dst) ic.add(ctx->stage_i + (size_t)stage_col * n, dst);
     };
-    int rc = 0;
-    rc |= fget(0, m->position, D);
-    rc |= fget(sf_vel(D), m->velocity, D);
-    rc |= fget(sf_dvel(D), m->dvelocity, D);
-    rc |= fget(sf_mass(D), m->mass, 1);
-    rc |= fget(sf_vol(D), m->volume, 1);
-    rc |= fget(sf_rho(D), m->density, 1);
-    rc |= fget(sf_drho(D), m->ddensity, 1);
-    rc |= fget(sf_p(D), m->pressure, 1);
-    rc |= fget(sf_h(D), m->h, 1);
-    rc |= iget(SI_ALIVE, is_alive);
-    rc |= iget(SI_CELL, cell_index);
+    fget(0, m->position, D);
+    fget(sf_vel(D), m->velocity, D);
+    fget(sf_dvel(D), m->dvelocity, D);
+    fget(sf_mass(D), m->mass, 1);
+    fget(sf_vol(D), m->volume, 1);
+    fget(sf_rho(D), m->density, 1);
+    fget(sf_drho(D), m->ddensity, 1);
+    fget(sf_p(D), m->pressure, 1);
+    fget(sf_h(D), m->h, 1);
+    fc.flush();
     if (ip) {
-        if (m->tag >= 0) rc |= iget(SI_TAG, ip + (size_t)m->tag * ldi);
-        if (m->is_movable >= 0) rc |= iget(SI_MOV, ip + (size_t)m->is_movable * ldi);
-        if (m->n_count >= 0) rc |= iget(SI_NCOUNT, ip + (size_t)m->n_count * ldi);
-        if (m->instance >= 0) rc |= iget(SI_INST, ip + (size_t)m->instance * ldi);
+        if (m->tag >= 0) iget(SI_TAG, ip + (size_t)m->tag * ldi);
+        if (m->is_movable >= 0) iget(SI_MOV, ip + (size_t)m->is_movable * ldi);
+        if (m->n_count >= 0) iget(SI_NCOUNT, ip + (size_t)m->n_count * ldi);
+        if (m->instance >= 0) iget(SI_INST, ip + (size_t)m->instance * ldi);
+        ic.flush();
     }
-    if (rc) return rc;
+    iget(SI_ALIVE, is_alive);
+    ic.flush();
+    iget(SI_CELL, cell_index);
+    ic.flush();
+    CK(fc.err);
+    CK(ic.err);
     const bool want_lists = ctx->lists_valid && ((ip && m->n_index >= 0) ||
                             (fp && (m->n_rvec >= 0 || m->n_r >= 0 || m->n_w >= 0 || m->n_dw >= 0 || m->n_hinv >= 0)));
     if (want_lists) {
@@ -1396,21 +1426,21 @@ int32_t epp_download(epp_ctx* ctx, int32_t* is_alive, int32_t* cell_index, int32
         if (D == 2) launch2(std::integral_constant<int, 2>{});
         else launch2(std::integral_constant<int, 3>{});
         CK_LAUNCH();
-        auto cols = [&](const void* src, void* dstbase, int user_col, int64_t ld, int ncols) -> int {
-            if (user_col < 0 || !dstbase) return EPP_OK;
+        auto cols = [&](ColumnCopies& cc, const void* src, void* dstbase, int user_col, int64_t ld, int ncols) {
+            if (user_col < 0 || !dstbase) return;
             for (int k = 0; k < ncols; ++k)
-                CK(cudaMemcpyAsync((char*)dstbase + ((size_t)(user_col + k) * ld) * 4,
-                                   (const char*)src + (size_t)k * n * 4, (size_t)n * 4,
-                                   cudaMemcpyDeviceToHost, ctx->stream));
-            return EPP_OK;
+                cc.add((const char*)src + (size_t)k * n * 4, (char*)dstbase + ((size_t)(user_col + k) * ld) * 4);
         };
-        rc |= cols(nidx, ip, ip ? m->n_index : -1, ldi, (int)nb);
-        rc |= cols(nrvec, fp, fp ? m->n_rvec : -1, ldf, (int)(nb * D));
-        rc |= cols(nr, fp, fp ? m->n_r : -1, ldf, (int)nb);
-        rc |= cols(nw, fp, fp ? m->n_w : -1, ldf, (int)nb);
-        rc |= cols(ndw, fp, fp ? m->n_dw : -1, ldf, (int)nb);
-        rc |= cols(nh, fp, fp ? m->n_hinv : -1, ldf, (int)nb);
-        if (rc) return rc;
+        cols(ic, nidx, ip, ip ? m->n_index : -1, ldi, (int)nb);
+        cols(fc, nrvec, fp, fp ? m->n_rvec : -1, ldf, (int)(nb * D));
+        cols(fc, nr, fp, fp ? m->n_r : -1, ldf, (int)nb);
+        cols(fc, nw, fp, fp ? m->n_w : -1, ldf, (int)nb);
+        cols(fc, ndw, fp, fp ? m->n_dw : -1, ldf, (int)nb);
+        cols(fc, nh, fp, fp ? m->n_hinv : -1, ldf, (int)nb);
+        ic.flush();
+        fc.flush();
+        CK(fc.err);
+        CK(ic.err);
     }
     CK(cudaStreamSynchronize(ctx->stream));
     return EPP_OK;

@@ -188,3 +188,39 @@ def test_3d_search_variants_count_the_oracles_neighbours(dx, column, h_factor, k
         assert np.all(np.linalg.norm(x[j] - x[i], axis=1) <= 4 * h[i] * h[j] / (h[i] + h[j]) * (1 + 1e-6))
     assert o.status() & abi.EPP_STATUS_CELL_OVERFLOW == 0
     d.close()
+
+
+# Columns travel merged when the host matrices have no rows between them, one by one otherwise; absent
+# columns break a run.
+@pytest.mark.gpu
+@pytest.mark.parametrize("spare,drop", [(0, ()), (37, ()), (0, ("velocity", "n_count", "density")), (5, ("volume",))])
+def test_upload_and_download_of_padded_and_partial_matrices(spare, drop):
+    from epp.classes import ParticleSystem
+    a = casegen.dam_break_2d(dx=0.1, max_neighbour_number=3)
+    stir(a, 1)
+    tables = a.ps.named_index
+    p = ParticleSystem(a.domain, a.n, tables.int_table.capacity, tables.float_table.capacity, a.ps.basic_parameters,
+                       capacityExpand=lambda n: n + spare)
+    for name in list(tables.int_table.capacity) + list(tables.float_table.capacity):
+        p[name] = a.ps[name]
+    before_f, before_i = p.float_properties.copy(), p.int_properties.copy()
+    ns = NeighbourSystem(a.domain, casegen.DAM_BREAK_ACTIVE_PAIRS, max_neighbour_number=3)
+    d = DeviceParticleSystem(p, ns)
+    for f in drop:
+        setattr(d.cmap, f, -1)
+    d.syncto()
+    p.float_properties[:a.n] = -7.0
+    p.int_properties[:a.n] = -7
+    d.ctx.download(p.is_alive, p.cell_index, p.int_properties, p.float_properties, d.cmap)
+    m = d.cmap
+    fcols = [c + k for c, w in [(m.position, 2), (m.velocity, 2), (m.dvelocity, 2), (m.mass, 1), (m.volume, 1),
+                                (m.density, 1), (m.ddensity, 1), (m.pressure, 1), (m.h, 1)] if c >= 0 for k in range(w)]
+    icols = [c for c in (m.tag, m.is_movable, m.n_count) if c >= 0]
+    for c in range(before_f.shape[1]):
+        want = before_f[:a.n, c] if c in fcols else np.full(a.n, -7.0, np.float32)
+        assert np.array_equal(p.float_properties[:a.n, c], want), c
+    for c in range(before_i.shape[1]):
+        want = before_i[:a.n, c] if c in icols else np.full(a.n, -7, np.int32)
+        assert np.array_equal(p.int_properties[:a.n, c], want), c
+    assert np.array_equal(p.float_properties[a.n:], before_f[a.n:])   # rows beyond the particles stay
+    d.close()
