@@ -90,7 +90,11 @@ struct epp_ctx {
     FusedOut tmp{};       // xh/vm/comp of the fused momentum pass
     int* count = nullptr;
     int2* cs = nullptr;
-    int2* perm = nullptr;
+    int2* link = nullptr;
+    int* head[2]{};            // linked-list heads of the cells; the bin passes alternate between the two
+    int* head_mem = nullptr;   // their memory under the cell-centric family, which uses occ
+    int* tile[2]{};            // particles per scan tile, alternating with head
+    int tile_stride = 1;
     unsigned long long* scan_state = nullptr;
     unsigned* status = nullptr;
     unsigned long long* pairs = nullptr;
@@ -214,6 +218,9 @@ size_t state_bytes(int cap) {
     return (size_t)cap * (4 * 16 + 7 * 4) + 12 * 256;
 }
 
+// Ints between two scan-tile counters: a cache line while both buffers fit the arena's slack.
+int tile_stride(int n_tiles) { return n_tiles <= 3800 ? 32 : n_tiles <= 15000 ? 8 : 1; }
+
 size_t arena_bytes(int cap, int n_cells, int D, int n_tiles) {
     size_t b = 2 * state_bytes(cap);
     b += (size_t)cap * 3 * 16 + 3 * 256;                 // fused temp
@@ -225,11 +232,11 @@ size_t arena_bytes(int cap, int n_cells, int D, int n_tiles) {
     b += 256 * 3;                                        // status, pairs
     b += 2 * ((size_t)cap * 4 + 256);                    // nCount of each set
     b += (size_t)cap * 4 * (3 * D + 6) + 256;            // stage_f
-    b += (size_t)cap * 4 * SI_COUNT + 256;               // stage_i (cs and perm of the sort inside)
+    b += (size_t)cap * 4 * SI_COUNT + 256;               // stage_i (cs and link of the sort inside)
     b += (size_t)kIntegralBlocks * 8 * 8 + 8 * 8 + 4 * 256;
     b += 4 * ((size_t)cap * 4 + 256);                    // filter / extrapolation sums, gap by row
     b += 2 * 256;                                                                  // instance tables (small)
-    return b + (1 << 20);
+    return b + std::max((size_t)1 << 20, 2 * ((size_t)n_tiles * tile_stride(n_tiles) * 4 + 256) + 4096);   // tile counters
 }
 
 // Device memory of a context comes from the stream-ordered allocator on the context's stream:
@@ -438,11 +445,11 @@ template <class Act>
 int launch_win_build(epp_ctx* ctx, int set, int crit, const Act& act, unsigned long long* pairs) {
     PairArgs A = pair_args(ctx, set, crit);
     TileMask M{ctx->cap, ctx->nlist};
+    const int T = ctx->pass_threads;
     if (ctx->n <= kWinLanesMax<2>)
-        k_win_lanes<2, Act, 8><<<blocks_for((long long)ctx->n * 8, ctx->pass_threads), ctx->pass_threads, 0, ctx->stream>>>(
-            A, M, act, pairs);
+        k_win_lanes<2, Act, 8><<<blocks_for((long long)ctx->n * 8, T), T, 0, ctx->stream>>>(A, M, act, pairs);
     else
-        k_win_build<Act><<<blocks_for(ctx->n, ctx->pass_threads), ctx->pass_threads, 0, ctx->stream>>>(A, M, act, pairs);
+        k_win_build<Act><<<blocks_for(ctx->n, T), T, 0, ctx->stream>>>(A, M, act, pairs);
     CK_LAUNCH();
     return EPP_OK;
 }
@@ -488,7 +495,7 @@ int launch_list(epp_ctx* ctx, int set, int crit, const Act& act) {
     auto launch = [&](auto LL) {
         constexpr int L = decltype(LL)::value;
         k_list<D, Act, EPI, L><<<blocks_for((long long)ctx->n * L, ctx->pass_threads), ctx->pass_threads, 0, ctx->stream>>>(
-            A, M, ctx->ncnt[set], act, ctx->scan_state, ctx->n_tiles + 1);
+            A, M, ctx->ncnt[set], act);
     };
     if constexpr (kListInter<D, Act>) launch(std::integral_constant<int, 4>{});
     else if (list_lanes<D, Act>(ctx) == 4) launch(std::integral_constant<int, 4>{});
@@ -517,11 +524,10 @@ int launch_pass(epp_ctx* ctx, int set, int crit, const Act& act, unsigned long l
 template <int D, class Act, bool EPI>
 int launch_pair_g(epp_ctx* ctx, const PairArgs& A, const Act& act, unsigned long long* pairs, long long groups) {
     const int G = lanes_of(ctx);
-    const int nw = ctx->n_tiles + 1;
 #define EPP_G(GG)                                                                                 \
     case GG:                                                                                      \
         k_pair_g<D, GG, Act, EPI><<<blocks_for(groups * GG), kThreads, 0, ctx->stream>>>(          \
-            A, act, pairs, ctx->scan_state, nw);                                                  \
+            A, act, pairs);                                                  \
         break;
     switch (G) {
         EPP_G(2)
@@ -585,25 +591,37 @@ int prepare_kernels(epp_ctx* ctx) {
     return g ? EPP_ERR_CUDA : EPP_OK;
 }
 
-// clean! + insert (bin, count, scan, scatter, rank-by-id gather) from set `from` into 1-from.
+// The bin buffers of step parity / call `b`, and what the scan of that sort resets.
+BinOut bin_out(epp_ctx* ctx, int b) { return BinOut{ctx->cs, ctx->link, ctx->count, ctx->head[b], ctx->tile[b], ctx->tile_stride}; }
+
+// Words of look-back state a bin pass clears: only the cell-centric family scans with it.
+int scan_words(const epp_ctx* ctx) { return ctx->lanes == 1 ? ctx->n_tiles + 1 : 0; }
+
+// The scan of the bin pass of buffers `b` into set `to`.
+int launch_scan(epp_ctx* ctx, int b, int to, int max_cell) {
+    const ScanReset R{ctx->head[1 - b], ctx->tile[1 - b], ctx->tile_stride, max_cell};
+    if (ctx->lanes == 1)
+        k_scan<<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->start[to], ctx->occ[to],
+                                                              ctx->meta[to], ctx->scan_state, R, ctx->status);
+    else
+        k_scan_tiles<<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->tile[b],
+                                                                    ctx->start[to], R, ctx->status);
+    CK_LAUNCH();
+    return EPP_OK;
+}
+
+// clean! + insert (bin, scan, rank-by-id gather) from set `from` into 1-from.
 template <int D>
 int sort_cells(epp_ctx* ctx) {
-    const int from = ctx->cur, to = 1 - ctx->cur;
+    const int from = ctx->cur, to = 1 - ctx->cur, b = from;
     const int n = ctx->n;
-    k_bin_count<D><<<blocks_for(n), kThreads, 0, ctx->stream>>>(
-        n, ctx->dom, ctx->S[from], ctx->count, ctx->cs, ctx->cfg.max_cell_particles, ctx->status,
-        ctx->scan_state, ctx->n_tiles + 1);
+    k_bin_count<D><<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->dom, ctx->S[from], bin_out(ctx, b), ctx->status,
+                                                               ctx->scan_state, scan_words(ctx));
     CK_LAUNCH();
-    k_scan<<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->start[to],
-                                                          ctx->occ[to], ctx->meta[to], ctx->scan_state,
-                                                          ctx->status);
-    CK_LAUNCH();
-    k_scatter<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->cs, ctx->start[to], ctx->S[from].id,
-                                                           ctx->perm, ctx->status);
-    CK_LAUNCH();
+    if (const int rc = launch_scan(ctx, b, to, ctx->cfg.max_cell_particles)) return rc;
     ctx->nlist_valid = false;
     MoverAll mv{ctx->S[from], ctx->S[to]};
-    k_rank_gather<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->n_cells, ctx->perm, ctx->cs,
+    k_rank_gather<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->n_cells, ctx->link, ctx->cs, ctx->head[b],
                                                                ctx->start[to], mv, ctx->status);
     CK_LAUNCH();
     ctx->cur = to;
@@ -728,6 +746,7 @@ int enqueue_fused_step(epp_ctx* ctx, int c, const epp_physics& phys, cudaEvent_t
     mom.dom = ctx->dom;
     mom.F = ctx->tmp;
     mom.F.n = n;
+    mom.F.bin = bin_out(ctx, c);
     mom.F.accel = ctx->graph_accel ? ctx->accel : nullptr;
     mom.status = ctx->status;
     const bool gen = generic_physics(&phys);
@@ -755,17 +774,11 @@ int enqueue_fused_step(epp_ctx* ctx, int c, const epp_physics& phys, cudaEvent_t
         }
     }
     EPP_MARK(1);
-    k_scan<<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->start[to],
-                                                          ctx->occ[to], ctx->meta[to], ctx->scan_state,
-                                                          ctx->status);
-    CK_LAUNCH();
+    if (const int rc2 = launch_scan(ctx, c, to, 0)) return rc2;
     EPP_MARK(2);
-    k_scatter<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->cs, ctx->start[to], ctx->S[c].id,
-                                                           ctx->perm, ctx->status);
-    CK_LAUNCH();
-    EPP_MARK(3);
+    EPP_MARK(3);   // (no scatter pass: the gather ranks from the bin's linked lists)
     MoverFused mv{ctx->S[c], ctx->S[to], mom.F, ctx->start[c], ctx->n_cells, phys.fluid_tag, phys.wall_tag};
-    k_rank_gather<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->n_cells, ctx->perm, ctx->cs,
+    k_rank_gather<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->n_cells, ctx->link, ctx->cs, ctx->head[c],
                                                                ctx->start[to], mv, ctx->status);
     CK_LAUNCH();
     EPP_MARK(4);
@@ -1150,17 +1163,21 @@ int32_t epp_create(const epp_config* cfg, epp_ctx** out) {
     ctx->meta[0] = a.take<int>(64);
     ctx->meta[1] = a.take<int>(64);
     ctx->scan_state = a.take<unsigned long long>(ctx->n_tiles + 1);
+    ctx->tile_stride = tile_stride(ctx->n_tiles);
+    ctx->tile[0] = a.take<int>((size_t)ctx->n_tiles * ctx->tile_stride);
+    ctx->tile[1] = a.take<int>((size_t)ctx->n_tiles * ctx->tile_stride);
+    for (int k = 0; k < 2; ++k) ctx->head[k] = ctx->occ[k];   // the occupied cells are listed for family 1 only
     ctx->status = a.take<unsigned>(1);
     ctx->pairs = a.take<unsigned long long>(1);
     ctx->ncnt[0] = a.take<int>(ctx->cap);
     ctx->ncnt[1] = a.take<int>(ctx->cap);
     ctx->stage_f = a.take<float>((size_t)ctx->cap * (3 * D + 6));
-    // the sort's (cell, slot) and permutation live in the int staging columns: those are only in use
+    // the sort's (cell, slot) and cell lists live in the int staging columns: those are only in use
     // inside epp_upload and epp_download, these only between a bin pass and its gather
-    static_assert(SI_COUNT >= 4, "cs and perm take four ints a particle");
+    static_assert(SI_COUNT >= 4, "cs and link take four ints a particle");
     ctx->stage_i = a.take<int>((size_t)ctx->cap * SI_COUNT);
     ctx->cs = reinterpret_cast<int2*>(ctx->stage_i);
-    ctx->perm = ctx->cs + ctx->cap;
+    ctx->link = ctx->cs + ctx->cap;
     ctx->ipartial = a.take<double>(kIntegralBlocks * 8);
     ctx->iresult = a.take<double>(8);
     ctx->iticket = a.take<unsigned>(1);
@@ -1168,10 +1185,6 @@ int32_t epp_create(const epp_config* cfg, epp_ctx** out) {
     ctx->fwp = a.take<float>(ctx->cap);
     ctx->gap = a.take<float>(ctx->cap);
     ctx->fwr = a.take<float>(ctx->cap);
-    ctx->tmp.count = ctx->count;
-    ctx->tmp.cs = ctx->cs;
-    ctx->tmp.scan_state = ctx->scan_state;
-    ctx->tmp.n_scan_words = ctx->n_tiles + 1;
     ctx->tmp.accel = nullptr;
     if (!ctx->fwr) {   // the last part taken: the arena held everything
         epp_destroy(ctx);
@@ -1199,6 +1212,8 @@ int32_t epp_create(const epp_config* cfg, epp_ctx** out) {
     if (cudaMemsetAsync(ctx->arena.base, 0, need, ctx->stream) != cudaSuccess ||
         cudaMemsetAsync(ctx->nlist, 0, nlist_bytes(D, ctx->cap), ctx->stream) != cudaSuccess ||
         cudaMemsetAsync(ctx->cfl_ticket, 0, sizeof(unsigned), ctx->stream) != cudaSuccess ||
+        cudaMemsetAsync(ctx->occ[0], 0xff, sizeof(int) * (ctx->n_cells + 1), ctx->stream) != cudaSuccess ||
+        cudaMemsetAsync(ctx->occ[1], 0xff, sizeof(int) * (ctx->n_cells + 1), ctx->stream) != cudaSuccess ||
         cudaMemsetAsync(ctx->sim_time, 0, sizeof(double) * n_inst, ctx->stream) != cudaSuccess ||
         cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
@@ -1231,6 +1246,7 @@ int32_t epp_destroy(epp_ctx* ctx) {
     dev_free(ctx, ctx->sim_time);
     dev_free(ctx, ctx->list_mem);
     dev_free(ctx, ctx->list_stage);
+    dev_free(ctx, ctx->head_mem);
     dev_free(ctx, ctx->arena.base);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
@@ -1325,6 +1341,10 @@ int32_t epp_upload(epp_ctx* ctx, int32_t n, const int32_t* is_alive, const int32
             if (tc[k] < 0 || tc[k] > 255) return fail(ctx, EPP_ERR_INVALID_ARGUMENT, "tag %d out of range", tc[k]);
     }
     if (rc) return rc;
+    if (ctx->cur == 1) {   // the last sort left the bin buffers of set 1 ready; the next one is from set 0
+        CK(cudaMemsetAsync(ctx->head[0], 0xff, sizeof(int) * (ctx->n_cells + 1), ctx->stream));
+        CK(cudaMemsetAsync(ctx->tile[0], 0, sizeof(int) * (size_t)ctx->n_tiles * ctx->tile_stride, ctx->stream));
+    }
     ctx->cur = 0;
     auto launch = [&](auto Dt) {
         constexpr int DD = decltype(Dt)::value;
@@ -1832,6 +1852,27 @@ int32_t epp_set_tuning(epp_ctx* ctx, int32_t lanes_per_particle) {
     if (g != 0 && ctx->n_inst > 1)
         return fail(ctx, EPP_ERR_INVALID_ARGUMENT, "batches of %d instances use pair-pass family 0", ctx->n_inst);
     if (g != ctx->lanes || store != ctx->store) {
+        if ((g == 1) != (ctx->lanes == 1)) {   // family 1 lists the occupied cells where the others keep list heads
+            cudaSetDevice(ctx->dev);
+            const size_t cells = (size_t)ctx->n_cells + 1, pitch = (cells + 63) & ~(size_t)63;
+            if (g == 1 && !ctx->head_mem) CK(dev_alloc(ctx, &ctx->head_mem, 2 * pitch * sizeof(int)));
+            for (int k = 0; k < 2; ++k) {
+                ctx->head[k] = g == 1 ? ctx->head_mem + k * pitch : ctx->occ[k];
+                CK(cudaMemsetAsync(ctx->head[k], 0xff, cells * sizeof(int), ctx->stream));
+            }
+            if (g == 1 && ctx->sorted_once) {   // list those of the current order (a tuning switch may wait)
+                std::vector<int> st(cells + 1), list;
+                CK(cudaMemcpyAsync(st.data(), ctx->start[ctx->cur], sizeof(int) * cells, cudaMemcpyDeviceToHost, ctx->stream));
+                CK(cudaStreamSynchronize(ctx->stream));
+                for (int c = 0; c < ctx->n_cells; ++c)
+                    if (st[c + 1] > st[c]) list.push_back(c);
+                const int n_occ = (int)list.size();
+                if (n_occ > 0)
+                    CK(cudaMemcpyAsync(ctx->occ[ctx->cur], list.data(), sizeof(int) * n_occ, cudaMemcpyHostToDevice, ctx->stream));
+                CK(cudaMemcpyAsync(ctx->meta[ctx->cur], &n_occ, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
+                CK(cudaStreamSynchronize(ctx->stream));
+            }
+        }
         ctx->lanes = g;
         ctx->store = store;
         ctx->nlist_valid = false;

@@ -3,12 +3,13 @@
 // Some hosts of this library may not call cudaMalloc while they drive a simulation: a host
 // application whose device memory comes from its own fixed pool, or a caller in the middle of a
 // step where a device allocation would synchronise the device or is simply not permitted.  For
-// them epp_cell_sort_noalloc runs the same bin -> count -> scan -> scatter -> rank-by-id pipeline
+// them epp_cell_sort_noalloc runs the same bin -> scan -> rank-by-id pipeline
 // as the context's search!, on device buffers the caller passes in, with every intermediate
 // array in one statically sized device array declared below.  That array is part of the library:
 // every GPU that loads libepp.so holds it until the process exits.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 #include <mutex>
@@ -25,20 +26,21 @@ constexpr int kNaTiles = (kNaMaxCells + 1 + kScanTile - 1) / kScanTile;
 
 // Layout of the scratch (bytes, each part 256-aligned):
 //   counts   int   [kNaMaxCells + 2]
-//   scan     u64   [kNaTiles + 1]        look-back state of the scan
-//   cs       int2  [kNaMaxParticles]     (cell, slot) per particle
-//   perm     int2  [kNaMaxParticles]     (id, particle) in arrival order
+//   tile     int   [2 * kNaTiles * 32]   particles per scan tile, a line apart (and the spare the scan resets)
+//   cs       int2  [kNaMaxParticles]     (cell, slot in the dead bin) per particle
+//   link     int2  [kNaMaxParticles]     (next particle of the cell, id)
 //   start    int   [kNaMaxCells + 2]     offsets before they are copied out
-//   occ      int   [kNaMaxCells + 1]     occupied cells (written by the scan, unused here)
-//   meta     int   [64]
+//   head     int   [kNaMaxCells + 1]     first particle of each cell's list
+//   meta     int   [64]                  n_alive, status word
+constexpr int kTileStride = 32;
 constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 constexpr size_t kOffCounts = 0;
-constexpr size_t kOffScan = kOffCounts + align256(sizeof(int) * (kNaMaxCells + 2));
-constexpr size_t kOffCs = kOffScan + align256(sizeof(unsigned long long) * (kNaTiles + 1));
-constexpr size_t kOffPerm = kOffCs + align256(sizeof(int2) * kNaMaxParticles);
-constexpr size_t kOffStart = kOffPerm + align256(sizeof(int2) * kNaMaxParticles);
-constexpr size_t kOffOcc = kOffStart + align256(sizeof(int) * (kNaMaxCells + 2));
-constexpr size_t kOffMeta = kOffOcc + align256(sizeof(int) * (kNaMaxCells + 1));
+constexpr size_t kOffTile = kOffCounts + align256(sizeof(int) * (kNaMaxCells + 2));
+constexpr size_t kOffCs = kOffTile + align256(sizeof(int) * 2 * kNaTiles * kTileStride);
+constexpr size_t kOffLink = kOffCs + align256(sizeof(int2) * kNaMaxParticles);
+constexpr size_t kOffStart = kOffLink + align256(sizeof(int2) * kNaMaxParticles);
+constexpr size_t kOffHead = kOffStart + align256(sizeof(int) * (kNaMaxCells + 2));
+constexpr size_t kOffMeta = kOffHead + align256(sizeof(int) * (kNaMaxCells + 1));
 constexpr size_t kScratchBytes = kOffMeta + align256(sizeof(int) * 64);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
@@ -50,61 +52,50 @@ constexpr int kMaxDevices = 64;
 std::atomic<unsigned char*> g_scratch_addr[kMaxDevices];
 std::mutex g_scratch_mu;
 
+// Clears what a call starts from: counts, both tile buffers, list heads, the status word.
+__global__ void k_na_clear(int n_cells, int tiles, int* count, int* tile, int* head, int* meta) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c <= n_cells) {
+        count[c] = 0;
+        head[c] = -1;
+    }
+    if (c < tiles) tile[c * kTileStride] = 0;
+    if (c < 2) meta[c] = 0;
+}
+
 // Bin particle i (positions column-major: x at pos[i], y at pos[n + i], z at pos[2n + i]); outside
 // the domain -> dead bin (n_cells), as NeighbourSearch.jl:41-43 kills it.
 template <int D>
-__global__ void k_na_bin(int n, DevDomain dom, const float* pos, int* count, int2* cs) {
+__global__ void k_na_bin(int n, DevDomain dom, const float* pos, BinOut B) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 x = make_float4(pos[i], pos[(size_t)n + i], D == 3 ? pos[(size_t)2 * n + i] : 0.0f, 0.0f);
     int c = cell_of<D>(dom, x, 0);
     if (c < 0) c = dom.n_cells;
-    const int slot = atomicAdd(&count[c], 1);
-    cs[i] = make_int2(c, slot);
+    bin_particle(B, dom.n_cells, i, i, c);
 }
 
-// Rank inside the cell by particle id; writes the 1-based id to its sorted position.
-// A permutation entry or destination outside 0..n-1 is skipped and reported (EPP_STATUS_QUEUE).
-__global__ void k_na_rank(int n, int n_cells, const int2* perm, const int2* cs, const int* start,
-                          int* sorted_ids, unsigned* status) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const int2 e = perm[p];
-    const int src = e.y;
-    if (src < 0 || src >= n) {
-        atomicOr(status, EPP_STATUS_QUEUE);
-        return;
-    }
-    const int c = cs[src].x;
-    if (c >= n_cells) return;   // dead particles are not part of the cell list
-    const int s = start[c], en = min(start[c + 1], n);
-    int rank = 0;
-    for (int q = max(s, 0); q < en; ++q) rank += perm[q].x < e.x;
-    const int dst = s + rank;
-    if (dst < 0 || dst >= n) {
-        atomicOr(status, EPP_STATUS_QUEUE);
-        return;
-    }
-    sorted_ids[dst] = e.x + 1;
-}
-
-// Scatter in arrival order: perm[start[c] + slot] = (particle id, particle id).
-__global__ void k_na_scatter(int n, const int2* cs, const int* start, int2* perm, unsigned* status) {
+// Rank inside the cell by particle id: the 1-based id to its sorted position (a position outside
+// 0..n-1 is skipped and reported, EPP_STATUS_QUEUE); the same grid copies the counts and offsets out
+// and leaves the number of particles inside the domain beside the status word.
+__global__ void k_na_rank(int n, int n_cells, const int2* link, const int2* cs, const int* head, const int* start,
+                          int* sorted_ids, int* counts, int* offsets, int* meta) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i <= n_cells) {
+        const int s = start[i];
+        if (counts && i < n_cells) counts[i] = start[i + 1] - s;
+        if (offsets) offsets[i] = s;
+        if (i == n_cells) meta[0] = s;
+    }
     if (i >= n) return;
     const int2 c = cs[i];
-    const int dst = start[c.x] + c.y;
+    if (c.x >= n_cells) return;   // dead particles are not part of the cell list
+    const int dst = sorted_place(i, c, n_cells, link, head, start);
     if (dst < 0 || dst >= n) {
-        atomicOr(status, EPP_STATUS_QUEUE);
+        atomicOr(reinterpret_cast<unsigned*>(meta + 1), EPP_STATUS_QUEUE);
         return;
     }
-    perm[dst] = make_int2(i, i);
-}
-
-__global__ void k_na_counts(int n_cells, const int* start, int* counts, int* offsets) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < n_cells && counts) counts[c] = start[c + 1] - start[c];
-    if (c <= n_cells && offsets) offsets[c] = start[c];
+    sorted_ids[dst] = i + 1;
 }
 
 }  // namespace
@@ -139,41 +130,36 @@ int32_t epp_cell_sort_noalloc(const epp_domain* domain, int32_t n, const float* 
             g_scratch_addr[dev].store(base, std::memory_order_release);
         }
     }
-    int* count = reinterpret_cast<int*>(base + kOffCounts);
-    unsigned long long* scan = reinterpret_cast<unsigned long long*>(base + kOffScan);
-    int2* cs = reinterpret_cast<int2*>(base + kOffCs);
-    int2* perm = reinterpret_cast<int2*>(base + kOffPerm);
+    int* tile = reinterpret_cast<int*>(base + kOffTile);
     int* start = reinterpret_cast<int*>(base + kOffStart);
-    int* occ = reinterpret_cast<int*>(base + kOffOcc);
     int* meta = reinterpret_cast<int*>(base + kOffMeta);
+    const BinOut B{reinterpret_cast<int2*>(base + kOffCs), reinterpret_cast<int2*>(base + kOffLink),
+                   reinterpret_cast<int*>(base + kOffCounts), reinterpret_cast<int*>(base + kOffHead), tile,
+                   kTileStride};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int nc = dom.n_cells;
     const int tiles = (nc + 1 + kScanTile - 1) / kScanTile;
-    // the scratch keeps the last call's contents: clear what must start at zero
-    if (cudaMemsetAsync(count, 0, sizeof(int) * (nc + 2), s) != cudaSuccess ||
-        cudaMemsetAsync(scan, 0, sizeof(unsigned long long) * (tiles + 1), s) != cudaSuccess ||
-        cudaMemsetAsync(meta, 0, sizeof(int) * 64, s) != cudaSuccess)
-        return EPP_ERR_CUDA;
+    // the scratch keeps the last call's contents: what must start clear goes in one kernel, and the two
+    // words the host reads come back in one copy -- four launches and a copy in all (three memsets, five
+    // kernels and two copies before: 57 us against 39 at 165,888 particles, 74 against 61 at 955,668)
     const int T = 128;
-    const int gb = (n + T - 1) / T;
+    auto grid = [&](int k) { return (k + T - 1) / T; };
+    k_na_clear<<<grid(nc + 1), T, 0, s>>>(nc, tiles, B.count, tile, B.head, meta);
     if (n > 0) {
-        if (domain->dim == 2) k_na_bin<2><<<gb, T, 0, s>>>(n, dom, pos, count, cs);
-        else k_na_bin<3><<<gb, T, 0, s>>>(n, dom, pos, count, cs);
+        if (domain->dim == 2) k_na_bin<2><<<grid(n), T, 0, s>>>(n, dom, pos, B);
+        else k_na_bin<3><<<grid(n), T, 0, s>>>(n, dom, pos, B);
     }
-    k_scan<<<tiles, kScanThreads, 0, s>>>(nc + 1, count, start, occ, meta, scan,
-                                          reinterpret_cast<unsigned*>(meta + 1));
-    unsigned* status = reinterpret_cast<unsigned*>(meta + 1);
-    if (n > 0) {
-        k_na_scatter<<<gb, T, 0, s>>>(n, cs, start, perm, status);
-        k_na_rank<<<gb, T, 0, s>>>(n, nc, perm, cs, start, sorted_ids, status);
-    }
-    k_na_counts<<<(nc + 1 + T - 1) / T, T, 0, s>>>(nc, start, counts, offsets);
+    // (the scan's resets go to the spare tile counters and to the counts it has just cleared)
+    k_scan_tiles<<<tiles, kScanThreads, 0, s>>>(nc + 1, B.count, tile, start, ScanReset{B.count, tile + kNaTiles * kTileStride, kTileStride, 0},
+                                               reinterpret_cast<unsigned*>(meta + 1));
+    k_na_rank<<<grid(std::max(n, nc + 1)), T, 0, s>>>(n, nc, B.link, B.cs, B.head, start, sorted_ids, counts, offsets, meta);
     if (cudaGetLastError() != cudaSuccess) return EPP_ERR_CUDA;
-    unsigned st = 0;
-    if (cudaMemcpyAsync(n_alive, start + nc, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-        cudaMemcpyAsync(&st, status, sizeof st, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+    int back[2] = {0, 0};   // particles inside the domain, status
+    if (cudaMemcpyAsync(back, meta, sizeof back, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaStreamSynchronize(s) != cudaSuccess)
         return EPP_ERR_CUDA;
+    *n_alive = back[0];
+    const unsigned st = (unsigned)back[1];
     return st ? EPP_ERR_DEVICE_STATUS : EPP_OK;
 }
 

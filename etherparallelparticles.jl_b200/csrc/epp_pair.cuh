@@ -206,11 +206,8 @@ struct FusedOut {
     float4* xh;          // new (x, h)   in the current (old) order
     float4* vm;          // new (v, m)
     float4* comp;        // new Kahan compensation
-    int2* cs;            // (cell, slot) for the counting sort
-    int* count;          // per-cell counters (zero on entry)
+    BinOut bin;          // cell lists of the new positions for the counting sort
     float4* accel;       // optional dv/dt output (momentum + gravity), may be null
-    unsigned long long* scan_state;   // cleared by block 0 for the scan that follows
-    int n_scan_words;
     int n;               // all particles (alive first, dead bin last)
 };
 

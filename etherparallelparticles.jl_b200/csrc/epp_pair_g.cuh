@@ -301,8 +301,7 @@ struct ActMomG {
                 atomicOr(status, EPP_STATUS_KILLED);
             }
         }
-        const int slot = atomicAdd(&F.count[c], 1);
-        F.cs[i] = make_int2(c, slot);
+        bin_particle(F.bin, dom.n_cells, i, s.id[i], c);
     }
 };
 
@@ -351,12 +350,9 @@ __device__ __forceinline__ void act_epilogue_nf(const ActMomG<D, true>& act, int
 
 // One pair pass, G lanes per particle.  With FUSED_EPI (momentum of the fused step) the grid
 // covers every particle and lane 0 of each group runs the integrate + bin epilogue, also for the
-// dead bin; block 0 clears the scan's look-back state.
+// dead bin.
 template <int D, int G, class Act, bool FUSED_EPI>
-__global__ void __launch_bounds__(128) k_pair_g(PairArgs A, Act act, unsigned long long* pairs,
-                                                unsigned long long* scan_state, int n_scan_words) {
-    if (FUSED_EPI && blockIdx.x == 0)
-        for (int t = threadIdx.x; t < n_scan_words; t += blockDim.x) scan_state[t] = 0ull;
+__global__ void __launch_bounds__(128) k_pair_g(PairArgs A, Act act, unsigned long long* pairs) {
     const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     const int i = t / G;

@@ -541,12 +541,10 @@ constexpr bool kListInter = D == 3 && Act::NC == 3;
 template <int D, class Act, bool EPI, int L>
 __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 blocks (56 registers) beat 7, 8 and 10
     k_list(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M, const int* ncount,
-           const __grid_constant__ Act act, unsigned long long* scan_state, int n_scan_words) {
+           const __grid_constant__ Act act) {
     using T = ListTerm<D, Act>;
     constexpr bool ROW = ListConf<D>::ROW;
     constexpr bool INTER = kListInter<D, Act> && L > 1;
-    if (EPI && blockIdx.x == 0)
-        for (int t = threadIdx.x; t < n_scan_words; t += blockDim.x) scan_state[t] = 0ull;
     const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int i = (int)(tid / L), g = (int)(tid % L);

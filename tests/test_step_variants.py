@@ -224,3 +224,35 @@ def test_upload_and_download_of_padded_and_partial_matrices(spare, drop):
         assert np.array_equal(p.int_properties[:a.n, c], want), c
     assert np.array_equal(p.float_properties[a.n:], before_f[a.n:])   # rows beyond the particles stay
     d.close()
+
+
+# The sort's buffers alternate with the state sets: an upload at either parity, pair-pass families that
+# keep other lists in them, and a dead bin of many particles leave the next cell list right.
+@pytest.mark.gpu
+@pytest.mark.parametrize("steps,family", [(0, 0), (1, 0), (2, 0), (3, 1), (2, 1), (1, 4)])
+@pytest.mark.parametrize("dead", [0, 700])
+def test_cell_lists_after_uploads_and_family_switches(steps, family, dead):
+    c = casegen.dam_break_2d(dx=0.04, max_neighbour_number=1)
+    stir(c, 2)
+    x = c.ps["PositionVec"]
+    fluid = np.flatnonzero(c.ps["Tag"] == casegen.FLUID_TAG)
+    x[fluid[:dead]] = 100.0   # outside: the search kills them
+    c.ps["PositionVec"] = x
+    want = device(c)
+    want.ctx.search(SYM, CONT, c.physics, 0)
+    counts, offsets, ids = want.ctx.cell_stats()
+    want.close()
+    d = device(c)
+    d.ctx.search(SYM, CONT, c.physics, 0)
+    d.ctx.set_tuning(family)
+    if steps:
+        d.ctx.step(steps, c.physics)
+    d.syncto()
+    d.ctx.search(SYM, CONT, c.physics, 0)
+    for _ in range(2):   # once more: a search! in place keeps the order
+        got = d.ctx.cell_stats()
+        assert np.array_equal(got[0], counts) and np.array_equal(got[1], offsets) and np.array_equal(got[2], ids)
+        d.ctx.set_tuning(0)
+        d.ctx.search(SYM, abi.EPP_ACTION_NONE, c.physics, 0)
+    assert d.ctx.synchronize(raise_on_status=False) & ~abi.EPP_STATUS_KILLED == 0
+    d.close()
