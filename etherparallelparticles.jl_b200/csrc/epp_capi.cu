@@ -449,7 +449,7 @@ int launch_win_build(epp_ctx* ctx, int set, int crit, const Act& act, unsigned l
     if (ctx->n <= kWinLanesMax<2>)
         k_win_lanes<2, Act, 8><<<blocks_for((long long)ctx->n * 8, T), T, 0, ctx->stream>>>(A, M, act, pairs);
     else
-        k_win_build<Act><<<blocks_for(ctx->n, T), T, 0, ctx->stream>>>(A, M, act, pairs);
+        k_win_build<Act><<<blocks_for(ctx->n, T), T, T / 32 * sizeof(Stage2<Act>), ctx->stream>>>(A, M, act, pairs);
     CK_LAUNCH();
     return EPP_OK;
 }
@@ -469,7 +469,7 @@ int launch_build(epp_ctx* ctx, int set, int crit, unsigned long long* pairs) {
         k_win_lanes<3, CPCount<3>, 8><<<blocks_for((long long)ctx->n * 8, T), T, 0, ctx->stream>>>(
             A, M, CPCount<3>{ctx->ncnt[set]}, pairs);
     } else {
-        k_win_build3<<<blocks_for(ctx->n, T), T, 0, ctx->stream>>>(A, M, ctx->ncnt[set], pairs);
+        k_win_build3<<<blocks_for(ctx->n, T), T, T / 32 * sizeof(Stage3), ctx->stream>>>(A, M, ctx->ncnt[set], pairs);
     }
     CK_LAUNCH();
     return EPP_OK;

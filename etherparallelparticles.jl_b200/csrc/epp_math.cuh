@@ -297,7 +297,13 @@ __device__ __forceinline__ float root(float x) {
     const float s = __fmul_rn(x, y);
     return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, y), s);
 }
-__device__ __forceinline__ float rcp_fast(float x) { return __fdividef(1.0f, x); }
+// Approximate reciprocal (1 ulp) without the scaling that a division of possibly subnormal operands
+// carries along: for densities and squared lengths.
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 
 // The cell grid of a domain, on the host, in FP32 as the Domain2D constructor computes it
 // (Domain2D.jl:28-67): n_a = floor(span_a / gap) cells per axis, gap_a = span_a / n_a and

@@ -603,7 +603,8 @@ __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 bl
             const size_t stride = ROW ? L : (size_t)L * M.cap;
             const int first = (int)(threadIdx.x & 31u & ~(unsigned)(L - 1));
             const unsigned group = L == 1 ? 0u : ((1u << L) - 1u) << first;
-            int en = g < cnt ? (ROW ? *list : __ldcs(list)) : 0;
+            auto read = [&]() { return ROW ? *list : __ldcs(list); };
+            int en = g < cnt ? read() : 0;
             for (int k0 = 0; k0 < cnt; k0 += L) {
                 typename T::Term t{};
                 if (k0 + g < cnt) {
@@ -612,7 +613,7 @@ __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 bl
                     const typename T::Rec r = T::load(A, act, me, j, tj);
                     if (k0 + L + g < cnt) {
                         list += stride;
-                        en = ROW ? *list : __ldcs(list);
+                        en = read();
                     }
                     t = T::term(act, me, r, tj);
                     if (L == 1 || INTER) T::add(acc, t);

@@ -161,10 +161,10 @@ __device__ __forceinline__ WinOut win_lane_general(const PairArgs& A, const Tile
 template <class Act>
 __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M,
                                                    const __grid_constant__ Act act, unsigned long long* pairs) {
-    __shared__ Stage2<Act> stage[4];
+    extern __shared__ __align__(16) unsigned char win_smem[];   // a staging area per warp
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    Stage2<Act>& S = stage[threadIdx.x >> 5];
+    Stage2<Act>& S = reinterpret_cast<Stage2<Act>*>(win_smem)[threadIdx.x >> 5];
     const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int w0 = i - lane;
@@ -382,10 +382,10 @@ __device__ __forceinline__ unsigned window_bits3(const float4* sx, int off, int 
 
 __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M,
                                                        int* ncount, unsigned long long* pairs) {
-    __shared__ Stage3 stage[4];
+    extern __shared__ __align__(16) unsigned char win_smem[];   // a staging area per warp
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    Stage3& S = stage[threadIdx.x >> 5];
+    Stage3& S = reinterpret_cast<Stage3*>(win_smem)[threadIdx.x >> 5];
     const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int w0 = i - lane;
