@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <type_traits>
@@ -64,6 +65,46 @@ DevPhys to_dev(const epp_physics& p) {
     d.gap = nullptr;
     return d;
 }
+
+// Page-locked words the device results of blocking calls come back through: a copy to pageable memory
+// blocks on its own (about 10 us each), one to these is waited for with the stream.  One block of
+// kSlots for the process, taken on first use; a context holds one slot from its first blocking call to
+// its destruction and falls back to pageable copies when none is left.
+class HostSlots {
+public:
+    static constexpr int kSlots = 512, kBytes = 128;
+    static HostSlots& get() {
+        static HostSlots* s = new HostSlots;   // not destroyed: contexts may outlive static destructors
+        return *s;
+    }
+    char* take() {
+        std::lock_guard<std::mutex> lock(mu_);
+        if (!base_ && !failed_) {
+            void* p = nullptr;
+            failed_ = cudaHostAlloc(&p, (size_t)kSlots * kBytes, cudaHostAllocPortable) != cudaSuccess;
+            if (failed_) {
+                cudaGetLastError();
+            } else {
+                base_ = static_cast<char*>(p);
+                for (int k = kSlots - 1; k >= 0; --k) free_.push_back(base_ + (size_t)k * kBytes);
+            }
+        }
+        if (free_.empty()) return nullptr;
+        char* p = free_.back();
+        free_.pop_back();
+        return p;
+    }
+    void give(char* p) {
+        std::lock_guard<std::mutex> lock(mu_);
+        free_.push_back(p);
+    }
+
+private:
+    std::mutex mu_;
+    char* base_ = nullptr;
+    bool failed_ = false;
+    std::vector<char*> free_;
+};
 
 bool same_phys(const epp_physics& a, const epp_physics& b) { return std::memcmp(&a, &b, sizeof a) == 0; }
 
@@ -174,6 +215,7 @@ struct epp_ctx {
     cudaEvent_t idone[2]{};
     bool ipending[2]{};
     bool timed = false;
+    char* slot = nullptr;   // page-locked words for blocking results (HostSlots), taken on first use
     std::string err;
 };
 
@@ -200,6 +242,11 @@ int fail(epp_ctx* c, int code, const char* fmt, ...) {
     } while (0)
 
 #define CK_LAUNCH() CK(cudaGetLastError())
+
+char* host_slot(epp_ctx* ctx) {
+    if (!ctx->slot) ctx->slot = HostSlots::get().take();
+    return ctx->slot;
+}
 
 // Makes the context's stream wait for integrals still running beside it on set k (both sets when
 // k < 0).  Every entry point that may overwrite a state set, or run the integrals' reduction
@@ -1258,6 +1305,7 @@ int32_t epp_destroy(epp_ctx* ctx) {
         if (ctx->idone[k]) cudaEventDestroy(ctx->idone[k]);
     if (ctx->istream) cudaStreamDestroy(ctx->istream);
     if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
+    if (ctx->slot) HostSlots::get().give(ctx->slot);   // both streams have finished
     delete ctx;
     return EPP_OK;
 }
@@ -1597,12 +1645,13 @@ int32_t epp_get_integrals(epp_ctx* ctx, const epp_physics* phys, epp_integrals* 
     if (ctx->n == 0) return EPP_OK;
     if (!ctx->sorted_once) return fail(ctx, EPP_ERR_STATE, "integrals need a search! first");
     if (const int rc = launch_integrals(ctx, phys, ctx->stream)) return rc;
-    double r[8];
+    double own[9], *r = own;
+    if (char* slot = host_slot(ctx)) r = reinterpret_cast<double*>(slot);
     int n_alive = 0;
     CK(cudaMemcpyAsync(r, ctx->iresult, 8 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(&n_alive, ctx->start[ctx->cur] + ctx->n_cells, sizeof(int), cudaMemcpyDeviceToHost,
-                       ctx->stream));
+    CK(cudaMemcpyAsync(r + 8, ctx->start[ctx->cur] + ctx->n_cells, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
+    std::memcpy(&n_alive, r + 8, sizeof n_alive);
     fill_integrals(out, r, n_alive, phys->c0, phys->cfl);
     return EPP_OK;
 }
@@ -1735,10 +1784,13 @@ int32_t epp_synchronize(epp_ctx* ctx, uint32_t* device_status) {
     if (!ctx) return EPP_ERR_INVALID_ARGUMENT;
     cudaSetDevice(ctx->dev);
     if (const int rc_ = join_integrals(ctx)) return rc_;
-    CK(cudaStreamSynchronize(ctx->stream));
+    // the status word comes back with the wait for the stream, and is cleared (in stream order) when set
     unsigned st = 0;
-    CK(cudaMemcpy(&st, ctx->status, sizeof st, cudaMemcpyDeviceToHost));
-    CK(cudaMemset(ctx->status, 0, sizeof st));
+    char* slot = host_slot(ctx);
+    CK(cudaMemcpyAsync(slot ? (void*)slot : &st, ctx->status, sizeof st, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    if (slot) std::memcpy(&st, slot, sizeof st);
+    if (st) CK(cudaMemsetAsync(ctx->status, 0, sizeof st, ctx->stream));
     if (device_status) *device_status = st;
     if (st & ~(unsigned)EPP_STATUS_KILLED)
         return fail(ctx, EPP_ERR_DEVICE_STATUS, "device status 0x%x", st);
