@@ -342,11 +342,14 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
 // one, and a row beyond it is read from global memory.  One warp per cell, its lanes on the candidates
 // and ballots in place of the walk, measured 528 us: two POPC per target and chunk, no fewer
 // instructions.
-constexpr int kStage3 = 320;   // staged candidates per warp: 7 blocks of 128 threads fit an SM
+// Staged candidates per warp: both parts of a warp that crosses a cell-row end (about 360; with room for
+// 320 only, such warps searched a plane in two passes and were the pass's tail: 121 us at 165,888
+// particles); 7 blocks of 128 threads fit an SM.
+constexpr int kStage3 = 432;
 
 struct Stage3 {
-    float4 x[kStage3];   // (x, y, z, h)
-    int e[kStage3];      // list entry (index and tag)
+    float4 x[kStage3];          // (x, y, z, h)
+    unsigned char t[kStage3];   // tag
 };
 
 // Acceptance bits of `len` <= 32 staged candidates from slot `off`, candidate 0 in the top bit; see
@@ -453,6 +456,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
                         pending &= ~taken;
                         break;
                     }
+#pragma unroll 4   // their loads in flight together (2% at 955,668 particles, 4% at 165,888; the 2D pass lost 3%)
                     for (int k = lane; k < total; k += 32) {
                         const int j = k < len[0] ? lo[0] + k
                                                  : k < len[0] + len[1] ? lo[1] + (k - len[0]) : lo[2] + (k - len[0] - len[1]);
@@ -461,7 +465,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
                         const bool bad = tj < 1 || tj > A.n_tags;   // never a neighbour: fails every test
                         if (bad) xj.x = __int_as_float(0x7fffffff);
                         S.x[used + k] = xj;
-                        S.e[used + k] = list_entry(j, bad ? 1 : tj);
+                        S.t[used + k] = (unsigned char)(bad ? 1 : tj);
                         if (xj.w != hw) {
                             two_h = two_h && (!other || hb == xj.w);
                             other = true;
@@ -526,8 +530,8 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
                         while (word) {
                             const int b = __clz(word);
                             word ^= 0x80000000u >> b;
-                            const int e = S.e[o + k0 + b];
-                            if ((amask >> (entry_tag(e) - 1)) & 1u) L.put(cnt++, e);   // the active-pair matrix
+                            const int tj = S.t[o + k0 + b];
+                            if ((amask >> (tj - 1)) & 1u) L.put(cnt++, list_entry(lo + k0 + b, tj));   // the active-pair matrix
                         }
                     }
                 }
