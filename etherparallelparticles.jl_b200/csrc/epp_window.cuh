@@ -72,23 +72,22 @@ struct Stage2 {
 
 // Acceptance bits of a lane's window of `len` <= 32 candidates from slot `off`: bit k set when
 // candidate k passes the criterion by the reference's IEEE arithmetic.  `one`: every candidate has the
-// lane's h (or the default criterion), so one exact bound serves; otherwise it is looked up per
-// candidate.  Cells hold their fluid before their walls, so h alternates along a row between the
-// lane's own and a wall's: the last other h and its bound (a division) are kept in (ho, ro).
-__device__ __forceinline__ unsigned window_bits(const float4* sx, int off, int len, float4 xi, bool one, float own, bool dflt,
-                                                float& ho, float& ro) {
+// lane's h (or the default criterion), so one exact bound serves (bias nO); otherwise those of another
+// h take its bound, the bias of the last one kept in (ho, no): cells hold their fluid before their
+// walls, so along a row h alternates between the lane's own and one other.
+__device__ __forceinline__ unsigned window_bits(const float4* sx, int off, int len, float4 xi, bool one, int nO, float& ho,
+                                                int& no) {
     // (dx, dy) and (dx^2, dy^2) on the packed f32x2 pipe (each half rounds like __fsub_rn /
     // __fmul_rn), the sum scalar
     const f32x2 XY = f2_pack(xi.x, xi.y);
     unsigned word = 0u;
     if (one) {
-        const int nR2 = accept_bias(own);
 #pragma unroll 4
         for (int k = len - 1; k >= 0; --k) {
             const f32x2 d = f2_sub(XY, *reinterpret_cast<const f32x2*>(&sx[off + k]));
             float dx2, dy2;
             f2_unpack(f2_mul(d, d), dx2, dy2);
-            word = (word << 1) | ((unsigned)(__float_as_int(__fadd_rn(dx2, dy2)) + nR2) >> 31);
+            word = (word << 1) | ((unsigned)(__float_as_int(__fadd_rn(dx2, dy2)) + nO) >> 31);
         }
         return word;
     }
@@ -100,9 +99,9 @@ __device__ __forceinline__ unsigned window_bits(const float4* sx, int off, int l
         f2_unpack(f2_mul(d, d), dx2, dy2);
         if (hj != xi.w && hj != ho) {
             ho = hj;
-            ro = dflt ? own : pair_r2(xi.w, ho);
+            no = accept_bias(pair_r2(xi.w, ho));
         }
-        word = (word << 1) | (__fadd_rn(dx2, dy2) <= (hj == xi.w ? own : ro) ? 1u : 0u);
+        word = (word << 1) | ((unsigned)(__float_as_int(__fadd_rn(dx2, dy2)) + (hj == xi.w ? nO : no)) >> 31);
     }
     return word;
 }
@@ -193,7 +192,8 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
             const int head = __ffs(pending) - 1;
             const float hw = __shfl_sync(FULL, xi.w, head);   // the pass is plain when every candidate has
             const int tw = __shfl_sync(FULL, ti, head);       // the first lane's h and tag
-            bool same_h = true, same_t = true, staged = false;
+            bool same_t = true, staged = false, other = false;
+            float hb = hw;   // an h other than hw that this lane staged
             int used = 0, off[3] = {0, 0, 0};
             unsigned taken = 0u;
             __syncwarp();
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
                     S.x[used + k] = make_float4(bad ? __int_as_float(0x7fffffff) : xj.x, xj.y,
                                                 __int_as_float(list_entry(j, bad ? 1 : tj)), xj.w);
                     if (Act::NC != 0) S.nb[used + k] = act.fetch(j, 0, tj);
-                    same_h = same_h && xj.w == hw;
+                    if (xj.w != hw) other = true, hb = xj.w;
                     same_t = same_t && tj == tw;
                 }
                 const unsigned part = ((2u << last) - 1u) & ~((1u << lead) - 1u);
@@ -241,7 +241,8 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
                 taken |= part;
                 pending &= ~part;
             }
-            same_h = __all_sync(FULL, same_h);   // (also orders the staging before its use)
+            const unsigned others = __ballot_sync(FULL, other);
+            const float h2 = __shfl_sync(FULL, hb, others ? __ffs(others) - 1 : 0);   // another h of the pass, if any
             same_t = __all_sync(FULL, same_t);
             __syncwarp();
             if (!(((taken >> lane) & 1u) && valid)) continue;
@@ -259,9 +260,20 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
             }
             const TargetConst tc = target_const<2>(xi.w);
             if (same_t && !((amask >> (tw - 1)) & 1u)) continue;   // nothing the lane may see: walls among walls
-            const bool one = dflt || (same_h && xi.w == hw);
-            const float own = dflt ? A.dom.gap_square : tc.h2sq;
-            float ho = xi.w, ro = own;   // the last other h and its bound
+            const bool one = dflt || !others;
+            const int nO = accept_bias(dflt ? A.dom.gap_square : tc.h2sq);
+            // kernel constants and bound with the pass's other h (walls against fluid), so that the walk
+            // selects instead of dividing per pair (182 -> 174 us for 64 dam breaks of 1,217,760 particles,
+            // step 34.6 -> 33.6 at 22,279); a third h is computed where it is met
+            TargetConst to = tc;
+            int no = nO;
+            if (others) {
+                to.h = xi.w == hw ? h2 : hw;
+                to.hinv = invharmonic_exact(tc.h, to.h);
+                to.kdw = wc2_kdw<2>(to.hinv);
+                no = accept_bias(pair_r2(xi.w, to.h));
+            }
+            float ho = to.h;
             typename Act::Self me = act.self(i);
             ListWriter<2> L = list_writer<2>(M, i);
             const f32x2 XI = f2_pack(xi.x, xi.y);
@@ -273,16 +285,16 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
                 if (!two) {
                     // the three words first, then one walk over all of them, so a warp iterates as often as
                     // its busiest lane's neighbour count (not the sum over rows of each row's busiest lane)
-                    a = window_bits(S.x, o0, l0, xi, one, own, dflt, ho, ro);
-                    b = window_bits(S.x, o1, l1, xi, one, own, dflt, ho, ro);
-                    c2 = window_bits(S.x, o2, l2, xi, one, own, dflt, ho, ro);
+                    a = window_bits(S.x, o0, l0, xi, one, nO, ho, no);
+                    b = window_bits(S.x, o1, l1, xi, one, nO, ho, no);
+                    c2 = window_bits(S.x, o2, l2, xi, one, nO, ho, no);
                     b &= ~(1u << (i - win[1].lo));   // not its own neighbour
                     if (!b) b = c2, o1 = o2, c2 = 0u;   // empty rows last: one word is current, the next follows
                     if (!a) a = b, o0 = o1, b = c2, o1 = o2, c2 = 0u;
                 } else {
                     const int r = q >> 1, k0 = (q & 1) * 32;
                     o0 = (r == 0 ? off[0] : r == 1 ? off[1] : off[2]) + k0;
-                    a = window_bits(S.x, o0, min((r == 0 ? l0 : r == 1 ? l1 : l2) - k0, 32), xi, one, own, dflt, ho, ro);
+                    a = window_bits(S.x, o0, min((r == 0 ? l0 : r == 1 ? l1 : l2) - k0, 32), xi, one, nO, ho, no);
                     const int self = i - win[1].lo - k0;
                     if (r == 1 && self >= 0 && self < 32) a &= ~(1u << self);
                 }
@@ -310,7 +322,9 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
                         if (Act::NC != 0) {
                             const int tj = entry_tag(e);
                             const float4 xj = make_float4(xs.x, xs.y, 0.0f, xs.w);
-                            const float4 t = act.term(me, S.nb[slot], ti, tj, xj, geometry<2>(xi, xj), tc);
+                            TargetConst tq = tc;
+                            if (xs.w == to.h) tq.h = to.h, tq.hinv = to.hinv, tq.kdw = to.kdw;
+                            const float4 t = act.term(me, S.nb[slot], ti, tj, xj, geometry<2>(xi, xj), tq);
                             sum.x = __fadd_rn(sum.x, t.x);
                             sum.y = __fadd_rn(sum.y, t.y);
                         }
@@ -334,8 +348,8 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
 // The 3D search pass: neighbour lists and nCount.  Windows as in 2D, nine stencil rows of about 53
 // candidates at h = 1.3 dx, one plane (three rows) staged at a time; a particle's 480 candidates are
 // tested by its own lane.  It replaces a lockstep search of the warp's whole union of stencils (about
-// 700 candidates, 32 at a time, with a divergent append after each chunk): 574 -> 387 us at 955,668
-// particles, 182 -> 119 at 165,888.  Issue-bound (79% of the slots): about half on the tests, 40% on the
+// 700 candidates, 32 at a time, with a divergent append after each chunk): 574 -> 356 us at 955,668
+// particles, 182 -> 84 at 165,888.  Issue-bound (79% of the slots): about half on the tests, 40% on the
 // walk over their bits, which is why a word whose candidates have one tag computes its entries and
 // checks the list's capacity once.  Warps near walls stage two h's and take the two bounds by a select.
 // When one particle's plane is longer than the staging area (dense neighbourhoods) the rows go one by

@@ -134,6 +134,40 @@ def test_eight_lane_search_equals_the_staged_search(dx, h_factor, jitter, physic
     d.close()
 
 
+# Three h's mixed at random (walls of a third one, or of the fluid's): staged warps then see their own,
+# one other and further ones.  Same bits as the eight-lane search of each instance alone.
+@pytest.mark.gpu
+@pytest.mark.parametrize("share", [0.5, 0.002])
+def test_staged_search_with_three_smoothing_lengths(share):
+    dx, n_inst = 0.0231, 24
+    columns = [(0.5 + 0.03 * k, 1.0 + 0.05 * k) for k in range(n_inst)]
+    b = casegen.dam_break_batch(columns=columns, dx=dx)
+    stir(b, 17)
+    rng = np.random.default_rng(4)
+    h = b.ps["H"].copy()
+    pick = rng.random(b.n) < share   # smaller h only: every neighbour stays inside the 9 cells
+    h[pick] *= rng.choice(np.float32([0.93, 0.8]), int(pick.sum()))
+    b.ps["H"] = h
+    d = device(b, n_inst)
+    d.ctx.search(SYM, CONT, b.physics, 0)
+    d.ctx.synchronize()
+    d.asyncto()
+    for k in (0, 23):
+        r0, r1 = b.rows[k]
+        c = casegen.dam_break_2d(dx=dx, column=columns[k], max_neighbour_number=1)
+        for name in ("PositionVec", "VelocityVec"):
+            c.ps[name] = d.host[name][r0:r1]
+        c.ps["H"] = h[r0:r1]
+        a = device(c)
+        a.ctx.search(SYM, CONT, c.physics, 0)
+        a.ctx.synchronize()
+        a.asyncto()
+        for name in ("dDensity", "nCount"):
+            assert np.array_equal(a.host[name], d.host[name][r0:r1]), (k, name)
+        a.close()
+    d.close()
+
+
 # v / d by multiplication, on the CPU: the same arithmetic as csrc/epp_math.cuh FastDiv
 @pytest.mark.parametrize("d", [1, 2, 3, 7, 64, 1000, 1367, 65535, 65537, (1 << 22) + 1, (1 << 30) - 1, 1 << 30])
 def test_fast_division(d):
