@@ -483,9 +483,9 @@ bool uses_windows(const epp_ctx* ctx) { return ctx->D == 2 && ctx->store != EPP_
 
 // Largest particle count at which the search pass takes eight lanes per particle: measured, us with
 // eight lanes and with one, 2D 12 / 25 at 1,418 particles, 14 / 23 at 6,518, 22 / 22 at 22,279, 33 / 27
-// at 45,203; 3D 52 / 88 at 33,123, 83 / 82 at 62,721, 216 / 119 at 165,888.
+// at 45,203; 3D 51 / 59 at 33,123, 67 / 69 at 47,040, 83 / 70 at 62,721, 216 / 84 at 165,888.
 template <int D>
-constexpr int kWinLanesMax = D == 2 ? 20000 : 60000;
+constexpr int kWinLanesMax = D == 2 ? 20000 : 50000;
 
 // The 2D window search pass with search action `act` (CPCount: lists and nCount only).
 template <class Act>

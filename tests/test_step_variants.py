@@ -184,7 +184,7 @@ def test_fast_division(d):
         assert q == x // d, (x, d)
 
 
-# 3D search: eight lanes per particle (small system) and staged planes (beyond 60,000 particles), with
+# 3D search: eight lanes per particle (small system) and staged planes (beyond 50,000 particles), with
 # one h, the two of fluid and walls, and three mixed at random; h = 2.5 dx takes rows one by one.  The
 # neighbour counts are the oracle's.
 @pytest.mark.gpu
