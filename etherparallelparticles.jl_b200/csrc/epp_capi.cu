@@ -7,6 +7,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -74,8 +75,8 @@ class HostSlots {
 public:
     static constexpr int kSlots = 512, kBytes = 128;
     static HostSlots& get() {
-        static HostSlots* s = new HostSlots;   // not destroyed: contexts may outlive static destructors
-        return *s;
+        static HostSlots s;   // nothing to destroy: contexts may outlive static destructors
+        return s;
     }
     char* take() {
         std::lock_guard<std::mutex> lock(mu_);
@@ -86,24 +87,22 @@ public:
                 cudaGetLastError();
             } else {
                 base_ = static_cast<char*>(p);
-                for (int k = kSlots - 1; k >= 0; --k) free_.push_back(base_ + (size_t)k * kBytes);
+                for (n_free_ = 0; n_free_ < kSlots; ++n_free_) free_[n_free_] = base_ + (size_t)n_free_ * kBytes;
             }
         }
-        if (free_.empty()) return nullptr;
-        char* p = free_.back();
-        free_.pop_back();
-        return p;
+        return n_free_ > 0 ? free_[--n_free_] : nullptr;
     }
-    void give(char* p) {
+    void give(char* p) {   // of take()
         std::lock_guard<std::mutex> lock(mu_);
-        free_.push_back(p);
+        free_[n_free_++] = p;
     }
 
 private:
     std::mutex mu_;
     char* base_ = nullptr;
     bool failed_ = false;
-    std::vector<char*> free_;
+    char* free_[kSlots];
+    int n_free_ = 0;
 };
 
 bool same_phys(const epp_physics& a, const epp_physics& b) { return std::memcmp(&a, &b, sizeof a) == 0; }
@@ -1913,14 +1912,15 @@ int32_t epp_set_tuning(epp_ctx* ctx, int32_t lanes_per_particle) {
                 CK(cudaMemsetAsync(ctx->head[k], 0xff, cells * sizeof(int), ctx->stream));
             }
             if (g == 1 && ctx->sorted_once) {   // list those of the current order (a tuning switch may wait)
-                std::vector<int> st(cells + 1), list;
-                CK(cudaMemcpyAsync(st.data(), ctx->start[ctx->cur], sizeof(int) * cells, cudaMemcpyDeviceToHost, ctx->stream));
+                std::unique_ptr<int[]> st(new (std::nothrow) int[cells]);   // offsets, then the cells in their place
+                if (!st) return fail(ctx, EPP_ERR_OUT_OF_MEMORY, "host memory for %d cell offsets", ctx->n_cells);
+                CK(cudaMemcpyAsync(st.get(), ctx->start[ctx->cur], sizeof(int) * cells, cudaMemcpyDeviceToHost, ctx->stream));
                 CK(cudaStreamSynchronize(ctx->stream));
+                int n_occ = 0;
                 for (int c = 0; c < ctx->n_cells; ++c)
-                    if (st[c + 1] > st[c]) list.push_back(c);
-                const int n_occ = (int)list.size();
+                    if (st[c + 1] > st[c]) st[n_occ++] = c;   // n_occ <= c: only offsets already read
                 if (n_occ > 0)
-                    CK(cudaMemcpyAsync(ctx->occ[ctx->cur], list.data(), sizeof(int) * n_occ, cudaMemcpyHostToDevice, ctx->stream));
+                    CK(cudaMemcpyAsync(ctx->occ[ctx->cur], st.get(), sizeof(int) * n_occ, cudaMemcpyHostToDevice, ctx->stream));
                 CK(cudaMemcpyAsync(ctx->meta[ctx->cur], &n_occ, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
                 CK(cudaStreamSynchronize(ctx->stream));
             }
