@@ -88,9 +88,10 @@ struct State {
     int* id;         // 0-based row of the particle in the caller's matrices
     int* cell;       // 0-based cell (n_cells = dead bin)
     float4* rp4;     // (rho, p, p/rho^2, 1/rho) that the next momentum pass reads
-    float4* rec;     // 2D: what the momentum pass gathers of a neighbour, in one 32-byte load: (x, y, vx,
-                     // vy), (h, m, rho, p/rho^2), written with rp4.  Like rp4, one buffer serves both
-                     // state sets: it holds the current order.
+    float4* rec;     // What the momentum pass gathers of a neighbour, written with rp4.  2D: all of it in one
+                     // 32-byte load, (x, y, vx, vy), (h, m, rho, p/rho^2); 3D: beside xh and vm, (rho,
+                     // p/rho^2) of two particles per float4.  Like rp4, one buffer serves both state sets:
+                     // it holds the current order.
 };
 
 struct NeighbourList {   // EPP_SEARCH_EMIT_LIST output, column-major [k * cap + i]
@@ -237,7 +238,7 @@ __device__ __forceinline__ float4 make_rp4(float rho, float p) {
     return make_float4(rho, p, __fdiv_rn(p, __fmul_rn(rho, rho)), __fdiv_rn(1.0f, rho));
 }
 
-// rp4 of particle i and, in 2D, its neighbour record.
+// rp4 of particle i and its neighbour record.
 template <int D>
 __device__ __forceinline__ void store_rp(const State& s, int i, float4 rp) {
     s.rp4[i] = rp;
@@ -245,6 +246,8 @@ __device__ __forceinline__ void store_rp(const State& s, int i, float4 rp) {
         const float4 x = s.xh[i], v = s.vm[i];
         s.rec[2 * (size_t)i] = make_float4(x.x, x.y, v.x, v.y);
         s.rec[2 * (size_t)i + 1] = make_float4(x.w, v.w, rp.x, rp.z);
+    } else {
+        reinterpret_cast<float2*>(s.rec)[i] = make_float2(rp.x, rp.z);
     }
 }
 

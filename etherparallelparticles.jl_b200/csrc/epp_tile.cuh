@@ -466,7 +466,8 @@ struct ListTerm<D, CPMom<D, FUSED, false>> {
         TargetConst tc;
     };
     struct Rec3 {
-        float4 x, v, rp;
+        float4 x, v;
+        float2 rz;
     };
     using Rec = typename std::conditional<D == 2, Rec8, Rec3>::type;
     struct Term {
@@ -481,7 +482,7 @@ struct ListTerm<D, CPMom<D, FUSED, false>> {
     }
     static __device__ __forceinline__ Rec load(const PairArgs& A, const Act&, const Me&, int j, int) {
         if constexpr (D == 2) return load_rec(A.s.rec, j);
-        else return Rec{__ldg(&A.s.xh[j]), __ldg(&A.s.vm[j]), __ldg(&A.s.rp4[j])};
+        else return Rec{__ldg(&A.s.xh[j]), __ldg(&A.s.vm[j]), __ldg(reinterpret_cast<const float2*>(A.s.rec) + j)};
     }
     static __device__ __forceinline__ Term term(const Act& act, const Me& m, const Rec& r, int tj) {
         float px, py, ux, uy;   // the neighbour's position and velocity
@@ -505,7 +506,7 @@ struct ListTerm<D, CPMom<D, FUSED, false>> {
             t.dz = __fsub_rn(m.z, r.x.z);
             dr2 = __fadd_rn(dr2, __fmul_rn(t.dz, t.dz));
             vdx = __fmaf_rn(t.dz, __fsub_rn(m.vz, r.v.z), vdx);
-            t.f = act.pair_force(m.s, tj, r.x.w, r.v.w, r.rp.x, r.rp.z, dr2, vdx, m.tc);
+            t.f = act.pair_force(m.s, tj, r.x.w, r.v.w, r.rz.x, r.rz.y, dr2, vdx, m.tc);
         }
         return t;
     }
