@@ -185,16 +185,17 @@ struct CPCont {
         return term(self(i), fetch(j, ti, tj), ti, tj, xj, g, tc);
     }
     __device__ __forceinline__ void end(int i, int ti, float4 sum, int cnt) const {
-        ncount[i] = cnt;
-        const float rho_i = s.rho[i];
+        const float rho_i = s.rho[i];   // all loads before the first store
+        const int inst = inst_of(s.tagm[i]);
+        const RecSelf me = rec_self<D>(s, i);
         const float drho = FUSED ? sum.x : s.drho[i] + sum.x;
+        ncount[i] = cnt;
         s.drho[i] = drho;
         if (ti == P.fluid || ti == P.wall) {
-            const int inst = inst_of(s.tagm[i]);
             const float rho = __fadd_rn(rho_i, __fmul_rn(drho, P.dt_of(inst)));
-            store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)));
+            store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)), me);
         } else {
-            store_rp<D>(s, i, make_rp4(rho_i, s.p[i]));
+            store_rp<D>(s, i, make_rp4(rho_i, s.p[i]), me);
         }
     }
     __device__ __forceinline__ void end_idle(int i, int ti) const { end(i, ti, make_float4(0, 0, 0, 0), 0); }

@@ -323,28 +323,40 @@ __global__ void k_rank_gather(int n, int n_cells, const int2* link, const int2* 
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int2 c = cs[i];
+    // in flight while the rank is found, and none behind a store (a load cannot pass one): 18.9 -> 14.8 us at
+    // 515,018 particles, 182 -> 160 at 6,207,228
+    const typename Mover::Item m = mv.load(i);
     const int dst = sorted_place(i, c, n_cells, link, head, start);
     if (dst < 0 || dst >= n) {
         atomicOr(status, EPP_STATUS_QUEUE);
         return;
     }
-    mv(i, dst, c.x);
+    mv.store(m, dst, c.x);
 }
 
 // Mover of the per-call search: every state array follows the particle.
 struct MoverAll {
     State a, b;
-    __device__ __forceinline__ void operator()(int src, int dst, int c) const {
-        b.xh[dst] = a.xh[src];
-        b.vm[dst] = a.vm[src];
-        b.dv[dst] = a.dv[src];
-        b.comp[dst] = a.comp[src];
-        b.rho[dst] = a.rho[src];
-        b.drho[dst] = a.drho[src];
-        b.vol[dst] = a.vol[src];
-        b.p[dst] = a.p[src];
-        b.tagm[dst] = a.tagm[src];
-        b.id[dst] = a.id[src];
+    struct Item {
+        float4 xh, vm, dv, comp;
+        float rho, drho, vol, p;
+        int tagm, id;
+    };
+    __device__ __forceinline__ Item load(int src) const {
+        return Item{a.xh[src],   a.vm[src],  a.dv[src], a.comp[src], a.rho[src],
+                    a.drho[src], a.vol[src], a.p[src],  a.tagm[src], a.id[src]};
+    }
+    __device__ __forceinline__ void store(const Item& m, int dst, int c) const {
+        b.xh[dst] = m.xh;
+        b.vm[dst] = m.vm;
+        b.dv[dst] = m.dv;
+        b.comp[dst] = m.comp;
+        b.rho[dst] = m.rho;
+        b.drho[dst] = m.drho;
+        b.vol[dst] = m.vol;
+        b.p[dst] = m.p;
+        b.tagm[dst] = m.tagm;
+        b.id[dst] = m.id;
         b.cell[dst] = c;
     }
 };

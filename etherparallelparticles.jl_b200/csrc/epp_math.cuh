@@ -239,16 +239,28 @@ __device__ __forceinline__ float4 make_rp4(float rho, float p) {
 }
 
 // rp4 of particle i and its neighbour record.
+// (The record's other fields are read apart: a load behind a store cannot be issued before it.)
+struct RecSelf {
+    float4 x, v;
+};
 template <int D>
-__device__ __forceinline__ void store_rp(const State& s, int i, float4 rp) {
+__device__ __forceinline__ RecSelf rec_self(const State& s, int i) {
+    if constexpr (D == 2) return RecSelf{s.xh[i], s.vm[i]};
+    else return RecSelf{};
+}
+template <int D>
+__device__ __forceinline__ void store_rp(const State& s, int i, float4 rp, const RecSelf& me) {
     s.rp4[i] = rp;
     if (D == 2) {
-        const float4 x = s.xh[i], v = s.vm[i];
-        s.rec[2 * (size_t)i] = make_float4(x.x, x.y, v.x, v.y);
-        s.rec[2 * (size_t)i + 1] = make_float4(x.w, v.w, rp.x, rp.z);
+        s.rec[2 * (size_t)i] = make_float4(me.x.x, me.x.y, me.v.x, me.v.y);
+        s.rec[2 * (size_t)i + 1] = make_float4(me.x.w, me.v.w, rp.x, rp.z);
     } else {
         reinterpret_cast<float2*>(s.rec)[i] = make_float2(rp.x, rp.z);
     }
+}
+template <int D>
+__device__ __forceinline__ void store_rp(const State& s, int i, float4 rp) {
+    store_rp<D>(s, i, rp, rec_self<D>(s, i));
 }
 
 // A neighbour record in one 256-bit load through the read-only path.

@@ -276,6 +276,7 @@ struct ActMomG {
         float4 cp = s.comp[i];
         const int tm = s.tagm[i];
         int c = s.cell[i];
+        const int id = s.id[i];   // all loads before the first store
         const bool alive = c != dom.n_cells;
         const float dt = P.dt_of(inst_of(tm));
         if (alive && ti == P.fluid && a) {
@@ -301,7 +302,7 @@ struct ActMomG {
                 atomicOr(status, EPP_STATUS_KILLED);
             }
         }
-        bin_particle(F.bin, dom.n_cells, i, s.id[i], c);
+        bin_particle(F.bin, dom.n_cells, i, id, c);
     }
 };
 

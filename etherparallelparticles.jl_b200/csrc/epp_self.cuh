@@ -123,26 +123,41 @@ struct MoverFused {
     const int* start_old;
     int n_cells;
     int fluid, wall;
-    __device__ __forceinline__ void operator()(int src, int dst, int c) const {
-        const float4 vm = F.vm[src];
-        b.xh[dst] = F.xh[src];
-        b.vm[dst] = vm;
-        b.comp[dst] = F.comp[src];
-        const int tm = a.tagm[src];
-        b.tagm[dst] = tm;
-        b.id[dst] = a.id[src];
-        b.cell[dst] = c;
-        const int t = tag_of(tm);
+    struct Item {
+        float4 xh, vm, comp;
+        float rho, p, vol;
+        int tagm, id;
+    };
+    __device__ __forceinline__ Item load(int src) const {
+        Item m;
+        m.xh = F.xh[src];
+        m.vm = F.vm[src];
+        m.comp = F.comp[src];
+        m.tagm = a.tagm[src];
+        m.id = a.id[src];
+        const float2 rp = *reinterpret_cast<const float2*>(&a.rp4[src]);
+        const int t = tag_of(m.tagm);
         if (src < start_old[n_cells] && (t == fluid || t == wall)) {
-            const float4 rp = a.rp4[src];
-            b.rho[dst] = rp.x;
-            b.p[dst] = rp.y;
-            b.vol[dst] = __fdiv_rn(vm.w, rp.x);
+            m.rho = rp.x;
+            m.p = rp.y;
+            m.vol = __fdiv_rn(m.vm.w, rp.x);
         } else {
-            b.rho[dst] = a.rho[src];
-            b.p[dst] = a.p[src];
-            b.vol[dst] = a.vol[src];
+            m.rho = a.rho[src];
+            m.p = a.p[src];
+            m.vol = a.vol[src];
         }
+        return m;
+    }
+    __device__ __forceinline__ void store(const Item& m, int dst, int c) const {
+        b.xh[dst] = m.xh;
+        b.vm[dst] = m.vm;
+        b.comp[dst] = m.comp;
+        b.rho[dst] = m.rho;
+        b.p[dst] = m.p;
+        b.vol[dst] = m.vol;
+        b.tagm[dst] = m.tagm;
+        b.id[dst] = m.id;
+        b.cell[dst] = c;
     }
 };
 

@@ -535,7 +535,9 @@ constexpr bool kListInter = D == 3 && Act::NC == 3;
 // few warps in flight, one thread's serial walk.  Lanes that share a particle gather consecutive
 // entries, whose records share cache lines: 3D momentum, 955,668 particles, 308 us with L = 1 and 271
 // with L = 4 (three 16-byte gathers each way; one 32-byte record for x, v made it no faster, as half as
-// many particles share a line).  In 2D a neighbour's record fits one 32-byte load: momentum 79 -> 68 us
+// many particles share a line); 259 with (rho, p/rho^2) in 8 bytes as the third gather, 1968 -> 1870 at
+// 6,207,228, where L = 2, 8 and 16 took 2270, 2420 and 3500.  3D continuity there: 1443 with L = 1, 1553
+// with four partial sums in L = 4.  In 2D a neighbour's record fits one 32-byte load: momentum 79 -> 68 us
 // at 515,018 particles.
 // EPI: fused momentum step (integrate + bin for every particle, dead bin included; block 0 clears the
 // scan state).
@@ -546,17 +548,23 @@ __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 bl
     using T = ListTerm<D, Act>;
     constexpr bool ROW = ListConf<D>::ROW;
     constexpr bool INTER = kListInter<D, Act> && L > 1;
-    const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
     const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const int i = (int)(tid / L), g = (int)(tid % L);
+    // what the pass starts from, read at once: one after the other (alive count, then tag, nCount, first
+    // entry) these cost four latencies (2D momentum 254 -> 243 us at 2,030,018 particles with the epilogue's
+    // loads before its stores, 3D 261 -> 250 at 955,668)
+    const int ic = min(i, A.n_max - 1);
+    const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
+    const float4 xi = A.s.xh[ic];
+    const int ti = tag_of(A.s.tagm[ic]), cnt = ncount[ic];
+    const int* const first_entry = ROW ? M.list + (size_t)ic * ListConf<D>::LCAP + g : M.list + ic + (size_t)g * M.cap;
+    int en = 0;
+    if constexpr (!(L == 1 && ROW)) en = ROW ? *first_entry : __ldcs(first_entry);   // stale where the list is empty
     if (i < n_alive) {
-        const float4 xi = A.s.xh[i];
-        const int ti = tag_of(A.s.tagm[i]);
         if (ti < 1 || ti > A.n_tags || !act.wants(ti)) {
             if (g == 0) act.end_idle(i, ti);
             return;
         }
-        const int cnt = ncount[i];
         if (cnt > ListConf<D>::LCAP) {   // more neighbours than the list keeps
             if (g == 0) {
                 const TargetConst tc = target_const<D>(xi.w);
@@ -576,7 +584,7 @@ __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 bl
             const int4* row = reinterpret_cast<const int4*>(M.list + (size_t)i * ListConf<D>::LCAP);
             int4 q = cnt > 0 ? row[0] : make_int4(0, 0, 0, 0);
             int4 qn = cnt > 4 ? row[1] : make_int4(0, 0, 0, 0);
-            int en = cnt > 0 ? q.x : list_entry(0, 1);
+            en = cnt > 0 ? q.x : list_entry(0, 1);
             EPP_CHECK(entry_index(en) < A.n_max, 16, entry_index(en));
             typename T::Rec rn = T::load(A, act, me, entry_index(en), entry_tag(en));
             for (int k0 = 0; k0 < cnt; k0 += 4) {
@@ -600,12 +608,11 @@ __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 bl
         } else {
             // the lane's next entry is read ahead.  2D lists are column-major and read once each:
             // streaming loads keep the L1 for the records.
-            const int* list = ROW ? M.list + (size_t)i * ListConf<D>::LCAP + g : M.list + i + (size_t)g * M.cap;
+            const int* list = first_entry;
             const size_t stride = ROW ? L : (size_t)L * M.cap;
             const int first = (int)(threadIdx.x & 31u & ~(unsigned)(L - 1));
             const unsigned group = L == 1 ? 0u : ((1u << L) - 1u) << first;
             auto read = [&]() { return ROW ? *list : __ldcs(list); };
-            int en = g < cnt ? read() : 0;
             for (int k0 = 0; k0 < cnt; k0 += L) {
                 typename T::Term t{};
                 if (k0 + g < cnt) {
@@ -638,7 +645,7 @@ __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 bl
         }
         if (g == 0) act.end(i, ti, make_float4(acc.x, acc.y, acc.z, 0.0f), cnt);
     } else if (EPI && i < A.n_max && g == 0) {
-        act.end_idle(i, tag_of(A.s.tagm[i]));
+        act.end_idle(i, ti);
     }
 }
 
