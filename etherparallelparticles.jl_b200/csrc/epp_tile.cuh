@@ -539,8 +539,7 @@ constexpr bool kListInter = D == 3 && Act::NC == 3;
 // 6,207,228, where L = 2, 8 and 16 took 2270, 2420 and 3500.  3D continuity there: 1443 with L = 1, 1553
 // with four partial sums in L = 4.  In 2D a neighbour's record fits one 32-byte load: momentum 79 -> 68 us
 // at 515,018 particles.
-// EPI: fused momentum step (integrate + bin for every particle, dead bin included; block 0 clears the
-// scan state).
+// EPI: fused momentum step (integrate + bin for every particle, dead bin included).
 template <int D, class Act, bool EPI, int L>
 __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 blocks (56 registers) beat 7, 8 and 10
     k_list(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M, const int* ncount,
@@ -613,15 +612,46 @@ __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 bl
             const int first = (int)(threadIdx.x & 31u & ~(unsigned)(L - 1));
             const unsigned group = L == 1 ? 0u : ((1u << L) - 1u) << first;
             auto read = [&]() { return ROW ? *list : __ldcs(list); };
+            // 2D, four lanes: the next record in flight too (step 22.5 -> 21.1 us at 1,418 particles); 3D loses to
+            // the registers it takes (momentum 250 -> 300 us at 955,668)
+            constexpr bool PIPE = L > 1 && D == 2;
+            typename T::Rec rn;
+            int tn = 1;
+            if (PIPE && g < cnt) {
+                EPP_CHECK(entry_index(en) < A.n_max, 16, entry_index(en));
+                tn = entry_tag(en);
+                rn = T::load(A, act, me, entry_index(en), tn);
+                if (L + g < cnt) {
+                    list += stride;
+                    en = read();
+                }
+            }
             for (int k0 = 0; k0 < cnt; k0 += L) {
                 typename T::Term t{};
                 if (k0 + g < cnt) {
-                    const int j = entry_index(en), tj = entry_tag(en);
-                    EPP_CHECK(j < A.n_max, 16, j);
-                    const typename T::Rec r = T::load(A, act, me, j, tj);
-                    if (k0 + L + g < cnt) {
-                        list += stride;
-                        en = read();
+                    typename T::Rec r;
+                    int tj;
+                    if (PIPE) {
+                        r = rn;
+                        tj = tn;
+                        if (k0 + L + g < cnt) {
+                            EPP_CHECK(entry_index(en) < A.n_max, 16, entry_index(en));
+                            tn = entry_tag(en);
+                            rn = T::load(A, act, me, entry_index(en), tn);
+                            if (k0 + 2 * L + g < cnt) {
+                                list += stride;
+                                en = read();
+                            }
+                        }
+                    } else {
+                        const int j = entry_index(en);
+                        tj = entry_tag(en);
+                        EPP_CHECK(j < A.n_max, 16, j);
+                        r = T::load(A, act, me, j, tj);
+                        if (k0 + L + g < cnt) {
+                            list += stride;
+                            en = read();
+                        }
                     }
                     t = T::term(act, me, r, tj);
                     if (L == 1 || INTER) T::add(acc, t);

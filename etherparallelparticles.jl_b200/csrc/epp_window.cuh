@@ -62,6 +62,16 @@ __device__ __forceinline__ RowWin row_range(const PairArgs& A, int row, int xa, 
     return w;
 }
 
+// What a search pass starts from, read at once rather than after the alive count (i may lie beyond it).
+struct WinSelf {
+    float4 x;
+    int n_alive, tag, cell;
+};
+__device__ __forceinline__ WinSelf win_self(const PairArgs& A, int i) {
+    const int k = min(i, A.n_max - 1);
+    return WinSelf{A.s.xh[k], min(A.start[A.dom.n_cells], A.n_max), tag_of(A.s.tagm[k]), A.s.cell[k]};
+}
+
 constexpr int kStage2 = 240;   // staged candidates per warp: 7 blocks of 128 threads still fit an SM
 
 template <class Act>
@@ -164,18 +174,19 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     Stage2<Act>& S = reinterpret_cast<Stage2<Act>*>(win_smem)[threadIdx.x >> 5];
-    const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int w0 = i - lane;
+    const WinSelf me0 = win_self(A, i);
+    const int n_alive = me0.n_alive;
     int cnt = 0;
     if (w0 < n_alive) {   // warp-uniform
         const bool on = i < n_alive;
-        const int c = A.s.cell[min(i, n_alive - 1)];
+        const int c = __shfl_sync(FULL, me0.cell, min(lane, n_alive - 1 - w0));
         EPP_CHECK(!__any_sync(FULL, c < 0 || c >= A.dom.n_cells), 34, c);
         const int rid = A.dom.by[0].div(max(c, 0)), cx = c - rid * A.dom.n[0];
         const int z = A.dom.by[1].div(rid), y = rid - z * A.dom.n[1];
-        const float4 xi = on ? A.s.xh[i] : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-        const int ti = on ? tag_of(A.s.tagm[i]) : 0;
+        const float4 xi = on ? me0.x : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+        const int ti = on ? me0.tag : 0;
         const bool valid = on && ti >= 1 && ti <= A.n_tags;
         const unsigned amask = valid ? A.adj[ti - 1] : 0u;   // bits of valid tags only
         const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
@@ -403,18 +414,19 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     Stage3& S = reinterpret_cast<Stage3*>(win_smem)[threadIdx.x >> 5];
-    const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int w0 = i - lane;
+    const WinSelf me0 = win_self(A, i);
+    const int n_alive = me0.n_alive;
     int cnt = 0;
     if (w0 < n_alive) {   // warp-uniform
         const bool on = i < n_alive;
-        const int c = A.s.cell[min(i, n_alive - 1)];
+        const int c = __shfl_sync(FULL, me0.cell, min(lane, n_alive - 1 - w0));
         EPP_CHECK(!__any_sync(FULL, c < 0 || c >= A.dom.n_cells), 36, c);
         const int rid = A.dom.by[0].div(max(c, 0)), cx = c - rid * A.dom.n[0];
         const int z = A.dom.by[1].div(rid), y = rid - z * A.dom.n[1];
-        const float4 xi = on ? A.s.xh[i] : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
-        const int ti = on ? tag_of(A.s.tagm[i]) : 0;
+        const float4 xi = on ? me0.x : make_float4(0.0f, 0.0f, 0.0f, 1.0f);
+        const int ti = on ? me0.tag : 0;
         const bool valid = on && ti >= 1 && ti <= A.n_tags;
         const unsigned amask = valid ? A.adj[ti - 1] : 0u;   // bits of valid tags only
         const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
@@ -572,16 +584,15 @@ __global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairA
     constexpr int P = 128 / L, CAP = ListConf<D>::LCAP, NR = D == 3 ? 9 : 3;
     __shared__ int s_e[P][CAP + 1];                           // accepted entries (odd rows: no bank conflicts)
     __shared__ float s_t[Act::NC != 0 ? P : 1][CAP + 1];      // their terms
-    const int n_alive = min(A.start[A.dom.n_cells], A.n_max);
     const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) / L);
+    const WinSelf me0 = win_self(A, i);
     const int g = threadIdx.x % L, p = threadIdx.x / L;
     const int first = (int)(threadIdx.x & 31u & ~(unsigned)(L - 1));
     const unsigned group = ((1u << L) - 1u) << first;
     int cnt = 0;
-    if (i < n_alive) {
-        const float4 xi = A.s.xh[i];
-        const int ti = tag_of(A.s.tagm[i]);
-        const int c = A.s.cell[i];
+    if (i < me0.n_alive) {
+        const float4 xi = me0.x;
+        const int ti = me0.tag, c = me0.cell;
         if (ti < 1 || ti > A.n_tags) {
             if (g == 0) {
                 act.end_idle(i, ti);
