@@ -48,10 +48,10 @@ B_ALG_STAGE = {"momentum_integrate_bin": {2: 80.0, 3: 108.0}, "scan": {2: 5.0, 3
                "search": {2: 12.0, 3: 16.0}, "continuity": {2: 12.0, 3: 16.0}}
 PAIR_STAGES = ("momentum_integrate_bin", "search", "continuity")
 KERNEL_OF_STAGE = {"momentum_integrate_bin": "k_list<CPMom> (momentum + integrate + bin, fused)",
-                   "scan": "k_scan (decoupled look-back exclusive scan)",
-                   "scatter": "k_scatter (arrival-order scatter)",
+                   "scan": "k_scan_tiles (exclusive scan from the tile counters of the bin)",
+                   "scatter": "none (the gather ranks from the linked cell lists)",
                    "rank_gather": "k_rank_gather (rank by id + state gather + density update)",
-                   "search": "k_build (neighbour lists + nCount)",
+                   "search": "k_win_build3 (neighbour lists + nCount)",
                    "continuity": "k_list<CPCont> (continuity + density preview, fused)"}
 
 

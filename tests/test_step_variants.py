@@ -290,3 +290,27 @@ def test_cell_lists_after_uploads_and_family_switches(steps, family, dead):
         d.ctx.search(SYM, abi.EPP_ACTION_NONE, c.physics, 0)
     assert d.ctx.synchronize(raise_on_status=False) & ~abi.EPP_STATUS_KILLED == 0
     d.close()
+
+
+# The allocation-free sort on particles in no cell order: a shuffled column, a cell of many particles, and
+# some outside the domain; the context's cell lists.
+@pytest.mark.gpu
+@pytest.mark.parametrize("dim,dx", [(2, 0.05), (2, 0.0231), (3, 0.1), (3, 0.041)])
+@pytest.mark.parametrize("crowd,outside", [(0, 0), (700, 33)])
+def test_noalloc_sort_of_shuffled_particles(dim, dx, crowd, outside):
+    from test_zz_no_alloc import _noalloc
+    c = casegen.dam_break_2d(dx=dx, max_neighbour_number=1) if dim == 2 else \
+        casegen.dam_break_3d(dx=dx, max_neighbour_number=1)
+    rng = np.random.default_rng(31)
+    x = c.ps["PositionVec"][rng.permutation(c.n)].copy()
+    x[: min(crowd, c.n // 3)] = x[c.n // 2]
+    x[c.n - outside:] = 100.0
+    c.ps["PositionVec"] = x
+    d = device(c)
+    d.ctx.search(SYM, abi.EPP_ACTION_NONE, c.physics, 0)
+    counts, offsets, ids = d.ctx.cell_stats()
+    got_c, got_o, got_ids, n_alive = _noalloc(c.domain, x)
+    assert n_alive == c.n - outside
+    assert np.array_equal(got_c, counts) and np.array_equal(got_o[:len(offsets)], offsets[:len(got_o)])
+    assert np.array_equal(got_ids[:n_alive], ids[:n_alive])
+    d.close()
