@@ -37,8 +37,8 @@ import numpy as np  # noqa: E402
 #   scatter / reorder  read key + rank; gather state; write sorted state           2D 80,  3D 104
 #   continuity         read x, v, id; write drho                                   2D 24,  3D 32
 #   whole step                                                                     2D 189, 3D 245
-# The six kernels of a step re-split those stages: the momentum pass also bins (momentum + hash
-# and count), the reorder is the scatter (key + rank, 8 B) and the rank-by-id gather (the rest),
+# The kernels of a step re-split those stages: the momentum pass also bins (momentum + hash and
+# count), the reorder is the scatter (key + rank, 8 B; no kernel of its own) and the rank-by-id gather,
 # and the continuity stage is split between the search pass (reads x and id) and the continuity
 # pass (reads v, writes drho).  The per-kernel figures add up to the whole step.
 B_ALG_STEP = {2: 189.0, 3: 245.0}
@@ -465,7 +465,7 @@ def run_batch(args):
             "pairs_per_s": pairs / (ms * 1e-3) if world == 1 else None,
             "energy_drift": {"steps": S, "bar": 1e-4, "instances": drift,
                              "max_abs_diff": max(v["abs_diff"] for v in drift.values())},
-            "gpu_launches": 5 * args.steps,
+            "gpu_launches": 4 * args.steps,
             "roofline": {"bound": "hbm", "stage_ms": dict(zip(STAGES, [round(float(x), 4) for x in stage])),
                          "achieved": B_ALG_STEP[2] * b.n / (step_ms * 1e-3) / 1e9,
                          "peak": peaks.get("hbm_gbs", 6650.0), "unit": "GB/s",
@@ -591,7 +591,7 @@ def run_serve(args):
            "speedup_vs_plain": served["sims_per_s"] / plain_all["sims_per_s"],
            "p99_vs_plain": served["latency_p99_s"] / plain_all["latency_p99_s"],
            "autotune": {k: {"family": v[0], "block_threads": v[1]} for e in every for k, v in e["tuned"].items()},
-           "gpu_launches": 6 * args.sim_steps * len(specs),
+           "gpu_launches": args.sim_steps * sum(5 if s.dim == 3 else 4 for s in specs),
            "clocks": every[0]["clocks"],
            "e2e": {"value": served["sims_per_s"], "unit": "sims/s",
                    "h2d_bytes_per_step": int(h2d / args.sim_steps / len(specs)), "d2h_bytes_per_step": 0,
@@ -755,7 +755,7 @@ def main():
             "step_roofline_frac": step_bytes / (step_ms * 1e-3) / 1e9 / peak,
             # per fused step: momentum+integrate+bin, scan, scatter, rank+gather, search, continuity
             # (2D family 0 and the other families run the continuity action inside the search pass)
-            "gpu_launches": (6 if (args.lanes == 0 and dim == 3) or args.lanes == 64 else 5) * args.steps
+            "gpu_launches": (5 if (args.lanes == 0 and dim == 3) or args.lanes == 64 else 4) * args.steps
                             + (2 * (args.steps // phys.filter_interval) if phys.filter_interval else 0),
             "roofline": {"bound": "hbm", "kernel": kernel_of[dom_stage], "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,
@@ -936,7 +936,7 @@ def measure_3d(device, steps=20, warmup=3):
             "pairs_per_step": pairs / steps,
             "step_hbm_gbs_algorithmic": gbs, "step_roofline_frac": gbs / peak,
             "stage_ms": dict(zip(STAGES, [round(float(x), 5) for x in stage])),
-            "gpu_launches": 6 * steps, "clocks": clk, "device_status": st,
+            "gpu_launches": 5 * steps, "clocks": clk, "device_status": st,
             "leg_seconds": time.perf_counter() - t_leg}
 
 
@@ -1028,7 +1028,7 @@ def measure_batch(device, steps=50, warmup=3, instances=256, sim_steps=2000):
             "autotune": {"family": tuned[0], "block_threads": tuned[1], "resort_every": 1},
             "energy_drift": {"steps": S, "bar": 1e-4, "instances": drift,
                              "max_abs_diff": max(v["abs_diff"] for v in drift.values())},
-            "gpu_launches": 5 * steps, "clocks": clk, "device_status": st,
+            "gpu_launches": 4 * steps, "clocks": clk, "device_status": st,
             "leg_seconds": time.perf_counter() - t_leg}
 
 
