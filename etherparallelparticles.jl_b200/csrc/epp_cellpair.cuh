@@ -146,7 +146,7 @@ struct CPCont {
         if (!(ff || fw || wf)) return out;
         // every operation rounded on its own (no contraction into fused multiply-adds), so the term
         // is the same bit for bit wherever a pass evaluates it
-        const float r = root(g.dr2);
+        const float r = sqrtf(g.dr2);
         float hinv = tc.hinv, kdw = tc.kdw;
         if (xj.w != tc.h) {
             hinv = invharmonic_exact(tc.h, xj.w);
@@ -169,7 +169,7 @@ struct CPCont {
         float ex, ey, vx, vy;
         f2_unpack(f2_mul(d, d), ex, ey);
         f2_unpack(f2_mul(d, f2_sub(vi, f2_pack(nb.x, nb.y))), vx, vy);
-        const float q = __fmul_rn(root(__fadd_rn(ex, ey)), tc.hinv);
+        const float q = __fmul_rn(sqrtf(__fadd_rn(ex, ey)), tc.hinv);
         float dwr;
         if constexpr (GEN) {
             dwr = pair_dwr<D, GEN>(P.kernel, q, tc.hinv, tc.kdw);
@@ -307,7 +307,7 @@ struct CPMom {
             kdw = c.y;
             hh = c.z;
         }
-        const float u = fmaxf(__fsub_rn(2.0f, __fmul_rn(root(dr2), hinv)), 0.0f);   // W = dW = 0 at q >= 2
+        const float u = fmaxf(__fsub_rn(2.0f, __fmul_rn(sqrtf(dr2), hinv)), 0.0f);   // W = dW = 0 at q >= 2
         const float md = __fmul_rn(mj, __fmul_rn(kdw, __fmul_rn(__fmul_rn(u, u), u)));
         float s = __fadd_rn(me.rp.z, zj);                                              // iClassicPressure!
         if (!ff) s = __fmul_rn(__fmaf_rn(me.rp.y, rcp_fast(rhoj), __fmul_rn(zj, rhoj)), me.rp.w);   // iBalancedPressure!
@@ -338,7 +338,7 @@ struct CPMom {
             const bool ff = tj == P.fluid;
             const bool fw = tj == P.wall;
             if (!(ff || fw)) return out;
-            const float r = root(g.dr2);
+            const float r = sqrtf(g.dr2);
             float hinv, kdw, hh;
             pair_consts<D>(tc, xj.w, hinv, kdw, hh);
             const float dwr = pair_dwr<D, GEN>(P.kernel, r * hinv, hinv, kdw);

@@ -299,19 +299,6 @@ __device__ __forceinline__ f32x2 f2_mul(f32x2 a, f32x2 b) {
     return r;
 }
 
-
-// Square root by Newton's iteration on 1 / sqrt(x) from the approximate reciprocal root, the last
-// step on the residual x - s^2: no branch for special operands.  Equal to the IEEE square root for
-// every mantissa (both binades of 1, 2^-20, 2^-40, 2^20 and 2^-93 compared with __fsqrt_rn on
-// B200); arguments below 1e-30 (coincident particles) give 1e-15, whose q = r / h rounds as 0 does
-// in 2 - q.  Infinity gives NaN: outside the support, as the infinite root is.
-__device__ __forceinline__ float root(float x) {
-    x = fmaxf(x, 1e-30f);
-    float y;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    const float s = __fmul_rn(x, y);
-    return __fmaf_rn(__fmaf_rn(-s, s, x), __fmul_rn(0.5f, y), s);
-}
 // Approximate reciprocal (1 ulp) without the scaling that a division of possibly subnormal operands
 // carries along: for densities and squared lengths.
 __device__ __forceinline__ float rcp_fast(float x) {
