@@ -968,7 +968,7 @@ int run_interaction(epp_ctx* ctx, int action, const epp_physics* phys) {
     }
     if (action == EPP_ACTION_DAMBREAK_MOMENTUM) {
         k_prep_rp4<D><<<blocks_for(ctx->n), kThreads, 0, ctx->stream>>>(ctx->start[ctx->cur], ctx->n_cells, ctx->n,
-                                                                      ctx->S[ctx->cur]);
+                                                                      ctx->S[ctx->cur], phys->fluid_tag);
         CK_LAUNCH();
         ActMomG<D, false> act;
         act.s = ctx->S[ctx->cur];

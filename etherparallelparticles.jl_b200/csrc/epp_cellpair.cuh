@@ -193,9 +193,9 @@ struct CPCont {
         s.drho[i] = drho;
         if (ti == P.fluid || ti == P.wall) {
             const float rho = __fadd_rn(rho_i, __fmul_rn(drho, P.dt_of(inst)));
-            store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)), me);
+            store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)), me, ti == P.fluid);
         } else {
-            store_rp<D>(s, i, make_rp4(rho_i, s.p[i]), me);
+            store_rp<D>(s, i, make_rp4(rho_i, s.p[i]), me, false);
         }
     }
     __device__ __forceinline__ void end_idle(int i, int ti) const { end(i, ti, make_float4(0, 0, 0, 0), 0); }
@@ -295,8 +295,10 @@ struct CPMom {
     // and artificial viscosity) as one factor: du += pair_force d.  Straight-line (the viscosity is a
     // select: warps hold approaching and receding pairs alike) with one reciprocal for the viscosity's
     // three densities; every operation has its own rounding or an explicit fused multiply-add, so the
-    // value does not depend on the kernel that evaluates it.  z_j = p_j / rho_j^2.
-    __device__ __forceinline__ float pair_force(const Self& me, int tj, float hj, float mj, float rhoj, float zj,
+    // value does not depend on the kernel that evaluates it.  pz is what the pressure term needs of the
+    // neighbour: p_j / rho_j^2 of a fluid one, p_j of a wall, whose sum with p_i comes first (pressures
+    // of opposite sign cancel exactly).
+    __device__ __forceinline__ float pair_force(const Self& me, int tj, float hj, float mj, float rhoj, float pz,
                                                 float dr2, float vdx, const TargetConst& tc) const {
         const DevPhys& P = m.P;
         const bool ff = tj == P.fluid;
@@ -309,8 +311,8 @@ struct CPMom {
         }
         const float u = fmaxf(__fsub_rn(2.0f, __fmul_rn(sqrtf(dr2), hinv)), 0.0f);   // W = dW = 0 at q >= 2
         const float md = __fmul_rn(mj, __fmul_rn(kdw, __fmul_rn(__fmul_rn(u, u), u)));
-        float s = __fadd_rn(me.rp.z, zj);                                              // iClassicPressure!
-        if (!ff) s = __fmul_rn(__fmaf_rn(me.rp.y, rcp_fast(rhoj), __fmul_rn(zj, rhoj)), me.rp.w);   // iBalancedPressure!
+        float s = __fadd_rn(me.rp.z, pz);                                                               // iClassicPressure!
+        if (!ff) s = __fmul_rn(__fmul_rn(__fadd_rn(me.rp.y, pz), me.rp.w), __frcp_rn(rhoj));   // iBalancedPressure!
         // sArtificialViscosity!: approaching pairs only
         const bool ref = P.visc == EPP_VISCOSITY_REFERENCE;
         const float az = __fmaf_rn(__fmul_rn(0.01f, hh), hh, dr2);
@@ -329,7 +331,7 @@ struct CPMom {
             const float4 vi = me.v, vj = nb.v;
             float vdx = __fmaf_rn(g.dy, __fsub_rn(vi.y, vj.y), __fmul_rn(g.dx, __fsub_rn(vi.x, vj.x)));
             if (D == 3) vdx = __fmaf_rn(g.dz, __fsub_rn(vi.z, vj.z), vdx);
-            const float f = pair_force(me, tj, xj.w, vj.w, nb.rp.x, nb.rp.z, g.dr2, vdx, tc);
+            const float f = pair_force(me, tj, xj.w, vj.w, nb.rp.x, tj == P.fluid ? nb.rp.z : nb.rp.y, g.dr2, vdx, tc);
             out.x = __fmul_rn(f, g.dx);
             out.y = __fmul_rn(f, g.dy);
             if (D == 3) out.z = __fmul_rn(f, g.dz);
@@ -484,7 +486,7 @@ struct CPExtrap {
     __device__ __forceinline__ void end(int i, int, float4 sum, int) const {
         if (FUSED) {
             const float p = sum.x > 0.0f ? __fdiv_rn(sum.y, sum.x) : P.p0;
-            store_rp<D>(s, i, make_rp4(s.rp4[i].x, p));
+            store_rp<D>(s, i, make_rp4(s.rp4[i].x, p), P.wall == P.fluid);
         } else {
             wv[i] += sum.x;
             wvp[i] += sum.y;

@@ -89,9 +89,9 @@ struct State {
     int* cell;       // 0-based cell (n_cells = dead bin)
     float4* rp4;     // (rho, p, p/rho^2, 1/rho) that the next momentum pass reads
     float4* rec;     // What the momentum pass gathers of a neighbour, written with rp4.  2D: all of it in one
-                     // 32-byte load, (x, y, vx, vy), (h, m, rho, p/rho^2); 3D: beside xh and vm, (rho,
-                     // p/rho^2) of two particles per float4.  Like rp4, one buffer serves both state sets:
-                     // it holds the current order.
+                     // 32-byte load, (x, y, vx, vy), (h, m, rho, pz); 3D: beside xh and vm, (rho, pz) of two
+                     // particles per float4; pz = p/rho^2 of a fluid particle, p of any other.  Like rp4,
+                     // one buffer serves both state sets: it holds the current order.
 };
 
 struct NeighbourList {   // EPP_SEARCH_EMIT_LIST output, column-major [k * cap + i]
@@ -238,7 +238,7 @@ __device__ __forceinline__ float4 make_rp4(float rho, float p) {
     return make_float4(rho, p, __fdiv_rn(p, __fmul_rn(rho, rho)), __fdiv_rn(1.0f, rho));
 }
 
-// rp4 of particle i and its neighbour record.
+// rp4 of particle i and its neighbour record (fluid: the particle has the physics' fluid tag).
 // (The record's other fields are read apart: a load behind a store cannot be issued before it.)
 struct RecSelf {
     float4 x, v;
@@ -249,18 +249,19 @@ __device__ __forceinline__ RecSelf rec_self(const State& s, int i) {
     else return RecSelf{};
 }
 template <int D>
-__device__ __forceinline__ void store_rp(const State& s, int i, float4 rp, const RecSelf& me) {
+__device__ __forceinline__ void store_rp(const State& s, int i, float4 rp, const RecSelf& me, bool fluid) {
     s.rp4[i] = rp;
+    const float pz = fluid ? rp.z : rp.y;
     if (D == 2) {
         s.rec[2 * (size_t)i] = make_float4(me.x.x, me.x.y, me.v.x, me.v.y);
-        s.rec[2 * (size_t)i + 1] = make_float4(me.x.w, me.v.w, rp.x, rp.z);
+        s.rec[2 * (size_t)i + 1] = make_float4(me.x.w, me.v.w, rp.x, pz);
     } else {
-        reinterpret_cast<float2*>(s.rec)[i] = make_float2(rp.x, rp.z);
+        reinterpret_cast<float2*>(s.rec)[i] = make_float2(rp.x, pz);
     }
 }
 template <int D>
-__device__ __forceinline__ void store_rp(const State& s, int i, float4 rp) {
-    store_rp<D>(s, i, rp, rec_self<D>(s, i));
+__device__ __forceinline__ void store_rp(const State& s, int i, float4 rp, bool fluid) {
+    store_rp<D>(s, i, rp, rec_self<D>(s, i), fluid);
 }
 
 // A neighbour record in one 256-bit load through the read-only path.

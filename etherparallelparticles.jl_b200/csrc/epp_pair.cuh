@@ -192,9 +192,9 @@ struct ActSearch {
             if (ti == P.fluid || ti == P.wall) {
                 const int inst = inst_of(s.tagm[i]);
                 const float rho = __fadd_rn(a.rho_i, __fmul_rn(a.drho, P.dt_of(inst)));
-                store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)));
+                store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)), ti == P.fluid);
             } else {
-                store_rp<D>(s, i, make_rp4(a.rho_i, s.p[i]));
+                store_rp<D>(s, i, make_rp4(a.rho_i, s.p[i]), false);
             }
         }
     }

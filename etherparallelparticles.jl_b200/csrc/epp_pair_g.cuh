@@ -161,9 +161,9 @@ struct ActContG {
         if (ti == P.fluid || ti == P.wall) {
             const int inst = inst_of(s.tagm[i]);
             const float rho = __fadd_rn(a.rho_i, __fmul_rn(drho, P.dt_of(inst)));
-            store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)));
+            store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)), ti == P.fluid);
         } else {
-            store_rp<D>(s, i, make_rp4(a.rho_i, s.p[i]));
+            store_rp<D>(s, i, make_rp4(a.rho_i, s.p[i]), false);
         }
     }
     __device__ __forceinline__ int count(const Acc& a) const { return a.cnt; }
@@ -391,11 +391,11 @@ __global__ void __launch_bounds__(128) k_pair_g(PairArgs A, Act act, unsigned lo
 
 // rp4 from the current density and pressure (per-call momentum after a density selfaction!).
 template <int D>
-__global__ void k_prep_rp4(const int* start, int n_cells, int n_max, State s) {
+__global__ void k_prep_rp4(const int* start, int n_cells, int n_max, State s, int fluid) {
     const int n_alive = min(start[n_cells], n_max);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_alive) return;
-    store_rp<D>(s, i, make_rp4(s.rho[i], s.p[i]));
+    store_rp<D>(s, i, make_rp4(s.rho[i], s.p[i]), tag_of(s.tagm[i]) == fluid);
 }
 
 }  // namespace epp

@@ -77,7 +77,7 @@ __global__ void k_filter_finish(const int* start, int n_cells, int n_max, State 
     }
     if (preview && (ti == P.fluid || ti == P.wall)) {
         const float rn = __fadd_rn(s.rho[i], __fmul_rn(s.drho[i], P.dt_of(inst)));
-        store_rp<D>(s, i, make_rp4(rn, eos(P, inst, rn)));
+        store_rp<D>(s, i, make_rp4(rn, eos(P, inst, rn)), ti == P.fluid);
     }
 }
 
@@ -108,9 +108,9 @@ __global__ void k_density_preview(const int* start, int n_cells, int n_max, Stat
     if (ti == P.fluid || ti == P.wall) {
         const int inst = inst_of(s.tagm[i]);
         const float rho = __fadd_rn(s.rho[i], __fmul_rn(s.drho[i], P.dt_of(inst)));
-        store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)));
+        store_rp<D>(s, i, make_rp4(rho, eos(P, inst, rho)), ti == P.fluid);
     } else {
-        store_rp<D>(s, i, make_rp4(s.rho[i], s.p[i]));
+        store_rp<D>(s, i, make_rp4(s.rho[i], s.p[i]), false);
     }
 }
 

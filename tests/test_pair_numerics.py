@@ -94,3 +94,25 @@ def test_continuity_of_close_pairs(h, lo):
     assert ok.sum() > 50 and (ok[0] or h > 1e-6)
     assert np.all(np.abs(got - want)[ok] <= 1e-6 * np.abs(want[ok])), np.max(np.abs(got / want - 1)[ok])
     d.close()
+
+
+# Fluid beside walls of the opposite pressure and another density: p_i + p_j is exactly zero, and so
+# is the force.
+@pytest.mark.parametrize("family", [0, 1, 4])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_opposite_pressures_of_fluid_and_wall_cancel(dim, family):
+    ps, domain, rng = pairs(dim, 0.01, 0.8, 2, tags=(FLUID, WALL))
+    n = ps["Mass"].size
+    p = rng.uniform(1.0, 1e5, n // 2).astype(np.float32)
+    ps["Pressure"] = np.stack([p, -p], 1).reshape(-1)
+    ps["Density"] = rng.uniform(700.0, 1300.0, n).astype(np.float32)
+    ps["VelocityVec"] = np.zeros((n, dim), np.float32)
+    d = device(ps, domain, family)
+    phys = physics(dim)
+    d.ctx.search(SYM, abi.EPP_ACTION_NONE, phys, 0)
+    d.ctx.interaction(MOMENTUM, phys)
+    d.ctx.synchronize()
+    d.asyncto()
+    assert np.array_equal(d.host["nCount"], np.ones(n, np.int32))
+    assert not np.any(d.host["dVelocityVec"])
+    d.close()
