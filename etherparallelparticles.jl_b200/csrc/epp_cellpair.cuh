@@ -293,9 +293,9 @@ struct CPMom {
     }
     // The benchmark physics' pair (the dam break's classic fluid-fluid, balanced fluid-wall pressure
     // and artificial viscosity) as one factor: du += pair_force d.  Straight-line (the viscosity is a
-    // select: warps hold approaching and receding pairs alike) with one reciprocal for the viscosity's
-    // three densities; every operation has its own rounding or an explicit fused multiply-add, so the
-    // value does not depend on the kernel that evaluates it.  pz is what the pressure term needs of the
+    // select: warps hold approaching and receding pairs alike), a reciprocal for each density (their product
+    // leaves FP32's range below 1e-19 and above 1e19); every operation has its own rounding or an explicit
+    // fused multiply-add, so the value does not depend on the kernel that evaluates it.  pz is what the pressure term needs of the
     // neighbour: p_j / rho_j^2 of a fluid one, p_j of a wall, whose sum with p_i comes first (pressures
     // of opposite sign cancel exactly).
     __device__ __forceinline__ float pair_force(const Self& me, int tj, float hj, float mj, float rhoj, float pz,
@@ -310,18 +310,19 @@ struct CPMom {
             hh = c.z;
         }
         const float u = fmaxf(__fsub_rn(2.0f, __fmul_rn(sqrtf(dr2), hinv)), 0.0f);   // W = dW = 0 at q >= 2
-        const float md = __fmul_rn(mj, __fmul_rn(kdw, __fmul_rn(__fmul_rn(u, u), u)));
+        const float dwr = __fmul_rn(kdw, __fmul_rn(__fmul_rn(u, u), u));
         float s = __fadd_rn(me.rp.z, pz);                                                               // iClassicPressure!
         if (!ff) s = __fmul_rn(__fmul_rn(__fadd_rn(me.rp.y, pz), me.rp.w), __frcp_rn(rhoj));   // iBalancedPressure!
+        float f = __fmul_rn(s, __fmul_rn(mj, dwr));
         // sArtificialViscosity!: approaching pairs only
-        const bool ref = P.visc == EPP_VISCOSITY_REFERENCE;
         const float az = __fmaf_rn(__fmul_rn(0.01f, hh), hh, dr2);
         const float phi = __fmul_rn(vdx, rcp_fast(__fmul_rn(hinv, az)));
-        const float k = rcp_fast(__fmul_rn(__fadd_rn(me.rp.x, rhoj), ref ? rhoj : 1.0f));
         const float w = __fmul_rn(__fmul_rn(__fmaf_rn(P.beta, phi, -__fmul_rn(P.alpha, me.c0)), phi),
-                                  __fmul_rn(k, __fmul_rn(2.0f, ref ? me.rp.w : 1.0f)));
-        if (vdx < 0.0f) s = __fadd_rn(s, w);
-        return u > 0.0f && (ff || tj == P.wall) ? -__fmul_rn(md, s) : 0.0f;
+                                  __fmul_rn(2.0f, rcp_fast(__fadd_rn(me.rp.x, rhoj))));
+        float mv = mj;
+        if (P.visc == EPP_VISCOSITY_REFERENCE) mv = __fmul_rn(__fmul_rn(mj, me.rp.w), rcp_fast(rhoj));
+        if (vdx < 0.0f) f = __fmaf_rn(w, __fmul_rn(mv, dwr), f);
+        return u > 0.0f && (ff || tj == P.wall) ? -f : 0.0f;
     }
     __device__ __forceinline__ float4 term(const Self& me, const Nb& nb, int ti, int tj, float4 xj,
                                            const PairGeo& g, const TargetConst& tc) const {

@@ -116,3 +116,40 @@ def test_opposite_pressures_of_fluid_and_wall_cancel(dim, family):
     assert np.array_equal(d.host["nCount"], np.ones(n, np.int32))
     assert not np.any(d.host["dVelocityVec"])
     d.close()
+
+
+# The pressure and viscosity of pairs over FP32's densities, p = 0 where p / rho^2 leaves the range.  Three
+# reciprocals of 1 ulp and about 25 roundings: 3 * 2^-23 + 25 * 2^-24 < 2e-6.
+@pytest.mark.parametrize("viscosity", [abi.EPP_VISCOSITY_REFERENCE, abi.EPP_VISCOSITY_MONAGHAN])
+@pytest.mark.parametrize("rho,mass", [(1000.0, 0.1), (2e-20, 1e-35), (1e20, 1e28)])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_viscosity_over_the_range_of_densities(dim, rho, mass, viscosity):
+    ps, domain, rng = pairs(dim, 0.01, rng_apart(dim), 3)
+    n = ps["Mass"].size
+    ps["Density"] = (rho * rng.uniform(0.7, 1.3, n)).astype(np.float32)
+    ps["Mass"] = np.full(n, mass, np.float32)
+    v, x = ps["VelocityVec"], ps["PositionVec"]
+    v[0::2], v[1::2] = x[1::2] - x[0::2], 0.0   # head on: v . dx does not cancel
+    ps["VelocityVec"] = v * np.float32(100.0)
+    d = device(ps, domain)
+    phys = physics(dim, viscosity=viscosity)
+    d.ctx.search(SYM, abi.EPP_ACTION_NONE, phys, 0)
+    d.ctx.interaction(MOMENTUM, phys)
+    d.ctx.synchronize()
+    d.asyncto()
+    dx, r, dv, dwr, h = geometry(ps, dim)
+    den, m = ps["Density"].astype(np.float64), ps["Mass"].astype(np.float64)[1::2]
+    phi = (dx * dv).sum(1) * h / (r * r + 0.01 * h * h)
+    al, be, c0 = (float(np.float32(a)) for a in (phys.alpha, phys.beta, phys.c0))
+    f = (-al * c0 + be * phi) * phi / (0.5 * (den[0::2] + den[1::2])) * -m * dwr
+    if viscosity == abi.EPP_VISCOSITY_REFERENCE:
+        f /= den[0::2] * den[1::2]
+    want = f[:, None] * dx
+    got = d.host["dVelocityVec"][0::2].astype(np.float64)
+    err = np.abs(got - want).max(1) / np.abs(want).max(1)
+    assert np.all(np.isfinite(got)) and err.max() <= 2e-6, err.max()
+    d.close()
+
+
+def rng_apart(dim):
+    return np.random.default_rng(dim).uniform(0.1, 1.2, 200)
