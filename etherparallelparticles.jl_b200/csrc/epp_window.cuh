@@ -13,7 +13,9 @@
 // -- position and h, the list entry (index and tag) in the unused z lane, and the search action's
 // neighbour record -- and every lane reads its own windows from there.  The staging area holds both
 // parts of a warp that crosses a cell-row end; what does not fit (a free surface, whose warps span
-// many cells over a dense row; dense neighbourhoods) is split into passes over fewer lanes.  The lane
+// many cells over a dense row) is split into passes over fewer lanes, and lanes whose own windows do
+// not fit (dense neighbourhoods, h of 2.5 dx and more) all read theirs from global memory at once: 2D
+// search at h = 3 dx, 132,518 particles, 195 us, where a pass for each such lane took 2990.  The lane
 // builds one acceptance word per stencil row with the reference's IEEE criterion and the active-pair
 // matrix, then walks the set bits of the three words in list order, in one loop: it appends the
 // neighbour to its list (the lists the momentum, filter and extrapolation passes read; same layout
@@ -122,42 +124,73 @@ struct WinOut {
     float sx, sy;
 };
 
-// The per-lane search in its general form, candidate by candidate from global memory: dense
-// neighbourhoods only (a window beyond 32 candidates, or windows beyond the staging area).  Inlined:
-// as an out-of-line call it cost the kernel registers (the values live across the call) and 13% of
-// its time.
+// The bound that window_from_memory keeps from one candidate to the next: that of the last h_j met
+// that is not the lane's own.
+struct OtherBound {
+    float h, r2;
+};
+
+// Candidates [lo, hi) of one window straight from global memory, 32 at a time: the acceptance bits of
+// a word first, its loads in flight together, then one walk over the set bits.  (Candidate by candidate,
+// each accepted one evaluated where it was met, a warp ran the term once for nearly every candidate.)
+// own: the bound against candidates of the lane's h, or of the default criterion.
+template <int D, class Act>
+__device__ __forceinline__ void window_from_memory(const PairArgs& A, const Act& act, const typename Act::Self& me,
+                                                   const TargetConst& tc, ListWriter<D>& L, int lo, int hi, int i, int ti,
+                                                   float4 xi, unsigned amask, float own, OtherBound& other, WinOut& o) {
+    const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
+#pragma unroll 1
+    for (int k0 = lo; k0 < hi; k0 += 32) {
+        const int len = min(hi - k0, 32);
+        unsigned word = 0u;
+#pragma unroll 4
+        for (int k = len - 1; k >= 0; --k) {
+            const float4 xj = A.s.xh[k0 + k];
+            const float dr2 = geometry<D>(xi, xj).dr2;
+            float bound = own;
+            if (xj.w != xi.w && !dflt) {
+                if (xj.w != other.h) other = OtherBound{xj.w, pair_r2(xi.w, xj.w)};
+                bound = other.r2;
+            }
+            word = (word << 1) | (dr2 <= bound ? 1u : 0u);
+        }
+        const int self = i - k0;   // not its own neighbour
+        if (self >= 0 && self < 32) word &= ~(1u << self);
+        while (word) {
+            const int j = k0 + __ffs(word) - 1;
+            word &= word - 1u;
+            const int tj = tag_of(A.s.tagm[j]);
+            if (!(__funnelshift_rc(amask, 0u, (unsigned)(tj - 1)) & 1u)) continue;   // the active-pair matrix
+            L.put(o.cnt++, list_entry(j, tj));
+            if (Act::NC != 0) {
+                const float4 xj = A.s.xh[j];
+                const float4 t = act.term(me, act.fetch(j, ti, tj), ti, tj, xj, geometry<D>(xi, xj), tc);
+                o.sx = __fadd_rn(o.sx, t.x);
+                o.sy = __fadd_rn(o.sy, t.y);
+            }
+        }
+    }
+}
+
+// The per-lane search in its general form, from global memory: dense neighbourhoods only (a window
+// beyond 64 candidates, or windows beyond the staging area).  Inlined: as an out-of-line call it cost
+// the kernel registers (the values live across the call) and 13% of its time.
 template <int D, class Act>
 __device__ __forceinline__ WinOut win_lane_general(const PairArgs& A, const TileMask& M, const Act& act,
                                                 const RowWin (&win)[D == 3 ? 9 : 3], int i, int ti, float4 xi, unsigned amask) {
     const TargetConst tc = target_const<D>(xi.w);
-    const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
-    typename Act::Self me = act.self(i);
+    const typename Act::Self me = act.self(i);
     ListWriter<D> L = list_writer<D>(M, i);
     WinOut o{0, 0.0f, 0.0f};
-    float ho = xi.w, ro = dflt ? A.dom.gap_square : tc.h2sq;
+    OtherBound other{xi.w, 0.0f};
 #pragma unroll 1
     for (int r = 0; r < (D == 3 ? 9 : 3); ++r) {
         int lo = 0, hi = 0;
 #pragma unroll
         for (int q = 0; q < (D == 3 ? 9 : 3); ++q)
             if (q == r) lo = win[q].lo, hi = win[q].hi;
-#pragma unroll 1
-        for (int j = lo; j < hi; ++j) {
-            const float4 xj = A.s.xh[j];
-            const int tj = tag_of(A.s.tagm[j]);
-            const PairGeo g = geometry<D>(xi, xj);
-            if (xj.w != ho) {
-                ho = xj.w;
-                ro = dflt ? A.dom.gap_square : ho == xi.w ? tc.h2sq : pair_r2(xi.w, ho);
-            }
-            if (!(g.dr2 <= ro) || j == i || !(__funnelshift_rc(amask, 0u, (unsigned)(tj - 1)) & 1u)) continue;
-            L.put(o.cnt++, list_entry(j, tj));
-            if (Act::NC != 0) {
-                const float4 t = act.term(me, act.fetch(j, ti, tj), ti, tj, xj, g, tc);
-                o.sx = __fadd_rn(o.sx, t.x);
-                o.sy = __fadd_rn(o.sy, t.y);
-            }
-        }
+        window_from_memory<D>(A, act, me, tc, L, lo, hi, i, ti, xi, amask, A.crit == EPP_CRITERION_DEFAULT ? A.dom.gap_square : tc.h2sq,
+                              other, o);
     }
     L.flush(o.cnt);
     return o;
@@ -198,12 +231,16 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
         const int rid_p = __shfl_up_sync(FULL, rid, 1), cx_p = __shfl_up_sync(FULL, cx, 1);
         const unsigned starts = __ballot_sync(FULL, lane == 0 || rid != rid_p || cx - cx_p > 3);
         float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        unsigned pending = __ballot_sync(FULL, on);
+        const int l0 = win[0].hi - win[0].lo, l1 = win[1].hi - win[1].lo, l2 = win[2].hi - win[2].lo;
+        const int longest = max(l0, max(l1, l2));
+        // dense neighbourhoods go straight to memory, all of the warp's at once
+        const bool direct = longest > 64 || l0 + l1 + l2 > kStage2;
+        unsigned pending = __ballot_sync(FULL, on && !direct);
         while (pending) {   // warp-uniform: a pass over as many parts as the staging area holds
             const int head = __ffs(pending) - 1;
             const float hw = __shfl_sync(FULL, xi.w, head);   // the pass is plain when every candidate has
             const int tw = __shfl_sync(FULL, ti, head);       // the first lane's h and tag
-            bool same_t = true, staged = false, other = false;
+            bool same_t = true, other = false;
             float hb = hw;   // an h other than hw that this lane staged
             int used = 0, off[3] = {0, 0, 0};
             unsigned taken = 0u;
@@ -224,12 +261,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
                     if (total <= kStage2 - used || used > 0 || last == lead) break;
                     last = lead + (last - lead) / 2;
                 }
-                if (total > kStage2 - used) {
-                    if (used > 0) break;   // next pass
-                    taken = 1u << lead;    // one lane's windows are too long: read from global memory
-                    pending &= ~taken;
-                    break;
-                }
+                if (total > kStage2 - used) break;   // next pass (the first part of a pass fits)
                 for (int k = lane; k < total; k += 32) {
                     const int j = k < len[0] ? lo[0] + k : k < len[0] + len[1] ? lo[1] + (k - len[0]) : lo[2] + (k - len[0] - len[1]);
                     const float4 xj = A.s.xh[j];
@@ -241,9 +273,8 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
                     if (xj.w != hw) other = true, hb = xj.w;
                     same_t = same_t && tj == tw;
                 }
-                const unsigned part = ((2u << last) - 1u) & ~((1u << lead) - 1u);
+                const unsigned part = ((2u << last) - 1u) & ~((1u << lead) - 1u) & pending;
                 if ((part >> lane) & 1u) {
-                    staged = true;
                     off[0] = used + win[0].lo - lo[0];
                     off[1] = used + len[0] + win[1].lo - lo[1];
                     off[2] = used + len[0] + len[1] + win[2].lo - lo[2];
@@ -257,18 +288,9 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
             same_t = __all_sync(FULL, same_t);
             __syncwarp();
             if (!(((taken >> lane) & 1u) && valid)) continue;
-            const int l0 = win[0].hi - win[0].lo, l1 = win[1].hi - win[1].lo, l2 = win[2].hi - win[2].lo;
-            const int longest = max(l0, max(l1, l2));
             // cells of four particle rows or columns (where the lattice and the cells drift apart) make
             // windows of up to 40: the lanes of the pass then take each row in two words, one after the other
-            const bool two = __any_sync(__activemask(), staged && longest > 32);
-            if (!staged || longest > 64) {
-                const WinOut o = win_lane_general<2, Act>(A, M, act, win, i, ti, xi, amask);
-                cnt = o.cnt;
-                sum.x = o.sx;
-                sum.y = o.sy;
-                continue;
-            }
+            const bool two = __any_sync(__activemask(), longest > 32);
             const TargetConst tc = target_const<2>(xi.w);
             if (same_t && !((amask >> (tw - 1)) & 1u)) continue;   // nothing the lane may see: walls among walls
             const bool one = dflt || !others;
@@ -343,6 +365,12 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
                 }
             }
             L.flush(cnt);
+        }
+        if (direct && valid) {
+            const WinOut o = win_lane_general<2, Act>(A, M, act, win, i, ti, xi, amask);
+            cnt = o.cnt;
+            sum.x = o.sx;
+            sum.y = o.sy;
         }
         if (on) {
             if (!valid) {

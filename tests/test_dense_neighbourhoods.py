@@ -1,0 +1,39 @@
+"""More neighbours than a list keeps (h of 2.5 to 4 dx): windows beyond the staging areas, pair passes
+from the stencil.  The same neighbours and sums as the lists give, and no path that leaves most of a
+warp idle: the stages of a step stay within a few times those of another pair-pass family, where the
+faults these tests are for took 5 to 20 times as long."""
+import numpy as np
+import pytest
+
+from epp import abi, casegen
+from epp.algorithm import DeviceParticleSystem
+from epp.classes import NeighbourSystem
+
+pytestmark = pytest.mark.gpu
+
+SYM, CONT = abi.EPP_CRITERION_SYMMETRY, abi.EPP_ACTION_DAMBREAK_CONTINUITY
+MOMENTUM, SEARCH, CONTINUITY = 0, 4, 5   # stages of a step
+
+
+def device(case, family=0):
+    d = DeviceParticleSystem(case.ps, NeighbourSystem(case.domain, casegen.DAM_BREAK_ACTIVE_PAIRS, max_neighbour_number=1))
+    d.ctx.set_tuning(family)
+    d.syncto()
+    d.ctx.search(SYM, CONT, case.physics, 0)
+    return d
+
+
+def stages(case, family):
+    """Least time of each stage over some steps, ms."""
+    d = device(case, family)
+    times = [list(t.values()) if isinstance(t, dict) else list(t) for t in (d.ctx.profile_step(case.physics) for _ in range(6))]
+    d.close()
+    return np.min(np.array(times), axis=0)
+
+
+# the staged 2D search (above 20,000 particles) against the lockstep one
+@pytest.mark.parametrize("h_factor", [2.5, 3.0, 4.0])
+def test_dense_2d_search_time(h_factor):
+    case = casegen.dam_break_2d(dx=0.01, h_factor=h_factor, max_neighbour_number=1)
+    lists = stages(case, abi.EPP_TUNING_LISTS)
+    assert stages(case, 0)[SEARCH] <= 2.0 * (lists[SEARCH] + lists[CONTINUITY])
