@@ -391,8 +391,10 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
 // particles, 182 -> 84 at 165,888.  Issue-bound (79% of the slots): about half on the tests, 40% on the
 // walk over their bits, which is why a word whose candidates have one tag computes its entries and
 // checks the list's capacity once.  Warps near walls stage two h's and take the two bounds by a select.
-// When one particle's plane is longer than the staging area (dense neighbourhoods) the rows go one by
-// one, and a row beyond it is read from global memory.  One warp per cell, its lanes on the candidates
+// When one particle's plane is longer than the staging area (dense neighbourhoods) the stencil goes by
+// rows, or by cells, and a cell beyond it is read from global memory by all its lanes at once: 926 us
+// at h = 2.5 dx and 165,888 particles, where a pass for each lane with a long row took 12800.
+// One warp per cell, its lanes on the candidates
 // and ballots in place of the walk, measured 528 us: two POPC per target and chunk, no fewer
 // instructions.
 // Staged candidates per warp: both parts of a warp that crosses a cell-row end (about 360; with room for
@@ -464,25 +466,41 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
         const int rid_p = __shfl_up_sync(FULL, rid, 1), cx_p = __shfl_up_sync(FULL, cx, 1);
         const unsigned starts = __ballot_sync(FULL, lane == 0 || rid != rid_p || cx - cx_p > 3);
         const unsigned alive = __ballot_sync(FULL, on);
-        int rows = 3;
-        for (int r0 = 0; r0 < 9; r0 += rows) {   // warp-uniform
+        // u counts cells of the stencil; a step takes a plane of them, a row or, in dense neighbourhoods, one
+        int step = 9;
+        for (int u = 0; u < 27; u += step) {   // warp-uniform
             RowWin win[3];
             int mine = 0;
 #pragma unroll
             for (int q = 0; q < 3; ++q) {
-                win[q] = q < rows ? row_range(A, stencil_row<3>(A, rid, y, z, r0 + q), cx - 1, cx + 1) : RowWin{0, 0};
+                const int x = step == 1 ? cx - 1 + u % 3 : cx - 1;
+                win[q] = q == 0 || step == 9 ? row_range(A, stencil_row<3>(A, rid, y, z, u / 3 + q), x, step == 1 ? x : cx + 1) : RowWin{0, 0};
                 mine += win[q].hi - win[q].lo;
             }
-            if (rows == 3 && __any_sync(FULL, mine > kStage3)) {   // from here on one row at a time
-                rows = 1;
+            if (step == 9 && __any_sync(FULL, mine > kStage3)) {   // from here on one row at a time
+                step = 3;
                 win[1] = win[2] = RowWin{0, 0};
+                mine = win[0].hi - win[0].lo;
             }
-            unsigned pending = alive;
+            if (step == 3 && __any_sync(FULL, mine > kStage3)) {   // or one cell
+                step = 1;
+                win[0] = row_range(A, stencil_row<3>(A, rid, y, z, u / 3), cx - 1, cx - 1);
+                mine = win[0].hi - win[0].lo;
+            }
+            const bool direct = mine > kStage3;   // a cell beyond it: from memory, all such lanes at once
+            if (direct && valid) {
+                OtherBound other{xi.w, 0.0f};
+                WinOut o{cnt, 0.0f, 0.0f};
+                window_from_memory<3>(A, CPCount<3>{ncount}, CPCount<3>::Self{}, TargetConst{}, L, win[0].lo, win[0].hi, i, ti, xi,
+                                      amask, own, other, o);
+                cnt = o.cnt;
+            }
+            unsigned pending = alive & ~__ballot_sync(FULL, direct);
             while (pending) {   // warp-uniform: a pass over as many parts as the staging area holds
                 const int head = __ffs(pending) - 1;
                 const float hw = __shfl_sync(FULL, xi.w, head);
                 const int tw = __shfl_sync(FULL, ti, head);
-                bool same_t = true, staged = false;
+                bool same_t = true;
                 bool other = false, two_h = true;   // an h other than hw was staged by this lane; one such h only
                 float hb = hw;
                 int used = 0, off[3] = {0, 0, 0};
@@ -504,12 +522,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
                         if (total <= kStage3 - used || used > 0 || last == lead) break;
                         last = lead + (last - lead) / 2;
                     }
-                    if (total > kStage3 - used) {
-                        if (used > 0) break;   // next pass
-                        taken = 1u << lead;    // one lane's row is too long: read from global memory
-                        pending &= ~taken;
-                        break;
-                    }
+                    if (total > kStage3 - used) break;   // next pass (the first part of a pass fits)
 #pragma unroll 4   // their loads in flight together (2% at 955,668 particles, 4% at 165,888; the 2D pass lost 3%)
                     for (int k = lane; k < total; k += 32) {
                         const int j = k < len[0] ? lo[0] + k
@@ -527,9 +540,8 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
                         }
                         same_t = same_t && tj == tw;
                     }
-                    const unsigned part = ((2u << last) - 1u) & ~((1u << lead) - 1u);
+                    const unsigned part = ((2u << last) - 1u) & ~((1u << lead) - 1u) & pending;
                     if ((part >> lane) & 1u) {
-                        staged = true;
                         off[0] = used + win[0].lo - lo[0];
                         off[1] = used + len[0] + win[1].lo - lo[1];
                         off[2] = used + len[0] + len[1] + win[2].lo - lo[2];
@@ -544,7 +556,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
                 same_t = __all_sync(FULL, same_t);
                 __syncwarp();
                 if (!(((taken >> lane) & 1u) && valid)) continue;
-                if (same_t && staged && !((amask >> (tw - 1)) & 1u)) continue;   // walls among walls
+                if (same_t && !((amask >> (tw - 1)) & 1u)) continue;   // walls among walls
                 // exact bounds of this lane against hw and the other h, as window_bits3 takes them
                 const int hs = dflt || !others ? 1 : two_h ? 2 : 3;   // warp-uniform
                 const int nO = accept_bias(own);
@@ -553,25 +565,21 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
                 float ho = xi.w;
                 int no = nO;
 #pragma unroll 1
-                for (int q = 0; q < rows; ++q) {
+                for (int q = 0; q < (step == 9 ? 3 : 1); ++q) {
                     const int lo = q == 0 ? win[0].lo : q == 1 ? win[1].lo : win[2].lo;
                     const int n = (q == 0 ? win[0].hi : q == 1 ? win[1].hi : win[2].hi) - lo;
                     const int o = q == 0 ? off[0] : q == 1 ? off[1] : off[2];
-                    const int self = r0 + q == 4 ? i - lo : -1;   // not its own neighbour
-                    if (!staged) {
-                        for (int k = 0; k < n; ++k) {
-                            const int j = lo + k;
-                            unsigned st = 0u;
-                            if (accept<3>(A, i, xi, amask, own, j, A.s.xh[j], st)) L.put(cnt++, list_entry(j, tag_of(A.s.tagm[j])));
-                        }
-                        continue;
-                    }
+                    const int self = u / 3 + q == 4 ? i - lo : -1;   // not its own neighbour
                     for (int k0 = 0; k0 < n; k0 += 32) {
                         const int len = min(n - k0, 32);
                         unsigned word = hs == 1   ? window_bits3<1>(S.x, o + k0, len, xi, nA, hw, nB, nO, ho, no)
                                         : hs == 2 ? window_bits3<2>(S.x, o + k0, len, xi, nA, hw, nB, nO, ho, no)
                                                   : window_bits3<3>(S.x, o + k0, len, xi, nA, hw, nB, nO, ho, no);
                         if ((self >> 5) == (k0 >> 5)) word &= ~(0x80000000u >> (self & 31));
+                        if (same_t && cnt >= ListConf<3>::LCAP) {   // no list to keep
+                            cnt += __popc(word);
+                            continue;
+                        }
                         if (same_t && cnt + 32 <= ListConf<3>::LCAP) {   // entries from their index, room for all
                             const int e0 = list_entry(lo + k0, tw);
                             while (word) {

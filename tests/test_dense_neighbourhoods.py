@@ -37,3 +37,11 @@ def test_dense_2d_search_time(h_factor):
     case = casegen.dam_break_2d(dx=0.01, h_factor=h_factor, max_neighbour_number=1)
     lists = stages(case, abi.EPP_TUNING_LISTS)
     assert stages(case, 0)[SEARCH] <= 2.0 * (lists[SEARCH] + lists[CONTINUITY])
+
+
+# the staged 3D search (above 50,000 particles) against eight lanes per particle
+@pytest.mark.parametrize("h_factor", [2.0, 2.5])
+def test_dense_3d_search_time(h_factor):
+    case = casegen.dam_break_3d(dx=0.025, h_factor=h_factor, max_neighbour_number=1)
+    assert case.n > 50000
+    assert stages(case, 0)[SEARCH] <= 3.0 * stages(case, 8)[SEARCH]
