@@ -610,10 +610,12 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
 // particle's walk is L times shorter.  Lane g tests candidates g, g + L, ... of each window (four loads
 // in flight); a ballot of the group gives each accepted one its place in the list, kept in shared
 // memory; then lane g writes entries g, g + L, ... out and evaluates the action's terms for them, and
-// the first lane adds the terms in list order: lists, counts and sums have the bits of k_win_build.  A
-// particle with more neighbours than a list keeps goes through the general per-lane search.  It issues
-// four times k_win_build's instructions per particle (383 against 93) but a fifth of them one after
-// the other: 12 us against 25 at 1,418 particles, 22 each at 22,279; 3D 52 against 88 at 33,123.
+// the first lane adds the terms in list order: lists, counts and sums have the bits of k_win_build.  With
+// more neighbours than a list keeps, a search without terms is done (the first ones are stored: 3D, h =
+// 2.5 dx, 20,340 particles, 157 us against 588 with a second search), one with terms goes through the
+// general per-lane search.  It issues four times k_win_build's instructions per particle (383 against
+// 93) but a fifth of them one after the other: 12 us against 25 at 1,418 particles, 22 each at 22,279;
+// 3D 52 against 88 at 33,123.
 template <int D, class Act, int L>
 __global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M,
                                                    const __grid_constant__ Act act, unsigned long long* pairs) {
@@ -687,7 +689,7 @@ __global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairA
                 }
             }
             float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (cnt > CAP) {
+            if (Act::NC != 0 && cnt > CAP) {
                 if (g == 0) {
                     const WinOut o = win_lane_general<D, Act>(A, M, act, win, i, ti, xi, amask);
                     sum.x = o.sx;
@@ -697,7 +699,7 @@ __global__ void __launch_bounds__(128) k_win_lanes(const __grid_constant__ PairA
                 __syncwarp(group);
                 const typename Act::Self me = act.self(i);
 #pragma unroll 2
-                for (int k = g; k < cnt; k += L) {
+                for (int k = g; k < min(cnt, CAP); k += L) {
                     const int e = s_e[p][k], j = entry_index(e), tj = entry_tag(e);
                     if (D == 3) M.list[(size_t)i * CAP + k] = e;
                     else M.list[(size_t)k * M.cap + i] = e;

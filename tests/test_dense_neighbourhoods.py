@@ -45,3 +45,9 @@ def test_dense_3d_search_time(h_factor):
     case = casegen.dam_break_3d(dx=0.025, h_factor=h_factor, max_neighbour_number=1)
     assert case.n > 50000
     assert stages(case, 0)[SEARCH] <= 3.0 * stages(case, 8)[SEARCH]
+
+
+# eight lanes per particle (up to 50,000 particles), whose first pass has the list's entries already
+def test_dense_3d_search_time_of_small_systems():
+    few, many = (stages(casegen.dam_break_3d(dx=0.05, h_factor=h, max_neighbour_number=1), 0)[SEARCH] for h in (1.6, 2.5))
+    assert many <= 8.0 * few   # 3.8 times the candidates
