@@ -27,6 +27,21 @@ __device__ __noinline__ float pair_r2(float hi, float hj) {
     return __fmul_rn(h2, h2);
 }
 
+// The bound on dr2 against candidates of another h than the particle's own, kept from one candidate to
+// the next: along a row h alternates between the particle's own and one other (fluid and walls).
+struct OtherBound {
+    float h, r2;
+    // the bound for a candidate of h_j; own: against the particle's h, or of the default criterion
+    __device__ __forceinline__ float of(float hi, float hj, float own, bool dflt) {
+        if (hj == hi || dflt) return own;
+        if (hj != h) {
+            h = hj;
+            r2 = pair_r2(hi, hj);
+        }
+        return r2;
+    }
+};
+
 // Candidate filter: the reference's criterion (IEEE, exact) and the active-pair matrix.
 template <int D>
 __device__ __forceinline__ bool accept(const PairArgs& A, int i, float4 xi, unsigned amask, float h2sq,
@@ -525,6 +540,103 @@ struct ListTerm<D, CPMom<D, FUSED, false>> {
 template <int D, class Act>
 constexpr bool kListInter = D == 3 && Act::NC == 3;
 
+// neighbours_by_stencil by a group of four lanes, lanes first .. first + 3 of the warp, for the 3D list
+// passes: a word of acceptance bits of every fourth candidate a lane, then a walk over the set ones.
+// Where the sum is four partials each lane adds its own; an ordered one has the lanes' words
+// interleaved and takes the accepted candidates four at a time, as k_list takes a list.  One lane at
+// work while the others of its group waited made those passes twice as long as one thread per particle
+// where lists overflow (h = 2 dx, 165,888 particles: momentum 891 us with one thread, 1687 with one lane
+// of four, 444 with all four; continuity 849, 1560, 561).
+template <int D, class Act>
+__device__ __noinline__ float4 neighbours_by_group(const PairArgs& A, int i, float4 xi, int ti, float h2sq, const Act& act,
+                                                   int g, int first) {
+    using T = ListTerm<D, Act>;
+    constexpr bool INTER = kListInter<D, Act>;
+    constexpr int N = INTER ? 32 : 8;   // candidates of a lane's word
+    const unsigned group = 15u << first;
+    const int c = A.s.cell[i];
+    const int n0 = A.dom.n[0];
+    TileRanges<D> R;
+    R.n = 0;
+    R.total = 0;
+    R.stencil(A, (c / n0) % A.dom.n[1], (c / n0) / A.dom.n[1], c % n0, c % n0);
+    const unsigned amask = A.adj[ti - 1];
+    const bool dflt = A.crit == EPP_CRITERION_DEFAULT;
+    const float own = dflt ? A.dom.gap_square : h2sq;
+    OtherBound other{xi.w, own};
+    const typename T::Me me = T::me(act, i, xi, ti);
+    typename T::Acc acc{};
+    int cnt = 0;
+#pragma unroll 1
+    for (int r = 0; r < R.n; ++r) {
+        const int end = R.lo[r] + R.len[r];
+#pragma unroll 1
+        for (int j0 = R.lo[r]; j0 < end; j0 += 4 * N) {   // uniform in the group
+            unsigned word = 0u;   // bit k: candidate j0 + g + 4 k
+#pragma unroll 4
+            for (int k = min((end - j0 - g + 3) >> 2, N) - 1; k >= 0; --k) {
+                const float4 xj = A.s.xh[j0 + g + 4 * k];
+                word = (word << 1) | (geometry<D>(xi, xj).dr2 <= other.of(xi.w, xj.w, own, dflt) ? 1u : 0u);
+            }
+            if constexpr (INTER) {
+                while (word) {
+                    const int j = j0 + g + 4 * (__ffs(word) - 1), tj = tag_of(A.s.tagm[j]);
+                    word &= word - 1u;
+                    if (j == i || !(__funnelshift_rc(amask, 0u, (unsigned)(tj - 1)) & 1u)) continue;
+                    T::add(acc, T::term(act, me, T::load(A, act, me, j, tj), tj));
+                    ++cnt;
+                }
+            } else {
+                word = (word | word << 12) & 0x000f000fu;   // bit k to bit 4 k
+                word = (word | word << 6) & 0x03030303u;
+                word = (word | word << 3) & 0x11111111u;
+                unsigned mask = __reduce_or_sync(group, word << g);   // bit k: candidate j0 + k
+                if (i >= j0 && i < j0 + 32) mask &= ~(1u << (i - j0));
+                while (mask) {   // uniform in the group
+                    unsigned m = mask;   // lane g takes the g-th accepted one
+                    if (g > 0) m &= m - 1u;
+                    if (g > 1) m &= m - 1u;
+                    if (g > 2) m &= m - 1u;
+                    typename T::Term t{};
+                    bool ok = false;
+                    if (m) {
+                        const int j = j0 + __ffs(m) - 1, tj = tag_of(A.s.tagm[j]);
+                        ok = __funnelshift_rc(amask, 0u, (unsigned)(tj - 1)) & 1u;
+                        if (ok) t = T::term(act, me, T::load(A, act, me, j, tj), tj);
+                    }
+                    const unsigned hits = __ballot_sync(group, ok) >> first;
+                    cnt += __popc(hits & 15u);
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const typename T::Term tu = T::from(group, t, first + u);
+                        if ((hits >> u) & 1u) T::add(acc, tu);
+                        mask &= mask - 1u;
+                    }
+                }
+            }
+        }
+    }
+    if constexpr (INTER) {
+        cnt = __reduce_add_sync(group, cnt);
+#pragma unroll
+        for (int o = 1; o < 4; o <<= 1) {
+            acc.x = __fadd_rn(acc.x, __shfl_xor_sync(group, acc.x, o));
+            acc.y = __fadd_rn(acc.y, __shfl_xor_sync(group, acc.y, o));
+            acc.z = __fadd_rn(acc.z, __shfl_xor_sync(group, acc.z, o));
+        }
+    }
+    return make_float4(acc.x, acc.y, acc.z, (float)cnt);
+}
+
+// Blocks an SM of a list pass: 2D with one thread per particle 9 (56 registers; they beat 7, 8 and 10); in
+// 3D with four lanes what the loop over a list takes, the overflow path being longer (momentum of the
+// benchmark physics 64 registers, 1915 us at 6,207,228 particles, 2101 with 7 blocks; continuity 56, 41 us
+// at 165,888, 46 with 7).
+template <int D, class Act, int L>
+constexpr int kListBlocks = L == 1 ? (D == 2 ? 9 : 4) : D == 2 ? 6 : kListInter<D, Act> ? 7 : 9;
+template <bool FUSED>
+constexpr int kListBlocks<3, CPMom<3, FUSED, false>, 4> = 8;
+
 // A pair action over the neighbour lists written by the last search pass (same positions, cells and
 // criterion).  L lanes share a particle, lane g takes entries k = g mod L.
 //   L = 1        one thread per particle, terms added in list order
@@ -541,7 +653,7 @@ constexpr bool kListInter = D == 3 && Act::NC == 3;
 // at 515,018 particles.
 // EPI: fused momentum step (integrate + bin for every particle, dead bin included).
 template <int D, class Act, bool EPI, int L>
-__global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 blocks (56 registers) beat 7, 8 and 10
+__global__ void __launch_bounds__(128, kListBlocks<D, Act, L>)
     k_list(const __grid_constant__ PairArgs A, const __grid_constant__ TileMask M, const int* ncount,
            const __grid_constant__ Act act) {
     using T = ListTerm<D, Act>;
@@ -565,12 +677,17 @@ __global__ void __launch_bounds__(128, L > 1 ? 6 : D == 2 ? 9 : 4)   // 2D: 9 bl
             return;
         }
         if (cnt > ListConf<D>::LCAP) {   // more neighbours than the list keeps
-            if (g == 0) {
+            // (2D: one lane, the bits of one thread per particle whatever the physics; no slower there)
+            if (D == 3 || g == 0) {
                 const TargetConst tc = target_const<D>(xi.w);
-                float4 sum = neighbours_by_stencil<D>(A, i, xi, ti, tc, act);
+                float4 sum;
+                if constexpr (D == 3 && L > 1)
+                    sum = neighbours_by_group<D, Act>(A, i, xi, ti, tc.h2sq, act, g, (int)(threadIdx.x & 31u & ~(unsigned)(L - 1)));
+                else
+                    sum = neighbours_by_stencil<D>(A, i, xi, ti, tc, act);
                 const int got = (int)sum.w;
                 sum.w = 0.0f;
-                act.end(i, ti, sum, got);
+                if (g == 0) act.end(i, ti, sum, got);
             }
             return;
         }

@@ -124,12 +124,6 @@ struct WinOut {
     float sx, sy;
 };
 
-// The bound that window_from_memory keeps from one candidate to the next: that of the last h_j met
-// that is not the lane's own.
-struct OtherBound {
-    float h, r2;
-};
-
 // Candidates [lo, hi) of one window straight from global memory, 32 at a time: the acceptance bits of
 // a word first, its loads in flight together, then one walk over the set bits.  (Candidate by candidate,
 // each accepted one evaluated where it was met, a warp ran the term once for nearly every candidate.)
@@ -146,13 +140,7 @@ __device__ __forceinline__ void window_from_memory(const PairArgs& A, const Act&
 #pragma unroll 4
         for (int k = len - 1; k >= 0; --k) {
             const float4 xj = A.s.xh[k0 + k];
-            const float dr2 = geometry<D>(xi, xj).dr2;
-            float bound = own;
-            if (xj.w != xi.w && !dflt) {
-                if (xj.w != other.h) other = OtherBound{xj.w, pair_r2(xi.w, xj.w)};
-                bound = other.r2;
-            }
-            word = (word << 1) | (dr2 <= bound ? 1u : 0u);
+            word = (word << 1) | (geometry<D>(xi, xj).dr2 <= other.of(xi.w, xj.w, own, dflt) ? 1u : 0u);
         }
         const int self = i - k0;   // not its own neighbour
         if (self >= 0 && self < 32) word &= ~(1u << self);

@@ -51,3 +51,36 @@ def test_dense_3d_search_time(h_factor):
 def test_dense_3d_search_time_of_small_systems():
     few, many = (stages(casegen.dam_break_3d(dx=0.05, h_factor=h, max_neighbour_number=1), 0)[SEARCH] for h in (1.6, 2.5))
     assert many <= 8.0 * few   # 3.8 times the candidates
+
+
+# 3D list passes of four lanes per particle whose lists overflow, against eight lanes without lists
+@pytest.mark.parametrize("h_factor", [2.0, 2.5])
+def test_dense_3d_list_pass_time(h_factor):
+    case = casegen.dam_break_3d(dx=0.025, h_factor=h_factor, max_neighbour_number=1)
+    lists, lanes = stages(case, 0), stages(case, 8)   # lanes: search and continuity are one kernel
+    assert lists[MOMENTUM] <= 2.5 * lanes[MOMENTUM]
+    assert lists[CONTINUITY] <= 2.5 * lanes[SEARCH]
+
+
+# Overflowing 3D lists: the sums of a family that keeps no lists, to FP32 rounding of a few hundred terms
+# (400 * 2^-24 of the terms' magnitudes, which the column's own pressure bounds)
+@pytest.mark.parametrize("h_factor", [1.8, 2.5])
+def test_dense_3d_sums(h_factor):
+    got = []
+    for family in (0, 8):
+        case = casegen.dam_break_3d(dx=0.05, column=(0.6, 1.0, 0.5), h_factor=h_factor, max_neighbour_number=1)
+        rng = np.random.default_rng(6)
+        fl = case.ps["Tag"] == casegen.FLUID_TAG
+        v = case.ps["VelocityVec"]
+        v[fl] = rng.standard_normal(v[fl].shape)
+        case.ps["VelocityVec"] = v
+        d = device(case, family)
+        d.ctx.interaction(abi.EPP_ACTION_DAMBREAK_MOMENTUM, case.physics)
+        d.ctx.synchronize()
+        d.asyncto()
+        got.append({k: d.host[k].astype(np.float64) for k in ("nCount", "dDensity", "dVelocityVec")})
+        d.close()
+    assert np.array_equal(got[0]["nCount"], got[1]["nCount"]) and got[0]["nCount"].max() > 160
+    for k in ("dDensity", "dVelocityVec"):
+        scale = np.abs(got[1][k]).max()
+        assert np.abs(got[0][k] - got[1][k]).max() <= 400 * 2.0 ** -24 * scale, k
