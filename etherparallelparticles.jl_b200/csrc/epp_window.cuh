@@ -74,6 +74,13 @@ __device__ __forceinline__ WinSelf win_self(const PairArgs& A, int i) {
     return WinSelf{A.s.xh[k], min(A.start[A.dom.n_cells], A.n_max), tag_of(A.s.tagm[k]), A.s.cell[k]};
 }
 
+// A warp of more parts than this (spray: few particles to a cell) reads its windows from memory, all lanes
+// at once, in place of staging part after part.  Search, us, of particles at random places with the
+// rule at 5, 7, 10 and without it: 3D, 0.3 to a cell, 1,505,378 particles 280 / 293 / 364 / 494,
+// 209,361 54 / 57 / 71 / 93; 1 to a cell 70 / 70 / 72 / 74; 2D, 1 to a cell, 106,854 particles 20.5 / 18.5
+// / 18.5 / 18.5.
+constexpr int kPartsMax = 7;
+
 constexpr int kStage2 = 240;   // staged candidates per warp: 7 blocks of 128 threads still fit an SM
 
 template <class Act>
@@ -221,8 +228,8 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
         float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         const int l0 = win[0].hi - win[0].lo, l1 = win[1].hi - win[1].lo, l2 = win[2].hi - win[2].lo;
         const int longest = max(l0, max(l1, l2));
-        // dense neighbourhoods go straight to memory, all of the warp's at once
-        const bool direct = longest > 64 || l0 + l1 + l2 > kStage2;
+        // dense neighbourhoods and spray go straight to memory, all of the warp's at once
+        const bool direct = longest > 64 || l0 + l1 + l2 > kStage2 || __popc(starts) > kPartsMax;
         unsigned pending = __ballot_sync(FULL, on && !direct);
         while (pending) {   // warp-uniform: a pass over as many parts as the staging area holds
             const int head = __ffs(pending) - 1;
@@ -455,8 +462,10 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
         const unsigned starts = __ballot_sync(FULL, lane == 0 || rid != rid_p || cx - cx_p > 3);
         const unsigned alive = __ballot_sync(FULL, on);
         // u counts cells of the stencil; a step takes a plane of them, a row or, in dense neighbourhoods, one
-        int step = 9;
-        for (int u = 0; u < 27; u += step) {   // warp-uniform
+        // (spray: a row, its low bits)
+        constexpr int SPRAY = 16 + 3;
+        int step = __popc(starts) > kPartsMax ? SPRAY : 9;
+        for (int u = 0; u < 27; u += step & 15) {   // warp-uniform
             RowWin win[3];
             int mine = 0;
 #pragma unroll
@@ -475,7 +484,7 @@ __global__ void __launch_bounds__(128, 7) k_win_build3(const __grid_constant__ P
                 win[0] = row_range(A, stencil_row<3>(A, rid, y, z, u / 3), cx - 1, cx - 1);
                 mine = win[0].hi - win[0].lo;
             }
-            const bool direct = mine > kStage3;   // a cell beyond it: from memory, all such lanes at once
+            const bool direct = mine > kStage3 || step == SPRAY;   // from memory, all such lanes at once
             if (direct && valid) {
                 OtherBound other{xi.w, 0.0f};
                 WinOut o{cnt, 0.0f, 0.0f};

@@ -84,3 +84,22 @@ def test_dense_3d_sums(h_factor):
     for k in ("dDensity", "dVelocityVec"):
         scale = np.abs(got[1][k]).max()
         assert np.abs(got[0][k] - got[1][k]).max() <= 400 * 2.0 ** -24 * scale, k
+
+
+# spray: few particles to a cell, warps of many cell rows; the staged search against two lanes a particle
+@pytest.mark.parametrize("dim", [2, 3])
+def test_spray_search_time(dim):
+    from epp.classes import Domain2D, Domain3D
+    times = []
+    for family in (0, 2):
+        case = casegen.dam_break_2d(dx=0.0045, max_neighbour_number=1) if dim == 2 else \
+            casegen.dam_break_3d(dx=0.0185, max_neighbour_number=1)
+        gap = float(case.domain.gap)
+        side = float((case.n / 0.05) ** (1.0 / dim) * gap)
+        case.domain = case.ps.domain = Domain2D(gap, 0, 0, side, side) if dim == 2 else Domain3D(gap, 0, 0, 0, side, side, side)
+        rng = np.random.default_rng(3)
+        case.ps["PositionVec"] = rng.uniform(0.01 * side, 0.99 * side, (case.n, dim)).astype(np.float32)
+        case.physics.dt = 1e-9
+        times.append(stages(case, family)[SEARCH])
+    print(times)
+    assert times[0] <= 1.5 * times[1]
