@@ -298,6 +298,24 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int m, int* count,
     }
 }
 
+// Scatter in arrival order, for cells in no list: perm[start[c] + slot] = (id, source index).  A destination
+// outside [0, n) can only come from a failed scan; it is reported, never written.
+__device__ __forceinline__ void scatter_particle(int i, int n, int2 c, const int* start, int id, int2* perm, unsigned* status) {
+    const int dst = start[c.x] + c.y;
+    if (dst < 0 || dst >= n) atomicOr(status, EPP_STATUS_QUEUE);
+    else perm[dst] = make_int2(id, i);
+}
+
+// Sorted position of perm's entry p, a particle of cell c: start + rank by id among its cell's entries,
+// which lie side by side (independent loads, whatever order the particles came in).
+__device__ __forceinline__ int sorted_place_perm(int p, int2 e, int c, int n, int n_cells, const int2* perm, const int* start) {
+    if (c == n_cells) return p;
+    const int s = start[c], en = min(start[c + 1], n);
+    int rank = 0;
+    for (int q = max(s, 0); q < en; ++q) rank += perm[q].x < e.x;
+    return s + rank;
+}
+
 // Rank of each particle within its cell by id, from the cell's linked list, and its move to start +
 // rank by the mover (src, dst, cell).  A thread per particle in the old order: reads of the state are
 // coalesced, writes nearly so (a step moves few particles to another cell), and no scatter pass has to

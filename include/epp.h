@@ -393,7 +393,7 @@ int32_t epp_profile_step(epp_ctx* ctx, const epp_physics* phys, float* stage_ms)
  *   n_alive     host: number of particles inside the domain
  *   stream      cudaStream_t (NULL = default stream); the call waits for it before returning
  * All intermediate arrays live in one static device array of this library (see
- * epp_noalloc_limits: up to 2^20 particles and 2^20 cells, about 29 MB, held by every GPU that
+ * epp_noalloc_limits: up to 2^20 particles and 2^20 cells, about 25 MB, held by every GPU that
  * loads the library until the process exits).  Larger inputs return EPP_ERR_CAPACITY.  Every call
  * shares that array, so calls that overlap on the GPU (other streams, other host threads) race;
  * serialise them.  The first call on a device looks up the array's device address for that
