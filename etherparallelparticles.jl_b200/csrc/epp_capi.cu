@@ -7,7 +7,6 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
-#include <memory>
 #include <mutex>
 #include <new>
 #include <string>
@@ -131,9 +130,9 @@ struct epp_ctx {
     int* count = nullptr;
     int2* cs = nullptr;
     int2* link = nullptr;
-    int* head[2]{};            // linked-list heads of the cells; the bin passes alternate between the two
-    int* head_mem = nullptr;   // their memory under the cell-centric family, which uses occ
-    int* tile[2]{};            // particles per scan tile, alternating with head
+    int2* perm = nullptr;      // a sort by slots' entries, in link's memory
+    int* head = nullptr;       // linked-list heads of the cells (in occ[0], which only family 1 fills, by slots)
+    int* tile[2]{};            // particles per scan tile; the bin passes alternate between the two
     int tile_stride = 1;
     unsigned long long* scan_state = nullptr;
     unsigned* status = nullptr;
@@ -637,21 +636,47 @@ int prepare_kernels(epp_ctx* ctx) {
     return g ? EPP_ERR_CUDA : EPP_OK;
 }
 
-// The bin buffers of step parity / call `b`, and what the scan of that sort resets.
-BinOut bin_out(epp_ctx* ctx, int b) { return BinOut{ctx->cs, ctx->link, ctx->count, ctx->head[b], ctx->tile[b], ctx->tile_stride}; }
+// Whether a sort ranks a cell's particles from their linked list: one launch fewer than by slots and a
+// scatter pass.  Family 1 keeps the occupied cells where the heads would go.
+bool sorts_by_lists(const epp_ctx* ctx) { return ctx->lanes != 1; }
+
+// The bin buffers of step parity / call `b`.
+BinOut bin_out(epp_ctx* ctx, int b) {
+    return BinOut{ctx->cs, ctx->link, ctx->count, sorts_by_lists(ctx) ? ctx->head : nullptr, ctx->tile[b], ctx->tile_stride};
+}
 
 // Words of look-back state a bin pass clears: only the cell-centric family scans with it.
 int scan_words(const epp_ctx* ctx) { return ctx->lanes == 1 ? ctx->n_tiles + 1 : 0; }
 
 // The scan of the bin pass of buffers `b` into set `to`.
 int launch_scan(epp_ctx* ctx, int b, int to, int max_cell) {
-    const ScanReset R{ctx->head[1 - b], ctx->tile[1 - b], ctx->tile_stride, max_cell};
+    const ScanReset R{ctx->tile[1 - b], ctx->tile_stride, max_cell};
     if (ctx->lanes == 1)
         k_scan<<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->start[to], ctx->occ[to],
                                                               ctx->meta[to], ctx->scan_state, R, ctx->status);
     else
         k_scan_tiles<<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->tile[b],
                                                                     ctx->start[to], R, ctx->status);
+    CK_LAUNCH();
+    return EPP_OK;
+}
+
+// The moves of a sort from set `from` (its ids) to the order of set `to`; `scattered` (or null) is recorded
+// after a scatter pass.
+template <class Mover>
+int launch_gather(epp_ctx* ctx, int from, int to, const Mover& mv, cudaEvent_t scattered = nullptr) {
+    const int n = ctx->n;
+    if (!sorts_by_lists(ctx)) {
+        k_scatter<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->cs, ctx->start[to], ctx->S[from].id, ctx->perm, ctx->status);
+        CK_LAUNCH();
+    }
+    if (scattered) CK(cudaEventRecord(scattered, ctx->stream));
+    if (sorts_by_lists(ctx))
+        k_rank_gather<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->n_cells, ctx->link, ctx->cs, ctx->head, ctx->start[to],
+                                                                  mv, ctx->status);
+    else
+        k_rank_gather_perm<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->n_cells, ctx->perm, ctx->cs, ctx->start[to], mv,
+                                                                       ctx->status);
     CK_LAUNCH();
     return EPP_OK;
 }
@@ -667,9 +692,7 @@ int sort_cells(epp_ctx* ctx) {
     if (const int rc = launch_scan(ctx, b, to, ctx->cfg.max_cell_particles)) return rc;
     ctx->nlist_valid = false;
     MoverAll mv{ctx->S[from], ctx->S[to]};
-    k_rank_gather<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->n_cells, ctx->link, ctx->cs, ctx->head[b],
-                                                               ctx->start[to], mv, ctx->status);
-    CK_LAUNCH();
+    if (const int rc = launch_gather(ctx, from, to, mv)) return rc;
     ctx->cur = to;
     return EPP_OK;
 }
@@ -822,11 +845,8 @@ int enqueue_fused_step(epp_ctx* ctx, int c, const epp_physics& phys, cudaEvent_t
     EPP_MARK(1);
     if (const int rc2 = launch_scan(ctx, c, to, 0)) return rc2;
     EPP_MARK(2);
-    EPP_MARK(3);   // (no scatter pass: the gather ranks from the bin's linked lists)
     MoverFused mv{ctx->S[c], ctx->S[to], mom.F, ctx->start[c], ctx->n_cells, phys.fluid_tag, phys.wall_tag};
-    k_rank_gather<<<blocks_for(n), kThreads, 0, ctx->stream>>>(n, ctx->n_cells, ctx->link, ctx->cs, ctx->head[c],
-                                                               ctx->start[to], mv, ctx->status);
-    CK_LAUNCH();
+    if (const int rc3 = launch_gather(ctx, c, to, mv, ev ? ev[3] : nullptr)) return rc3;
     EPP_MARK(4);
     int rc;
     if (ctx->lanes == 0 && uses_windows(ctx)) {   // 2D windows: one search pass with the continuity action
@@ -1212,7 +1232,7 @@ int32_t epp_create(const epp_config* cfg, epp_ctx** out) {
     ctx->tile_stride = tile_stride(ctx->n_tiles);
     ctx->tile[0] = a.take<int>((size_t)ctx->n_tiles * ctx->tile_stride);
     ctx->tile[1] = a.take<int>((size_t)ctx->n_tiles * ctx->tile_stride);
-    for (int k = 0; k < 2; ++k) ctx->head[k] = ctx->occ[k];   // the occupied cells are listed for family 1 only
+    ctx->head = ctx->occ[0];   // the occupied cells are listed for family 1 only
     ctx->status = a.take<unsigned>(1);
     ctx->pairs = a.take<unsigned long long>(1);
     ctx->ncnt[0] = a.take<int>(ctx->cap);
@@ -1223,7 +1243,7 @@ int32_t epp_create(const epp_config* cfg, epp_ctx** out) {
     static_assert(SI_COUNT >= 4, "cs and link take four ints a particle");
     ctx->stage_i = a.take<int>((size_t)ctx->cap * SI_COUNT);
     ctx->cs = reinterpret_cast<int2*>(ctx->stage_i);
-    ctx->link = ctx->cs + ctx->cap;
+    ctx->link = ctx->perm = ctx->cs + ctx->cap;
     ctx->ipartial = a.take<double>(kIntegralBlocks * 8);
     ctx->iresult = a.take<double>(8);
     ctx->iticket = a.take<unsigned>(1);
@@ -1258,8 +1278,6 @@ int32_t epp_create(const epp_config* cfg, epp_ctx** out) {
     if (cudaMemsetAsync(ctx->arena.base, 0, need, ctx->stream) != cudaSuccess ||
         cudaMemsetAsync(ctx->nlist, 0, nlist_bytes(D, ctx->cap), ctx->stream) != cudaSuccess ||
         cudaMemsetAsync(ctx->cfl_ticket, 0, sizeof(unsigned), ctx->stream) != cudaSuccess ||
-        cudaMemsetAsync(ctx->occ[0], 0xff, sizeof(int) * (ctx->n_cells + 1), ctx->stream) != cudaSuccess ||
-        cudaMemsetAsync(ctx->occ[1], 0xff, sizeof(int) * (ctx->n_cells + 1), ctx->stream) != cudaSuccess ||
         cudaMemsetAsync(ctx->sim_time, 0, sizeof(double) * n_inst, ctx->stream) != cudaSuccess ||
         cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
         cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
@@ -1292,7 +1310,6 @@ int32_t epp_destroy(epp_ctx* ctx) {
     dev_free(ctx, ctx->sim_time);
     dev_free(ctx, ctx->list_mem);
     dev_free(ctx, ctx->list_stage);
-    dev_free(ctx, ctx->head_mem);
     dev_free(ctx, ctx->arena.base);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
@@ -1389,7 +1406,6 @@ int32_t epp_upload(epp_ctx* ctx, int32_t n, const int32_t* is_alive, const int32
     }
     if (rc) return rc;
     if (ctx->cur == 1) {   // the last sort left the bin buffers of set 1 ready; the next one is from set 0
-        CK(cudaMemsetAsync(ctx->head[0], 0xff, sizeof(int) * (ctx->n_cells + 1), ctx->stream));
         CK(cudaMemsetAsync(ctx->tile[0], 0, sizeof(int) * (size_t)ctx->n_tiles * ctx->tile_stride, ctx->stream));
     }
     ctx->cur = 0;
@@ -1903,27 +1919,13 @@ int32_t epp_set_tuning(epp_ctx* ctx, int32_t lanes_per_particle) {
     if (g != 0 && ctx->n_inst > 1)
         return fail(ctx, EPP_ERR_INVALID_ARGUMENT, "batches of %d instances use pair-pass family 0", ctx->n_inst);
     if (g != ctx->lanes || store != ctx->store) {
-        if ((g == 1) != (ctx->lanes == 1)) {   // family 1 lists the occupied cells where the others keep list heads
+        if (g == 1 && ctx->lanes != 1 && ctx->sorted_once) {   // family 1 goes by the occupied cells: list those of the current order
             cudaSetDevice(ctx->dev);
-            const size_t cells = (size_t)ctx->n_cells + 1, pitch = (cells + 63) & ~(size_t)63;
-            if (g == 1 && !ctx->head_mem) CK(dev_alloc(ctx, &ctx->head_mem, 2 * pitch * sizeof(int)));
-            for (int k = 0; k < 2; ++k) {
-                ctx->head[k] = g == 1 ? ctx->head_mem + k * pitch : ctx->occ[k];
-                CK(cudaMemsetAsync(ctx->head[k], 0xff, cells * sizeof(int), ctx->stream));
-            }
-            if (g == 1 && ctx->sorted_once) {   // list those of the current order (a tuning switch may wait)
-                std::unique_ptr<int[]> st(new (std::nothrow) int[cells]);   // offsets, then the cells in their place
-                if (!st) return fail(ctx, EPP_ERR_OUT_OF_MEMORY, "host memory for %d cell offsets", ctx->n_cells);
-                CK(cudaMemcpyAsync(st.get(), ctx->start[ctx->cur], sizeof(int) * cells, cudaMemcpyDeviceToHost, ctx->stream));
-                CK(cudaStreamSynchronize(ctx->stream));
-                int n_occ = 0;
-                for (int c = 0; c < ctx->n_cells; ++c)
-                    if (st[c + 1] > st[c]) st[n_occ++] = c;   // n_occ <= c: only offsets already read
-                if (n_occ > 0)
-                    CK(cudaMemcpyAsync(ctx->occ[ctx->cur], st.get(), sizeof(int) * n_occ, cudaMemcpyHostToDevice, ctx->stream));
-                CK(cudaMemcpyAsync(ctx->meta[ctx->cur], &n_occ, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-                CK(cudaStreamSynchronize(ctx->stream));
-            }
+            if (const int rc_ = join_integrals(ctx)) return rc_;
+            CK(cudaMemsetAsync(ctx->meta[ctx->cur], 0, sizeof(int), ctx->stream));
+            k_list_occupied<<<blocks_for(ctx->n_cells), kThreads, 0, ctx->stream>>>(ctx->n_cells, ctx->start[ctx->cur],
+                                                                                    ctx->occ[ctx->cur], ctx->meta[ctx->cur]);
+            CK_LAUNCH();
         }
         ctx->lanes = g;
         ctx->store = store;

@@ -1,5 +1,5 @@
-// epp_cells.cuh -- cell-list build: bin (atomic counts, linked lists of the cells), exclusive scan,
-// rank-by-id gather (a counting sort with a deterministic within-cell order).
+// epp_cells.cuh -- cell-list build: bin (atomic counts, linked lists of the cells or slots in them),
+// exclusive scan, rank-by-id gather (a counting sort with a deterministic within-cell order).
 //
 // Replaces the reference's fixed-capacity buckets (NeighbourSearch.jl:12-47, clean! at
 // NeighbourSystem.jl:43-54): the counts, offsets and membership of every cell equal the
@@ -19,14 +19,16 @@ __device__ __forceinline__ void set_status(unsigned* status, unsigned bits) {
 }
 
 // What a bin pass leaves for the counting sort, per particle i: its cell and its place among its
-// cell's particles.  The particles of a cell form a linked list from head[c] (-1: none) through
-// link[i] = (next, id), in arrival order; particles of the dead bin (c = n_cells), which can be many,
-// take a slot of it instead.  tile[t] counts the particles of scan tile t (2048 cells).
+// cell's particles.  With `head` the particles of a cell form a linked list of count[c] entries from
+// head[c] through link[i] = (next, id), in arrival order (the last one's next, like the head of an empty
+// cell, is whatever the memory held: the count ends a walk), and only particles of the dead bin (c =
+// n_cells), which can be many, take a slot.  Without it all take a slot of their cell, for a scatter pass
+// that brings a cell's particles together.  tile[t] counts the particles of scan tile t (2048 cells).
 struct BinOut {
-    int2* cs;      // (cell, slot in the dead bin)
+    int2* cs;      // (cell, slot: of the dead bin only where there are lists)
     int2* link;    // (next particle of the cell, id)
     int* count;    // [n_cells + 1] zero on entry
-    int* head;     // [n_cells] -1 on entry
+    int* head;     // [n_cells], or null
     int* tile;     // [tiles * stride] zero on entry
     int stride;    // ints between two tile counters: a cache line apart where there is room, since the
                    // atomics of one line are served one after the other (binning 955,668 particles in
@@ -40,7 +42,7 @@ __device__ __forceinline__ void bin_particle(const BinOut& B, int n_cells, int i
     const unsigned same = __match_any_sync(__activemask(), t);
     if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&B.tile[t * B.stride], __popc(same));
     int slot = 0;
-    if (c == n_cells) {
+    if (!B.head || c == n_cells) {
         slot = atomicAdd(&B.count[c], 1);
     } else {
         atomicAdd(&B.count[c], 1);
@@ -75,10 +77,9 @@ __global__ void k_bin_count(int n, DevDomain dom, State s, BinOut B, unsigned* s
     bin_particle(B, dom.n_cells, i, s.id[i], c);
 }
 
-// What a scan resets for the bin pass after the next: the head and tile buffers not in use (they
-// alternate), and per-cell checks of its counts.
+// What a scan resets for the bin pass after the next, the tile buffer not in use (they alternate), and
+// per-cell checks of its counts.
 struct ScanReset {
-    int* head;        // [n_cells] of the other buffer
     int* tile;        // [tiles * stride] of the other buffer
     int stride;
     int max_cell;     // > 0: a cell of the domain with more particles sets EPP_STATUS_CELL_OVERFLOW
@@ -111,15 +112,10 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(int m, int* 
     if (full) {
         reinterpret_cast<int4*>(count + base)[0] = make_int4(0, 0, 0, 0);
         reinterpret_cast<int4*>(count + base)[1] = make_int4(0, 0, 0, 0);
-        reinterpret_cast<int4*>(R.head + base)[0] = make_int4(-1, -1, -1, -1);
-        reinterpret_cast<int4*>(R.head + base)[1] = make_int4(-1, -1, -1, -1);
     } else {
 #pragma unroll
         for (int k = 0; k < kScanItems; ++k)
-            if (base + k < m) {
-                count[base + k] = 0;
-                R.head[base + k] = -1;
-            }
+            if (base + k < m) count[base + k] = 0;
     }
     int sum = 0;
     bool over = false;
@@ -188,8 +184,6 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int m, int* count,
     const int tile = s_tile;
     const int base = tile * kScanTile + threadIdx.x * kScanItems;
     if (threadIdx.x == 0) R.tile[tile * R.stride] = 0;
-    for (int k = 0; k < kScanItems; ++k)
-        if (base + k < m) R.head[base + k] = -1;
     const bool full = base + kScanItems <= m;   // the thread's 8 cells are all in range (aligned)
     int v[kScanItems];
     if (full) {   // two 16-byte loads, then zero the counts for the next step
@@ -298,6 +292,43 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int m, int* count,
     }
 }
 
+// Rank of each particle within its cell by id, from the cell's linked list, and its move to start +
+// rank by the mover (src, dst, cell).  A thread per particle in the old order: reads of the state are
+// coalesced, writes nearly so (a step moves few particles to another cell), and no scatter pass has to
+// bring a cell's particles together first (8 of 32 us of the sort at 515,018 particles).  The dead bin
+// keeps arrival order (dead particles never interact).  A destination outside [0, n) can only come from a failed
+// scan; it is reported, never written.
+__device__ __forceinline__ int sorted_place(int i, int2 cs, int n_cells, int n, const int2* link, const int* head,
+                                            const int* start) {
+    const int s = start[cs.x];
+    if (cs.x == n_cells) return s + cs.y;
+    const int id = link[i].y;
+    int rank = 0, j = head[cs.x];
+    for (int left = start[cs.x + 1] - s; left > 0 && (unsigned)j < (unsigned)n; --left) {   // the cell's particles
+        const int2 e = link[j];
+        rank += e.y < id;
+        j = e.x;
+    }
+    return s + rank;
+}
+
+template <class Mover>
+__global__ void k_rank_gather(int n, int n_cells, const int2* link, const int2* cs, const int* head, const int* start,
+                              Mover mv, unsigned* status) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int2 c = cs[i];
+    // in flight while the rank is found, and none behind a store (a load cannot pass one): 18.9 -> 14.8 us at
+    // 515,018 particles, 182 -> 160 at 6,207,228
+    const typename Mover::Item m = mv.load(i);
+    const int dst = sorted_place(i, c, n_cells, n, link, head, start);
+    if (dst < 0 || dst >= n) {
+        atomicOr(status, EPP_STATUS_QUEUE);
+        return;
+    }
+    mv.store(m, dst, c.x);
+}
+
 // Scatter in arrival order, for cells in no list: perm[start[c] + slot] = (id, source index).  A destination
 // outside [0, n) can only come from a failed scan; it is reported, never written.
 __device__ __forceinline__ void scatter_particle(int i, int n, int2 c, const int* start, int id, int2* perm, unsigned* status) {
@@ -316,40 +347,42 @@ __device__ __forceinline__ int sorted_place_perm(int p, int2 e, int c, int n, in
     return s + rank;
 }
 
-// Rank of each particle within its cell by id, from the cell's linked list, and its move to start +
-// rank by the mover (src, dst, cell).  A thread per particle in the old order: reads of the state are
-// coalesced, writes nearly so (a step moves few particles to another cell), and no scatter pass has to
-// bring a cell's particles together first (8 of 32 us of the sort at 515,018 particles).  The dead bin
-// keeps arrival order (dead particles never interact).  A destination outside [0, n) can only come from a failed
-// scan; it is reported, never written.
-__device__ __forceinline__ int sorted_place(int i, int2 cs, int n_cells, const int2* link, const int* head, const int* start) {
-    const int s = start[cs.x];
-    if (cs.x == n_cells) return s + cs.y;
-    const int id = link[i].y;
-    int rank = 0, j = head[cs.x];
-    for (int left = start[cs.x + 1] - s; left > 0 && j >= 0; --left) {   // at most the cell's particles
-        const int2 e = link[j];
-        rank += e.y < id;
-        j = e.x;
-    }
-    return s + rank;
+static __global__ void k_scatter(int n, const int2* cs, const int* start, const int* id, int2* perm, unsigned* status) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) scatter_particle(i, n, cs[i], start, id[i], perm, status);
 }
 
+// The gather of a sort by slots: a thread per entry of perm.
 template <class Mover>
-__global__ void k_rank_gather(int n, int n_cells, const int2* link, const int2* cs, const int* head, const int* start,
-                              Mover mv, unsigned* status) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int2 c = cs[i];
-    // in flight while the rank is found, and none behind a store (a load cannot pass one): 18.9 -> 14.8 us at
-    // 515,018 particles, 182 -> 160 at 6,207,228
-    const typename Mover::Item m = mv.load(i);
-    const int dst = sorted_place(i, c, n_cells, link, head, start);
+__global__ void k_rank_gather_perm(int n, int n_cells, const int2* perm, const int2* cs, const int* start, Mover mv,
+                                   unsigned* status) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= n) return;
+    const int2 e = perm[p];
+    if (e.y < 0 || e.y >= n) {
+        atomicOr(status, EPP_STATUS_QUEUE);
+        return;
+    }
+    const int c = cs[e.y].x;
+    const typename Mover::Item m = mv.load(e.y);
+    const int dst = sorted_place_perm(p, e, c, n, n_cells, perm, start);
     if (dst < 0 || dst >= n) {
         atomicOr(status, EPP_STATUS_QUEUE);
         return;
     }
-    mv.store(m, dst, c.x);
+    mv.store(m, dst, c);
+}
+
+// The occupied cells of a finished order, in no order of their own (family 1 taken up between searches;
+// *n_occ is zero on entry).
+static __global__ void k_list_occupied(int n_cells, const int* start, int* occ, int* n_occ) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const bool mine = c < n_cells && start[c + 1] > start[c];
+    const unsigned all = __ballot_sync(0xffffffffu, mine);
+    int base = 0;
+    if (lane == 0 && all) base = atomicAdd(n_occ, __popc(all));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (mine) occ[base + __popc(all & ((1u << lane) - 1u))] = c;
 }
 
 // Mover of the per-call search: every state array follows the particle.

@@ -51,3 +51,26 @@ def test_sort_time_of_shuffled_particles(dim):
 @pytest.mark.parametrize("dim", [2, 3])
 def test_sort_time_of_crowded_cells(dim):
     assert sort_time(dim, 300000, 300, False) <= 2.5 * sort_time(dim, 300000, 9, True)
+
+
+# Family 1 taken up by a context of a large grid: no device memory beyond the budget's, and no wait.
+def test_family_one_takes_no_memory():
+    import torch
+    from epp import casegen
+    from epp.algorithm import DeviceParticleSystem
+    from epp.classes import Domain2D, NeighbourSystem
+    case = casegen.dam_break_2d(dx=0.05, max_neighbour_number=1)
+    first = case.domain.first
+    case.ps.domain = case.domain = Domain2D(0.15, first[0], first[1], 0.15 * 8000, 0.15 * 8000)
+    assert case.domain.get_n() > 60e6
+    d = DeviceParticleSystem(case.ps, NeighbourSystem(case.domain, casegen.DAM_BREAK_ACTIVE_PAIRS, max_neighbour_number=1))
+    d.syncto()
+    d.ctx.search(abi.EPP_CRITERION_SYMMETRY, abi.EPP_ACTION_DAMBREAK_CONTINUITY, case.physics, 0)
+    d.ctx.step(2, case.physics)
+    d.ctx.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    d.ctx.set_tuning(1)
+    d.ctx.step(2, case.physics)
+    d.ctx.synchronize()
+    assert torch.cuda.mem_get_info()[0] >= free - (64 << 20)   # graphs, not heads of 60 million cells
+    d.close()
