@@ -636,9 +636,12 @@ int prepare_kernels(epp_ctx* ctx) {
     return g ? EPP_ERR_CUDA : EPP_OK;
 }
 
-// Whether a sort ranks a cell's particles from their linked list: one launch fewer than by slots and a
-// scatter pass.  Family 1 keeps the occupied cells where the heads would go.
-bool sorts_by_lists(const epp_ctx* ctx) { return ctx->lanes != 1; }
+// Whether a sort ranks a cell's particles from their linked list.  One launch fewer than by slots and a
+// scatter pass, but a dependent load per particle of the cell: rank and scatter, us, lists against slots
+// 18.8 / 27.6 with 36 to a cell (515,018 particles), 43 / 48 with 64 (955,668), 35 / 28 with 125 (381,720),
+// 21 / 17 with 144 (23,018); pair passes of such cells take 100 times that.  Family 1 keeps the occupied
+// cells where the heads would go.
+bool sorts_by_lists(const epp_ctx* ctx) { return ctx->lanes != 1 && (long long)ctx->n <= 64ll * ctx->n_cells; }
 
 // The bin buffers of step parity / call `b`.
 BinOut bin_out(epp_ctx* ctx, int b) {

@@ -53,6 +53,57 @@ def test_sort_time_of_crowded_cells(dim):
     assert sort_time(dim, 300000, 300, False) <= 2.5 * sort_time(dim, 300000, 9, True)
 
 
+def crowd(dim, side, n, seed=4):
+    """A context of n particles at random places of side^dim cells, a tenth of them outside."""
+    from collections import OrderedDict
+    from epp import casegen
+    from epp.algorithm import DeviceParticleSystem
+    from epp.classes import Domain2D, Domain3D, NeighbourSystem, ParticleSystem
+    rng = np.random.default_rng(seed)
+    domain = (Domain2D if dim == 2 else Domain3D)(1.0 / (side + 0.01), *[0.0] * dim, *[1.0] * dim)
+    ints, floats = casegen._layout(dim, 1)
+    ps = ParticleSystem(domain, n, ints, floats, OrderedDict([("rho0", 1000.0)]))
+    x = rng.random((n, dim)).astype(np.float32)
+    x[rng.random(n) < 0.1] += 5.0
+    one = np.ones(n, np.float32)
+    ps["PositionVec"], ps["H"], ps["Density"], ps["Mass"], ps["Volume"] = x, one * 1e-3, one, one, one
+    ps["Tag"], ps["IsMovable"] = np.full(n, casegen.FLUID_TAG, np.int32), np.ones(n, np.int32)
+    d = DeviceParticleSystem(ps, NeighbourSystem(domain, casegen.DAM_BREAK_ACTIVE_PAIRS, max_neighbour_number=1))
+    d.syncto()
+    return d, domain, x
+
+
+def numpy_cells(domain, x):
+    """(counts, ids in cell order, each cell's rising) of positions, by the domain's own FP32 cell index."""
+    dim = x.shape[1]
+    first, last = np.array(domain.first, np.float32), np.array(domain.last, np.float32)
+    inside = np.all((x >= first) & (x <= last), axis=1)
+    cell, stride = np.zeros(len(x), np.int64), 1
+    for a in range(dim):
+        k = np.floor((x[:, a] - first[a]) * np.float32(domain.gap_inv[a])).astype(np.int64)
+        cell += np.clip(k, 0, domain.n_axis[a] - 1) * stride
+        stride *= domain.n_axis[a]
+    ids = np.flatnonzero(inside)
+    order = ids[np.argsort(cell[inside], kind="stable")]
+    return np.bincount(cell[inside], minlength=stride), order + 1
+
+
+# Either side of 64 particles to a cell, where the sort goes from linked lists to slots; the families that
+# always take one of the two; more than one search, as the buffers alternate.
+@pytest.mark.parametrize("dim,side", [(2, 6), (3, 3)])
+@pytest.mark.parametrize("over", [-1, 0, 1])
+@pytest.mark.parametrize("family", [0, 1, 4])
+def test_cells_of_crowded_contexts(dim, side, over, family):
+    d, domain, x = crowd(dim, side, 64 * side ** dim + over)
+    d.ctx.set_tuning(family)
+    counts, ids = numpy_cells(domain, x)
+    for _ in range(3):
+        d.ctx.search(abi.EPP_CRITERION_SYMMETRY, abi.EPP_ACTION_NONE, None, 0)
+        got = d.ctx.cell_stats()
+        assert np.array_equal(got[0], counts) and np.array_equal(got[2][:len(ids)], ids)
+    d.close()
+
+
 # Family 1 taken up by a context of a large grid: no device memory beyond the budget's, and no wait.
 def test_family_one_takes_no_memory():
     import torch
