@@ -263,8 +263,15 @@ size_t state_bytes(int cap) {
     return (size_t)cap * (4 * 16 + 7 * 4) + 12 * 256;
 }
 
-// Ints between two scan-tile counters: a cache line while both buffers fit the arena's slack.
+// Ints between two scan-tile counters: a cache line while both buffers fit the arena's slack; of more tiles
+// they lie side by side in the look-back state of family 1.
 int tile_stride(int n_tiles) { return n_tiles <= 3800 ? 32 : n_tiles <= 15000 ? 8 : 1; }
+
+// Scan tiles beyond which their counters are summed once, by a launch of their own, and not by each tile.
+// A step of 6,518 particles in a nearly empty grid, us, each tile / once: 654 tiles 27.1 / 28.9, 952 29.7 /
+// 29.7, 1,306 32.1 / 32.0, 2,391 43.1 / 38.1, 22,393 147 / 123, 89,542 1466 / 387, 520,886 44350 / 2101 (look-back
+// there 11840).
+constexpr int kTileSumMax = 1250;
 
 size_t arena_bytes(int cap, int n_cells, int D, int n_tiles) {
     size_t b = 2 * state_bytes(cap);
@@ -281,7 +288,7 @@ size_t arena_bytes(int cap, int n_cells, int D, int n_tiles) {
     b += (size_t)kIntegralBlocks * 8 * 8 + 8 * 8 + 4 * 256;
     b += 4 * ((size_t)cap * 4 + 256);                    // filter / extrapolation sums, gap by row
     b += 2 * 256;                                                                  // instance tables (small)
-    return b + std::max((size_t)1 << 20, 2 * ((size_t)n_tiles * tile_stride(n_tiles) * 4 + 256) + 4096);   // tile counters
+    return b + (1 << 20);   // slack: the tile counters (2 * 4 * 32 * 3,800 bytes at most)
 }
 
 // Device memory of a context comes from the stream-ordered allocator on the context's stream:
@@ -645,7 +652,13 @@ bool sorts_by_lists(const epp_ctx* ctx) { return ctx->lanes != 1 && (long long)c
 
 // The bin buffers of step parity / call `b`.
 BinOut bin_out(epp_ctx* ctx, int b) {
-    return BinOut{ctx->cs, ctx->link, ctx->count, sorts_by_lists(ctx) ? ctx->head : nullptr, ctx->tile[b], ctx->tile_stride};
+    return BinOut{ctx->cs, ctx->link, ctx->count, sorts_by_lists(ctx) ? ctx->head : nullptr,
+                  ctx->lanes == 1 ? nullptr : ctx->tile[b], ctx->tile_stride};
+}
+
+int clear_tiles(epp_ctx* ctx, int k) {
+    CK(cudaMemsetAsync(ctx->tile[k], 0, sizeof(int) * (size_t)ctx->n_tiles * ctx->tile_stride, ctx->stream));
+    return EPP_OK;
 }
 
 // Words of look-back state a bin pass clears: only the cell-centric family scans with it.
@@ -653,13 +666,19 @@ int scan_words(const epp_ctx* ctx) { return ctx->lanes == 1 ? ctx->n_tiles + 1 :
 
 // The scan of the bin pass of buffers `b` into set `to`.
 int launch_scan(epp_ctx* ctx, int b, int to, int max_cell) {
-    const ScanReset R{ctx->tile[1 - b], ctx->tile_stride, max_cell};
+    const ScanReset R{ctx->tile[1 - b], ctx->tile_stride};
     if (ctx->lanes == 1)
         k_scan<<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->start[to], ctx->occ[to],
-                                                              ctx->meta[to], ctx->scan_state, R, ctx->status);
-    else
-        k_scan_tiles<<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->tile[b],
-                                                                    ctx->start[to], R, ctx->status);
+                                                              ctx->meta[to], ctx->scan_state, max_cell, ctx->status);
+    else if (ctx->n_tiles > kTileSumMax) {
+        k_tile_prefix<<<1, kPrefixThreads, 0, ctx->stream>>>(ctx->n_tiles, ctx->tile[b], ctx->tile_stride);
+        CK_LAUNCH();
+        k_scan_tiles<true><<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->tile[b],
+                                                                          ctx->start[to], R, max_cell, ctx->status);
+    } else {
+        k_scan_tiles<false><<<ctx->n_tiles, kScanThreads, 0, ctx->stream>>>(ctx->n_cells + 1, ctx->count, ctx->tile[b],
+                                                                           ctx->start[to], R, max_cell, ctx->status);
+    }
     CK_LAUNCH();
     return EPP_OK;
 }
@@ -1233,8 +1252,9 @@ int32_t epp_create(const epp_config* cfg, epp_ctx** out) {
     ctx->meta[1] = a.take<int>(64);
     ctx->scan_state = a.take<unsigned long long>(ctx->n_tiles + 1);
     ctx->tile_stride = tile_stride(ctx->n_tiles);
-    ctx->tile[0] = a.take<int>((size_t)ctx->n_tiles * ctx->tile_stride);
-    ctx->tile[1] = a.take<int>((size_t)ctx->n_tiles * ctx->tile_stride);
+    for (int k = 0; k < 2; ++k)
+        ctx->tile[k] = ctx->tile_stride > 1 ? a.take<int>((size_t)ctx->n_tiles * ctx->tile_stride)
+                                            : reinterpret_cast<int*>(ctx->scan_state) + k * (ctx->n_tiles + 1);
     ctx->head = ctx->occ[0];   // the occupied cells are listed for family 1 only
     ctx->status = a.take<unsigned>(1);
     ctx->pairs = a.take<unsigned long long>(1);
@@ -1408,9 +1428,9 @@ int32_t epp_upload(epp_ctx* ctx, int32_t n, const int32_t* is_alive, const int32
             if (tc[k] < 0 || tc[k] > 255) return fail(ctx, EPP_ERR_INVALID_ARGUMENT, "tag %d out of range", tc[k]);
     }
     if (rc) return rc;
-    if (ctx->cur == 1) {   // the last sort left the bin buffers of set 1 ready; the next one is from set 0
-        CK(cudaMemsetAsync(ctx->tile[0], 0, sizeof(int) * (size_t)ctx->n_tiles * ctx->tile_stride, ctx->stream));
-    }
+    // the last sort left the tile counters of set 1 ready; the next one is from set 0
+    if (ctx->cur == 1)
+        if (const int rc_ = clear_tiles(ctx, 0)) return rc_;
     ctx->cur = 0;
     auto launch = [&](auto Dt) {
         constexpr int DD = decltype(Dt)::value;
@@ -1922,6 +1942,11 @@ int32_t epp_set_tuning(epp_ctx* ctx, int32_t lanes_per_particle) {
     if (g != 0 && ctx->n_inst > 1)
         return fail(ctx, EPP_ERR_INVALID_ARGUMENT, "batches of %d instances use pair-pass family 0", ctx->n_inst);
     if (g != ctx->lanes || store != ctx->store) {
+        if (g != 1 && ctx->lanes == 1) {   // family 1's sorts use no tile counters, but may use their memory
+            cudaSetDevice(ctx->dev);
+            for (int k = 0; k < 2; ++k)
+                if (const int rc_ = clear_tiles(ctx, k)) return rc_;
+        }
         if (g == 1 && ctx->lanes != 1 && ctx->sorted_once) {   // family 1 goes by the occupied cells: list those of the current order
             cudaSetDevice(ctx->dev);
             if (const int rc_ = join_integrals(ctx)) return rc_;

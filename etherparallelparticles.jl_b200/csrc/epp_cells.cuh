@@ -29,7 +29,7 @@ struct BinOut {
     int2* link;    // (next particle of the cell, id)
     int* count;    // [n_cells + 1] zero on entry
     int* head;     // [n_cells], or null
-    int* tile;     // [tiles * stride] zero on entry
+    int* tile;     // [tiles * stride] zero on entry, or null (family 1, whose scan does not go by it)
     int stride;    // ints between two tile counters: a cache line apart where there is room, since the
                    // atomics of one line are served one after the other (binning 955,668 particles in
                    // lattice order: 29 us packed, 15 a line apart)
@@ -38,9 +38,11 @@ struct BinOut {
 // Adds particle i of id `id` to cell c.  The tile counters are updated once per group of the warp's
 // active lanes with one tile (sorted particles: nearly always all of them).
 __device__ __forceinline__ void bin_particle(const BinOut& B, int n_cells, int i, int id, int c) {
-    const int t = c / kScanTile;
-    const unsigned same = __match_any_sync(__activemask(), t);
-    if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&B.tile[t * B.stride], __popc(same));
+    if (B.tile) {
+        const int t = c / kScanTile;
+        const unsigned same = __match_any_sync(__activemask(), t);
+        if ((threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&B.tile[t * B.stride], __popc(same));
+    }
     int slot = 0;
     if (!B.head || c == n_cells) {
         slot = atomicAdd(&B.count[c], 1);
@@ -77,21 +79,55 @@ __global__ void k_bin_count(int n, DevDomain dom, State s, BinOut B, unsigned* s
     bin_particle(B, dom.n_cells, i, s.id[i], c);
 }
 
-// What a scan resets for the bin pass after the next, the tile buffer not in use (they alternate), and
-// per-cell checks of its counts.
+// What a scan by tile counters resets for the bin pass after the next: the buffer not in use (the two
+// alternate).
 struct ScanReset {
-    int* tile;        // [tiles * stride] of the other buffer
+    int* tile;        // [tiles * stride]
     int stride;
-    int max_cell;     // > 0: a cell of the domain with more particles sets EPP_STATUS_CELL_OVERFLOW
 };
+
+// The tile counters as their exclusive sums, in place, by one block: for grids of so many tiles that each
+// adding up all counters before its own is the longer way.
+constexpr int kPrefixThreads = 1024, kPrefixItems = 4;
+static __global__ void __launch_bounds__(kPrefixThreads) k_tile_prefix(int tiles, int* tile, int stride) {
+    __shared__ int s_warp[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int carry = 0;   // of the chunks before, in every thread
+    for (int t0 = 0; t0 < tiles; t0 += kPrefixThreads * kPrefixItems) {
+        const int t = t0 + threadIdx.x * kPrefixItems;
+        int v[kPrefixItems], sum = 0;
+#pragma unroll
+        for (int k = 0; k < kPrefixItems; ++k) v[k] = t + k < tiles ? tile[(size_t)(t + k) * stride] : 0;
+#pragma unroll
+        for (int k = 0; k < kPrefixItems; ++k) sum += v[k];
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        const int w = s_warp[lane];
+        int run = carry + incl - sum + __reduce_add_sync(0xffffffffu, lane < warp ? w : 0);
+        carry += __reduce_add_sync(0xffffffffu, w);
+#pragma unroll
+        for (int k = 0; k < kPrefixItems; ++k) {
+            if (t + k < tiles) tile[(size_t)(t + k) * stride] = run;
+            run += v[k];
+        }
+        __syncthreads();   // s_warp is written again
+    }
+}
 
 // Exclusive scan over m = n_cells + 1 counts (the last is the dead bin) from the tile counters of the
 // bin pass: start[0..m], with the counts cleared for the next binning pass.  A tile sums the counters
-// before it itself -- a few hundred, read at once -- so no tile waits for another (the look-back scan
-// below, which this replaces on the default path, is a chain through its tiles: 10 us against 4 at
-// 335,336 cells).
-static __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(int m, int* count, const int* tile, int* start,
-                                                                   ScanReset R, unsigned* status) {
+// before it itself, or (PREFIX) reads their sum, so no tile waits for another (the look-back scan below
+// is a chain through its tiles: 10 us against 4 at 335,336 cells).  A cell of the domain with more than
+// max_cell > 0 particles sets EPP_STATUS_CELL_OVERFLOW.
+template <bool PREFIX>
+__global__ void __launch_bounds__(kScanThreads) k_scan_tiles(int m, int* count, const int* tile, int* start,
+                                                                   ScanReset R, int max_cell, unsigned* status) {
     __shared__ int s_sum[kScanThreads / 32], s_warp[kScanThreads / 32];
     const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int base = t * kScanTile + threadIdx.x * kScanItems;
@@ -107,7 +143,11 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(int m, int* 
         for (int k = 0; k < kScanItems; ++k) v[k] = base + k < m ? count[base + k] : 0;
     }
     int before = 0;   // particles of the tiles before this one
-    for (int q = threadIdx.x; q < t; q += kScanThreads) before += tile[q * R.stride];
+    if (PREFIX) {
+        if (threadIdx.x == 0) before = tile[t * R.stride];
+    } else {
+        for (int q = threadIdx.x; q < t; q += kScanThreads) before += tile[q * R.stride];
+    }
     if (threadIdx.x == 0) R.tile[t * R.stride] = 0;
     if (full) {
         reinterpret_cast<int4*>(count + base)[0] = make_int4(0, 0, 0, 0);
@@ -122,7 +162,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(int m, int* 
 #pragma unroll
     for (int k = 0; k < kScanItems; ++k) {
         sum += v[k];
-        over = over || (R.max_cell > 0 && base + k < m - 1 && v[k] > R.max_cell);
+        over = over || (max_cell > 0 && base + k < m - 1 && v[k] > max_cell);
     }
     if (over) set_status(status, EPP_STATUS_CELL_OVERFLOW);
     int incl = sum;
@@ -158,8 +198,8 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan_tiles(int m, int* 
 }
 
 // The same for the cell-centric pair passes, which also need the occupied cells: single-pass scan with
-// decoupled look-back over m = n_cells + 1 counts (the last is the dead bin).  Writes start[0..m], the list of occupied cells occ[0..n_occ) in cell order
-// (meta[0] = n_occ) and clears the counts for the next binning pass.  Tiles take a ticket in
+// decoupled look-back over m = n_cells + 1 counts (the last is the dead bin).  Writes start[0..m], the list
+// of occupied cells occ[0..n_occ) in cell order (meta[0] = n_occ) and clears the counts for the next binning pass.  Tiles take a ticket in
 // launch order so every predecessor is already running; the wait on a predecessor is bounded
 // and reports EPP_STATUS_SPIN_TIMEOUT instead of hanging.
 // scan_state layout: [0] ticket, [1 + t] status word of tile t:
@@ -174,7 +214,7 @@ __device__ __forceinline__ unsigned long long unpack_status(unsigned long long w
 }
 
 static __global__ void __launch_bounds__(kScanThreads) k_scan(int m, int* count, int* start, int* occ,
-                                                       int* meta, unsigned long long* scan_state, ScanReset R,
+                                                       int* meta, unsigned long long* scan_state, int max_cell,
                                                        unsigned* status) {
     __shared__ int s_tile;
     __shared__ unsigned long long s_warp[kScanThreads / 32];
@@ -183,7 +223,6 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int m, int* count,
     __syncthreads();
     const int tile = s_tile;
     const int base = tile * kScanTile + threadIdx.x * kScanItems;
-    if (threadIdx.x == 0) R.tile[tile * R.stride] = 0;
     const bool full = base + kScanItems <= m;   // the thread's 8 cells are all in range (aligned)
     int v[kScanItems];
     if (full) {   // two 16-byte loads, then zero the counts for the next step
@@ -205,7 +244,7 @@ static __global__ void __launch_bounds__(kScanThreads) k_scan(int m, int* count,
     for (int k = 0; k < kScanItems; ++k) {
         const int idx = base + k;
         tsum += (unsigned long long)v[k] + ((idx < m - 1 && v[k] > 0) ? (1ull << 32) : 0ull);
-        if (R.max_cell > 0 && idx < m - 1 && v[k] > R.max_cell) set_status(status, EPP_STATUS_CELL_OVERFLOW);
+        if (max_cell > 0 && idx < m - 1 && v[k] > max_cell) set_status(status, EPP_STATUS_CELL_OVERFLOW);
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long incl = tsum;

@@ -175,8 +175,8 @@ int32_t epp_cell_sort_noalloc(const epp_domain* domain, int32_t n, const float* 
         else k_na_bin<3><<<gb, kNaBinThreads, 0, s>>>(n, dom, pos, tiles, cs, count, tile);
     }
     // (the scan resets the spare tile counters)
-    k_scan_tiles<<<tiles, kScanThreads, 0, s>>>(nc + 1, count, tile, start, ScanReset{tile + kNaTiles * kTileStride, kTileStride, 0},
-                                               reinterpret_cast<unsigned*>(meta + 1));
+    k_scan_tiles<false><<<tiles, kScanThreads, 0, s>>>(nc + 1, count, tile, start, ScanReset{tile + kNaTiles * kTileStride, kTileStride},
+                                                      0, reinterpret_cast<unsigned*>(meta + 1));
     if (n > 0) k_na_scatter<<<grid(n), T, 0, s>>>(n, cs, start, perm, meta);
     k_na_rank<<<grid(std::max(n, nc + 1)), T, 0, s>>>(n, nc, perm, cs, start, sorted_ids, counts, offsets, meta);
     if (cudaGetLastError() != cudaSuccess) return EPP_ERR_CUDA;

@@ -125,3 +125,61 @@ def test_family_one_takes_no_memory():
     d.ctx.synchronize()
     assert torch.cuda.mem_get_info()[0] >= free - (64 << 20)   # graphs, not heads of 60 million cells
     d.close()
+
+
+# The scan over either side of the tile counts at which its counters lie otherwise or are summed by a launch of
+# their own: a small column of water in the corner of a large domain steps as in its own, whatever family
+# sorted it in between, and through an upload at either parity.
+@pytest.mark.parametrize("tiles", [1250, 1251, 3800, 3801, 4097, 15000, 15001])
+def test_steps_in_large_grids(tiles):
+    from epp import casegen
+    from epp.algorithm import DeviceParticleSystem
+    from epp.classes import Domain2D, NeighbourSystem
+    out = []
+    for far in (False, True):
+        case = casegen.dam_break_2d(dx=0.05, max_neighbour_number=1)
+        if far:   # the same cells on x (the same order), more of them on y
+            dom = case.domain
+            gap, first, last = float(dom.gap), [float(v) for v in dom.first], [float(v) for v in dom.last]
+            rows = int(np.ceil((tiles * 2048 - 1) / dom.n_axis[0]))
+            case.ps.domain = case.domain = Domain2D(gap, first[0], first[1], last[0], first[1] + (rows + 0.4) * float(dom.gap_axis[1]))
+        d = DeviceParticleSystem(case.ps, NeighbourSystem(case.domain, casegen.DAM_BREAK_ACTIVE_PAIRS, max_neighbour_number=1))
+        d.syncto()
+        d.ctx.search(abi.EPP_CRITERION_SYMMETRY, abi.EPP_ACTION_DAMBREAK_CONTINUITY, case.physics, 0)
+        d.ctx.step(3, case.physics)
+        d.ctx.set_tuning(1)
+        d.ctx.step(2, case.physics)
+        d.ctx.set_tuning(0)
+        d.ctx.step(2, case.physics)
+        d.ctx.synchronize()
+        d.asyncto()
+        d.syncto()
+        d.ctx.search(abi.EPP_CRITERION_SYMMETRY, abi.EPP_ACTION_NONE, case.physics, 0)
+        ids = d.ctx.cell_stats()[2]
+        d.asyncto()
+        out.append([d.host[k].copy() for k in ("PositionVec", "VelocityVec", "nCount", "dDensity")] + [ids])
+        n = case.domain.get_n()
+        d.close()
+    assert (n + 2048) // 2048 >= tiles
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)
+
+
+# the scan's time follows the number of cells (each tile adding up all counters before it made it 5 times the
+# look-back scan's at this size, and growing with the square)
+def test_scan_time_of_a_large_grid():
+    from epp import casegen
+    from epp.algorithm import DeviceParticleSystem
+    from epp.classes import Domain2D, NeighbourSystem
+    times = []
+    for side in (4000, 16000):
+        case = casegen.dam_break_2d(dx=0.05, max_neighbour_number=1)
+        first = case.domain.first
+        case.ps.domain = case.domain = Domain2D(0.15, first[0], first[1], 0.15 * side, 0.15 * side)
+        d = DeviceParticleSystem(case.ps, NeighbourSystem(case.domain, casegen.DAM_BREAK_ACTIVE_PAIRS, max_neighbour_number=1))
+        d.syncto()
+        d.ctx.search(abi.EPP_CRITERION_SYMMETRY, abi.EPP_ACTION_DAMBREAK_CONTINUITY, case.physics, 0)
+        st = [list(s.values()) if isinstance(s, dict) else list(s) for s in (d.ctx.profile_step(case.physics) for _ in range(5))]
+        times.append(np.min(np.array(st), axis=0)[1])   # the scan
+        d.close()
+    assert times[1] <= 2.0 * 16 * times[0]
