@@ -79,8 +79,10 @@ __device__ __forceinline__ void traverse(const PairArgs& A, int i, float4 xi, in
 
 // Adds the per-thread neighbour counts of a block's warps to *counter (all lanes take part).
 __device__ __forceinline__ void count_pairs(unsigned long long* counter, int cnt) {
-    const int c = __reduce_add_sync(0xffffffffu, cnt);   // 32 counts of at most 2^26 candidates each
-    if ((threadIdx.x & 31) == 0 && counter && c) atomicAdd(counter, (unsigned long long)c);
+    const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)cnt & 0xffffu);   // 32 counts of up to 2^28
+    const unsigned hi = __reduce_add_sync(0xffffffffu, (unsigned)cnt >> 16);
+    const unsigned long long c = ((unsigned long long)hi << 16) + lo;
+    if ((threadIdx.x & 31) == 0 && counter && c) atomicAdd(counter, c);
 }
 
 template <int D, class Act>

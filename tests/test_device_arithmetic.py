@@ -1,5 +1,5 @@
 """Arithmetic of the kernels' headers, compiled from them: exact division by multiplication, packed FP32
-operations and the fast reciprocal."""
+operations, the fast reciprocal and the pair counter."""
 import ctypes as C
 import os
 import shutil
@@ -35,6 +35,7 @@ __global__ void rcp_kernel(const float* x, float* r, int n) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) r[i] = rcp_fast(x[i]);
 }
+__global__ void count_kernel(const int* cnt, unsigned long long* total) { count_pairs(total, cnt[threadIdx.x]); }
 
 static int grid(int n) { return (n + 127) / 128; }
 extern "C" {
@@ -55,6 +56,10 @@ int packed(const float* a, const float* b, unsigned* bad, int n) {
 }
 int reciprocal(const float* x, float* r, int n) {
     rcp_kernel<<<grid(n), 128>>>(x, r, n);
+    return (int)cudaDeviceSynchronize();
+}
+int count(const int* cnt, unsigned long long* total) {
+    count_kernel<<<1, 32>>>(cnt, total);
     return (int)cudaDeviceSynchronize();
 }
 }
@@ -136,3 +141,14 @@ def test_fast_reciprocal_is_within_one_ulp(lib):
         want = 1.0 / x.astype(np.float64)
         ulp = 2.0 ** (np.floor(np.log2(want)) - 23)
         assert np.all(np.abs(r.cpu().numpy().astype(np.float64) - want) <= ulp), e
+
+
+# 32 lanes of 2^27 neighbours and more (contexts hold 2^28 particles): beyond 32 bits
+@pytest.mark.gpu
+@pytest.mark.parametrize("cnt", [0, 1, 65535, 65536, (1 << 27) + 3, (1 << 28) - 1])
+def test_pair_counter_of_a_warp(lib, cnt):
+    import torch
+    c = torch.arange(32, dtype=torch.int32, device="cuda") * (1 if cnt else 0) + max(cnt - 31, 0)
+    total = torch.full((1,), 5, dtype=torch.int64, device="cuda")
+    assert lib.count(ptr(c), ptr(total)) == 0
+    assert int(total.item()) == 5 + int(c.to(torch.int64).sum().item())
