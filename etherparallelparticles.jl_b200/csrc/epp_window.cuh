@@ -49,14 +49,14 @@ __device__ __forceinline__ int stencil_row(const PairArgs& A, int rid, int y, in
     return rid + yy - y + (D == 3 ? A.dom.n[1] * dz : 0);
 }
 
-// Candidates of cells xa .. xb (clamped to the grid) of linear cell row `row` (-1: none).
+// Candidates of cells xa .. xb (clamped to the grid) of linear cell row `row` (-1: none).  A range beyond
+// either end of the row is empty where the row ends: the ranges of a part's lanes stay in order.
 __device__ __forceinline__ RowWin row_range(const PairArgs& A, int row, int xa, int xb) {
     RowWin w{0, 0};
     if (row < 0) return w;
     const int n0 = A.dom.n[0];
     xa = max(xa, 0);
     xb = min(xb, n0 - 1);
-    if (xa > xb) return w;
     const int l = max(A.start[row * n0 + xa], 0);
     const int h = min(A.start[row * n0 + xb + 1], A.n_max);
     w.lo = l;
