@@ -38,13 +38,13 @@ import numpy as np  # noqa: E402
 #   continuity         read x, v, id; write drho                                   2D 24,  3D 32
 #   whole step                                                                     2D 189, 3D 245
 # The kernels of a step re-split those stages: the momentum pass also bins (momentum + hash and
-# count), the reorder is the scatter (key + rank, 8 B; no kernel of its own) and the rank-by-id gather,
-# and the continuity stage is split between the search pass (reads x and id) and the continuity
+# count), the reorder is the rank-by-id gather alone (it ranks from the bin's linked cell lists; the scatter
+# stage is family 1's), and the continuity stage is split between the search pass (reads x and id) and the continuity
 # pass (reads v, writes drho).  The per-kernel figures add up to the whole step.
 B_ALG_STEP = {2: 189.0, 3: 245.0}
 STAGES = ["momentum_integrate_bin", "scan", "scatter", "rank_gather", "search", "continuity"]
 B_ALG_STAGE = {"momentum_integrate_bin": {2: 80.0, 3: 108.0}, "scan": {2: 5.0, 3: 0.5},
-               "scatter": {2: 8.0, 3: 8.0}, "rank_gather": {2: 72.0, 3: 96.0},
+               "scatter": {2: 0.0, 3: 0.0}, "rank_gather": {2: 80.0, 3: 104.0},
                "search": {2: 12.0, 3: 16.0}, "continuity": {2: 12.0, 3: 16.0}}
 PAIR_STAGES = ("momentum_integrate_bin", "search", "continuity")
 KERNEL_OF_STAGE = {"momentum_integrate_bin": "k_list<CPMom> (momentum + integrate + bin, fused)",
@@ -753,9 +753,9 @@ def main():
             "pairs_per_step": pairs_all / args.steps / world,
             "step_hbm_gbs_algorithmic": step_bytes / (step_ms * 1e-3) / 1e9,
             "step_roofline_frac": step_bytes / (step_ms * 1e-3) / 1e9 / peak,
-            # per fused step: momentum+integrate+bin, scan, scatter, rank+gather, search, continuity
+            # per fused step: momentum+integrate+bin, scan, scatter (family 1), rank+gather, search, continuity
             # (2D family 0 and the other families run the continuity action inside the search pass)
-            "gpu_launches": (5 if (args.lanes == 0 and dim == 3) or args.lanes == 64 else 4) * args.steps
+            "gpu_launches": (5 if (args.lanes == 0 and dim == 3) or args.lanes in (1, 64) else 4) * args.steps
                             + (2 * (args.steps // phys.filter_interval) if phys.filter_interval else 0),
             "roofline": {"bound": "hbm", "kernel": kernel_of[dom_stage], "achieved": achieved, "peak": peak,
                          "unit": "GB/s", "frac": achieved / peak, "traffic": traffic,

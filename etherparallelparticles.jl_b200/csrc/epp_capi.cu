@@ -2081,6 +2081,7 @@ int32_t epp_profile_step(epp_ctx* ctx, const epp_physics* phys, float* stage_ms)
         cudaError_t e = cudaEventSynchronize(ev[kProfileStages]);
         for (int k = 0; k < kProfileStages && e == cudaSuccess; ++k)
             e = cudaEventElapsedTime(&stage_ms[k], ev[k], ev[k + 1]);
+        if (sorts_by_lists(ctx)) stage_ms[2] = 0.0f;   // no scatter pass: two events side by side
         if (e != cudaSuccess) rc = fail(ctx, EPP_ERR_CUDA, "profile events: %s", cudaGetErrorString(e));
     }
     for (int k = 0; k <= kProfileStages; ++k) cudaEventDestroy(ev[k]);

@@ -375,7 +375,8 @@ int32_t epp_server_download(epp_server* server, int64_t request_id, int32_t* is_
                             int32_t* int_props, int64_t ld_int, float* float_props, int64_t ld_float);
 
 /* One dam-break step launched kernel by kernel (no graph) with CUDA events between the
- * kernels; stage_ms[0 .. EPP_PROFILE_STAGES-1] = momentum+integrate+bin, scan, 0 (once a scatter),
+ * kernels; stage_ms[0 .. EPP_PROFILE_STAGES-1] = momentum+integrate+bin, scan, scatter (0 where the
+ * sort has none: it ranks from linked lists, but for family 1 and grids of more than 64 particles a cell),
  * rank+gather, search (neighbour lists), continuity (0 for pair-pass families that fuse the
  * search and continuity into one kernel).  Same results as epp_step(ctx, 1, phys). */
 #define EPP_PROFILE_STAGES 6
