@@ -276,7 +276,7 @@ constexpr int kTileSumMax = 1250;
 size_t arena_bytes(int cap, int n_cells, int D, int n_tiles) {
     size_t b = 2 * state_bytes(cap);
     b += (size_t)cap * 3 * 16 + 3 * 256;                 // fused temp
-    b += (size_t)cap * (16 + 32) + 512;           // rp4, 2D neighbour records (both sets)
+    b += (size_t)cap * (16 + 32) + 512;           // rp4, neighbour records (one of each for both sets)
     b += (size_t)(n_cells + 2) * 4 + 256;                // count
     b += 2 * ((size_t)(n_cells + 2) * 4 + 256);          // start[2]
     b += (size_t)(n_tiles + 1) * 8 + 256;                // scan state
@@ -483,7 +483,8 @@ bool generic_physics(const epp_physics* p) {
 
 // Family 0 in 2D searches each particle's own stencil-row windows with the search action folded in
 // (epp_window.cuh), unless the context was set to the lockstep list search and a separate
-// continuity pass (epp_set_tuning EPP_TUNING_LISTS); 3D always uses the latter.
+// continuity pass (epp_set_tuning EPP_TUNING_LISTS).  In 3D the search pass (windows there too) only
+// lists and counts, and continuity is a pass of its own.
 bool uses_windows(const epp_ctx* ctx) { return ctx->D == 2 && ctx->store != EPP_TUNING_LISTS; }
 
 // Largest particle count at which the search pass takes eight lanes per particle: measured, us with
@@ -2108,8 +2109,8 @@ int32_t epp_get_accel(epp_ctx* ctx, float* out, int32_t n) {
     if (!ctx->accel) return fail(ctx, EPP_ERR_STATE, "accel output disabled");
     cudaSetDevice(ctx->dev);
     if (const int rc_ = join_integrals(ctx)) return rc_;
-    // accel is indexed by the order before the last gather; the permutation is cs/perm.  Copy
-    // with the id array of that order (the other ping-pong set).
+    // accel is indexed by the order before the last gather: copy with the id array of that order (the
+    // other ping-pong set)
     std::vector<float4> a(ctx->n);
     std::vector<int> ids(ctx->n);
     CK(cudaStreamSynchronize(ctx->stream));

@@ -1,21 +1,21 @@
-// epp_tile.cuh -- the default pair passes: warp tiles over a shared candidate list.
+// epp_tile.cuh -- neighbour lists: the pair passes over them (k_list), and the 2D lockstep search of
+// EPP_TUNING_LISTS that builds them (k_build; the default searches are in epp_window.cuh).
 //
-// A warp takes 32 consecutive particles in cell order.  When their cells lie in one cell row
-// (x from xa to xb at fixed y, z) the union of their 3^D stencils is, for each of the 3^(D-1)
-// stencil rows (y+dy, z+dz), the cells xa-1 .. xb+1 -- contiguous in cell order, so 3 (2D) or
-// 9 (3D) contiguous particle ranges shared by the whole warp.  A warp that crosses a row end
-// (about 2% of them) uses each lane's own stencil instead; both passes make the same choice.
+// k_list (continuity, momentum, filter, extrapolation, the count actions) walks each particle's list
+// with one or four lanes a particle, so every lane runs its own neighbours without waiting for the
+// others' candidates; a particle with more neighbours than a list keeps takes its stencil instead.
 //
-// The search pass (k_build) stages each chunk of 32 candidates in shared memory with one
-// coalesced load per lane; every lane then tests all 32 staged candidates against its own
-// particle with broadcast shared-memory reads -- all lanes in lockstep -- using the reference's
-// IEEE criterion and the active-pair matrix, and appends its accepted neighbours (sorted index
-// and tag, candidate order) to its list.  The pair passes (k_list: continuity, momentum, the
-// count actions) then walk each particle's list, one thread per particle, so every lane runs
-// its own neighbour count without waiting for the others' candidates.
+// k_build takes 32 consecutive particles in cell order a warp.  When their cells lie in one cell row (x
+// from xa to xb at fixed y) the union of their stencils is, for each of the three stencil rows, the
+// cells xa-1 .. xb+1 -- contiguous in cell order, so three particle ranges shared by the whole warp.  A
+// warp that crosses a row end (about 2% of them) uses each lane's own stencil instead.  Each chunk of
+// 32 candidates is staged in shared memory with one coalesced load per lane; every lane tests all of
+// them against its own particle -- all lanes in lockstep -- by the reference's IEEE criterion and the
+// active-pair matrix, and appends its accepted neighbours (sorted index and tag, candidate order).
 //
-// Summation order per particle = stencil rows (z, y offset), then cell order, then id order
-// inside a cell: deterministic, a rounding-level reordering of the reference's list order.
+// Summation order per particle = stencil rows (z, y offset), then cell order, then id order inside a
+// cell: deterministic, a rounding-level reordering of the reference's list order (3D momentum adds four
+// interleaved partial sums of it).
 #pragma once
 #include "epp_cellpair.cuh"
 
@@ -149,40 +149,6 @@ template <int D>
 __device__ __forceinline__ ListWriter<D> list_writer(const TileMask& M, int i) {
     return ListWriter<D>{ListConf<D>::ROW ? M.list + (size_t)i * ListConf<D>::LCAP : M.list + i, M.cap, 0, 0, 0};
 }
-
-// Reads a particle's list in order, the next entries already in flight: 2D (column-major) one
-// entry at a time through next(), with streaming loads (each entry is read once: evicted first,
-// so the neighbour records the pass gathers keep the L1; momentum -1.7%); 3D (row-major) rows are
-// read four entries at a time by k_list from the two groups start() loads, as ordinary loads (a
-// row's next group shares its line: streaming loads there cost the 3D list passes 5-9%).
-template <int D>
-struct ListReader {
-    const int* base;
-    int cap, cnt;
-    int4 q, qn;
-    __device__ __forceinline__ void start(const TileMask& M, int i, int n) {
-        cap = M.cap;
-        cnt = n;
-        if (ListConf<D>::ROW) {
-            base = M.list + (size_t)i * ListConf<D>::LCAP;
-            const int4* row = reinterpret_cast<const int4*>(base);
-            q = n > 0 ? row[0] : make_int4(0, 0, 0, 0);
-            qn = n > 4 ? row[1] : make_int4(0, 0, 0, 0);
-        } else {
-            base = M.list + i;
-            q.x = n > 0 ? __ldcs(base) : 0;
-        }
-    }
-    // entry k of a column-major list (called with k = 0, 1, 2, ... < cnt)
-    __device__ __forceinline__ int next(int k) {
-        const int j = q.x;
-        if (k + 1 < cnt) {   // the next entry one column on
-            base += cap;
-            q.x = __ldcs(base);
-        }
-        return j;
-    }
-};
 
 // Candidate ranges (contiguous particle index ranges) of a warp tile or of one particle.
 template <int D>

@@ -1,5 +1,6 @@
-// epp_window.cuh -- the 2D search pass over per-particle stencil-row windows, with the search
-// action folded in.
+// epp_window.cuh -- the default search passes, over per-particle stencil-row windows: in 2D with the
+// search action folded in (described here), in 3D lists and counts only (k_win_build3), and with eight
+// lanes per particle for small systems (k_win_lanes).
 //
 // A particle's 3x3 cell stencil is three stencil rows (dy = -1, 0, +1); in each row its
 // candidates are one contiguous cell-order range, cells cx-1 .. cx+1 (its "window", about 27
