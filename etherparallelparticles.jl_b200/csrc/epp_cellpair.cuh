@@ -313,15 +313,19 @@ struct CPMom {
         const float dwr = __fmul_rn(kdw, __fmul_rn(__fmul_rn(u, u), u));
         float s = __fadd_rn(me.rp.z, pz);                                                               // iClassicPressure!
         if (!ff) s = __fmul_rn(__fmul_rn(__fadd_rn(me.rp.y, pz), me.rp.w), __frcp_rn(rhoj));   // iBalancedPressure!
-        float f = __fmul_rn(s, __fmul_rn(mj, dwr));
+        const float md = __fmul_rn(mj, dwr);
+        float f = __fmul_rn(s, md);
         // sArtificialViscosity!: approaching pairs only
         const float az = __fmaf_rn(__fmul_rn(0.01f, hh), hh, dr2);
         const float phi = __fmul_rn(vdx, rcp_fast(__fmul_rn(hinv, az)));
         const float w = __fmul_rn(__fmul_rn(__fmaf_rn(P.beta, phi, -__fmul_rn(P.alpha, me.c0)), phi),
                                   __fmul_rn(2.0f, rcp_fast(__fadd_rn(me.rp.x, rhoj))));
-        float mv = mj;
-        if (P.visc == EPP_VISCOSITY_REFERENCE) mv = __fmul_rn(__fmul_rn(mj, me.rp.w), rcp_fast(rhoj));
-        if (vdx < 0.0f) f = __fmaf_rn(w, __fmul_rn(mv, dwr), f);
+        // m_j dW/r over both densities; the kernel's factor first in 3D and last in 2D (momentum, us, first /
+        // last: 3D 6,207,228 particles 1886 / 1940, 2D 1,217,760 169 / 164)
+        float mv = D == 3 ? md : mj;
+        if (P.visc == EPP_VISCOSITY_REFERENCE) mv = __fmul_rn(__fmul_rn(mv, me.rp.w), rcp_fast(rhoj));
+        if (D == 2) mv = __fmul_rn(mv, dwr);
+        if (vdx < 0.0f) f = __fmaf_rn(w, mv, f);
         return u > 0.0f && (ff || tj == P.wall) ? -f : 0.0f;
     }
     __device__ __forceinline__ float4 term(const Self& me, const Nb& nb, int ti, int tj, float4 xj,
