@@ -384,9 +384,9 @@ __global__ void __launch_bounds__(128, 7) k_win_build(const __grid_constant__ Pa
 // candidates at h = 1.3 dx, one plane (three rows) staged at a time; a particle's 480 candidates are
 // tested by its own lane.  It replaces a lockstep search of the warp's whole union of stencils (about
 // 700 candidates, 32 at a time, with a divergent append after each chunk): 574 -> 356 us at 955,668
-// particles, 182 -> 84 at 165,888.  Issue-bound (79% of the slots): about half on the tests, 40% on the
-// walk over their bits, which is why a word whose candidates have one tag computes its entries and
-// checks the list's capacity once.  Warps near walls stage two h's and take the two bounds by a select.
+// particles, 182 -> 84 at 165,888.  Issue-bound (80% of the slots, 22.7 of 32 lanes at
+// work: the walk over a word's bits is as long as the busiest lane's), which is why a word whose
+// candidates have one tag computes its entries and checks the list's capacity once.  Warps near walls stage two h's and take the two bounds by a select.
 // When one particle's plane is longer than the staging area (dense neighbourhoods) the stencil goes by
 // rows, or by cells, and a cell beyond it is read from global memory by all its lanes at once: 926 us
 // at h = 2.5 dx and 165,888 particles, where a pass for each lane with a long row took 12800.
