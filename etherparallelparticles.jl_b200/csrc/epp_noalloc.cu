@@ -3,9 +3,9 @@
 // Some hosts of this library may not call cudaMalloc while they drive a simulation: a host
 // application whose device memory comes from its own fixed pool, or a caller in the middle of a
 // step where a device allocation would synchronise the device or is simply not permitted.  For
-// them epp_cell_sort_noalloc runs the bin -> scan -> scatter -> rank-by-id pipeline
-// as the context's search!, on device buffers the caller passes in, with every intermediate
-// array in one statically sized device array declared below.  That array is part of the library:
+// them epp_cell_sort_noalloc builds the cell list of the context's search! (bin into slots, scan,
+// scatter, rank by id) on device buffers the caller passes in, with every intermediate array in one
+// statically sized device array declared below.  That array is part of the library:
 // every GPU that loads libepp.so holds it until the process exits.
 #include <cuda_runtime.h>
 
